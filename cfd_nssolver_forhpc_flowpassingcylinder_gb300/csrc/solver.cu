@@ -221,64 +221,89 @@ __global__ void __launch_bounds__(kBlock) k64_as(Geo g, Stencil<double> st, Kryl
   if (grid_sum<2>(a, part, &sc->cnt[2], out) && lin_tid() == 0) sc->omega = out[0] / out[1];
 }
 
-// stop test, beta and restart decision of bicgstabRe2.hpp:128-176 (last block, thread 0);
-// n2 = ||r1||^2, rr = <r1, r0>
+// The scalar work that ends an iteration is one thread's chain of FP64 divisions, each a
+// few dozen instructions at 64 cycles: warp 0 of the last block takes them on three lanes
+// at once (one division sequence instead of three).  a0 / b0, a1 / b1, a2 / b2 in every lane
+// of the warp.
+__device__ __forceinline__ void div3(double a0, double b0, double a1, double b1, double a2, double b2, double &q0,
+                                     double &q1, double &q2) {
+  const int l = lin_tid() & 31;
+  const double q = (l == 0 ? a0 : l == 1 ? a1 : a2) / (l == 0 ? b0 : l == 1 ? b1 : b2);
+  q0 = __shfl_sync(0xffffffffu, q, 0);
+  q1 = __shfl_sync(0xffffffffu, q, 1);
+  q2 = __shfl_sync(0xffffffffu, q, 2);
+}
+
+// stop test, beta and restart decision of bicgstabRe2.hpp:128-176 (last block, warp 0);
+// n2 = ||r1||^2, rr = <r1, r0>.  Every scalar is loaded before the decisions, so that their
+// latencies overlap.
 template <bool FP32>
 __device__ __forceinline__ void finish_iteration(SolverScal *sc, double n2, double rr) {
-  const double relres = sqrt(n2) / sc->norm0;
+  if (lin_tid() >= 32) return;
+  const double tol = sc->tol, rho_old = sc->rho, rn = sqrt(n2);
+  const double peak_max = sc->rmax, rstart = sc->rstart, delta = sc->delta, peak = sc->peak, best = sc->best,
+               snap_rel = sc->snap_rel, thr = sc->restart_thr;
+  const int iter = sc->iter, maxit = sc->maxit, timestep = sc->timestep, snap_iter = sc->snap_iter;
+  const double omega = sc->omega;
+  double relres, ao, rq;
+  div3(rn, sc->norm0, sc->alpha, omega, rr, rho_old, relres, ao, rq);
+  const double beta = ao * rq;
+  if (lin_tid() != 0) return;
   sc->relres = relres;
   if (FP32) {
     // MIXED sweep: hand over to the FP64 refinement once the residual has dropped by delta
     // below the sweep's start, or by peak below the sweep's largest one (BiCGSTAB's
     // residual can rise far above its start before it falls, and an FP32 recursion cannot
     // follow it down many decades below such a peak), or looks converged
-    const double rn = sqrt(n2);
-    if (relres < sc->best) sc->best = relres;
+    if (relres < best) sc->best = relres;
     // keep this iterate (the next x update copies it) once its residual has halved since
     // the last one kept: a few copies per sweep, and the sweep's correction is never worse
     // than that kept iterate, whatever the residual does afterwards
-    sc->snap = relres <= 0.5 * sc->snap_rel;
-    if (sc->snap) sc->snap_rel = relres;
+    const bool snap = relres <= 0.5 * snap_rel;
+    sc->snap = snap;
+    if (snap) {
+      sc->snap_rel = relres;
+      sc->snap_iter = iter;
+    }
     if (!isfinite(relres)) {
       sc->done = 1;
       sc->status = CFDGB_ENAN;
-    } else if (sc->iter > 16 && relres > 1e3 * sc->best) {
+    } else if (iter > 16 && relres > 1e3 * (relres < best ? relres : best)) {
       // runaway growth (BiCGSTAB's ordinary bumps stay far below this)
       sc->done = 1;
       sc->status = CFDGB_ENOCONV;
-    } else if (sc->iter >= sc->maxit) {
+    } else if (iter >= maxit) {
       sc->done = 1;
       sc->status = CFDGB_ENOCONV;
-      sc->iter += 1;
-    } else if (relres < sc->tol || rn < sc->delta * sc->rstart || rn < sc->peak * sc->rmax) {
+      sc->iter = iter + 1;
+    } else if (relres < tol || rn < delta * rstart || rn < peak * peak_max) {
       sc->done = 1;
       sc->status = kStatusRefine;
-      sc->iter += 1;
+      sc->iter = iter + 1;
+    } else if (!snap && iter - snap_iter >= kSweepStall) {
+      sc->done = 1;
+      sc->status = CFDGB_ENOCONV;
+      sc->iter = iter + 1;
     } else {
-      const double rho_old = sc->rho;
-      sc->rho = rr;
-      sc->beta = (sc->alpha / sc->omega) * (rr / rho_old);
-      sc->restart = 0;
-      if (!(isfinite(sc->beta) && sc->omega != 0.0 && rr != 0.0)) {  // Lanczos breakdown
-        sc->restart = 1;
-        sc->rho = n2;
-      }
-      sc->rmax = fmax(sc->rmax, rn);
-      sc->iter += 1;
+      sc->beta = beta;
+      const bool broke = !(isfinite(beta) && omega != 0.0 && rr != 0.0);  // Lanczos breakdown
+      sc->restart = broke ? 1 : 0;
+      sc->rho = broke ? n2 : rr;
+      sc->rmax = fmax(peak_max, rn);
+      sc->iter = iter + 1;
     }
     return;
   }
-  if (relres < sc->tol) {  // :129
+  if (relres < tol) {  // :129
     sc->done = 1;
-  } else if (sc->iter >= sc->maxit) {  // :133
+  } else if (iter >= maxit) {  // :133
     sc->done = 1;
     sc->status = CFDGB_ENOCONV;
   } else {  // :156-176
-    const double rho_old = sc->rho;
     sc->rho = rr;
-    sc->beta = (sc->alpha / sc->omega) * (sc->rho / rho_old);
-    sc->restart = !(sc->timestep < 10 || fabs(rho_old) > sc->restart_thr);
-    sc->iter += 1;
+    sc->beta = beta;
+    sc->restart = !(timestep < 10 || fabs(rho_old) > thr);
+    sc->iter = iter + 1;
   }
 }
 
@@ -297,7 +322,7 @@ __global__ void __launch_bounds__(kBlock) k64_xr(Geo g, KrylovVecs<double> v, do
     acc[1] += r1 * v.r0[row];
   }
   double out[2];
-  if (grid_sum<2>(acc, part, &sc->cnt[3], out) && lin_tid() == 0) finish_iteration<false>(sc, out[0], out[1]);
+  if (grid_sum<2>(acc, part, &sc->cnt[3], out)) finish_iteration<false>(sc, out[0], out[1]);
 }
 
 // K5: p1 = r1 + beta (p1 - omega ap), or restart r0 = p1 = r1
@@ -404,8 +429,8 @@ __global__ void __launch_bounds__(kBlock) k32_xr(Geo g, Vec32 v, double *part, S
     rr.add(r1 * v.r0[row]);
   }
   double acc[2] = {n2.get(), rr.get()}, out[2];
-  if (grid_sum<2>(acc, part, &sc->cnt[3], out) && lin_tid() == 0) {
-    sc->par ^= 1;  // this iteration's p and ap become the previous ones
+  if (grid_sum<2>(acc, part, &sc->cnt[3], out)) {
+    if (lin_tid() == 0) sc->par = parity ^ 1;  // this iteration's p and ap become the previous ones
     finish_iteration<true>(sc, out[0], out[1]);
   }
 }
@@ -497,7 +522,7 @@ __global__ void __launch_bounds__(kBlock) k32p_xr(Geo g, PrecVecs v, double *par
     rr.add(r1 * v.r0[row]);
   }
   double acc[2] = {n2.get(), rr.get()}, out[2];
-  if (grid_sum<2>(acc, part, &sc->cnt[3], out) && lin_tid() == 0) finish_iteration<true>(sc, out[0], out[1]);
+  if (grid_sum<2>(acc, part, &sc->cnt[3], out)) finish_iteration<true>(sc, out[0], out[1]);
 }
 
 // ---- FP64 BiCGSTAB with the FP64 V-cycle as right preconditioner ----
@@ -506,26 +531,28 @@ __global__ void __launch_bounds__(kBlock) k32p_xr(Geo g, PrecVecs v, double *par
 // reference's iteration, so no rho-restart rule: it stops on the tolerance, the cap or a
 // non-finite residual, and restarts only on a Lanczos breakdown.
 __device__ __forceinline__ void finish_prec64(SolverScal *sc, double n2, double rr) {
-  const double relres = sqrt(n2) / sc->norm0;
+  if (lin_tid() >= 32) return;
+  const double tol = sc->tol, omega = sc->omega;
+  const int iter = sc->iter + 1, maxit = sc->maxit;
+  double relres, ao, rq;
+  div3(sqrt(n2), sc->norm0, sc->alpha, omega, rr, sc->rho, relres, ao, rq);
+  const double beta = ao * rq;
+  if (lin_tid() != 0) return;
   sc->relres = relres;
-  sc->iter += 1;
+  sc->iter = iter;
   if (!isfinite(relres)) {
     sc->done = 1;
     sc->status = CFDGB_ENAN;
-  } else if (relres < sc->tol) {
+  } else if (relres < tol) {
     sc->done = 1;
-  } else if (sc->iter >= sc->maxit) {
+  } else if (iter >= maxit) {
     sc->done = 1;
     sc->status = CFDGB_ENOCONV;
   } else {
-    const double rho_old = sc->rho;
-    sc->rho = rr;
-    sc->beta = (sc->alpha / sc->omega) * (rr / rho_old);
-    sc->restart = 0;
-    if (!(isfinite(sc->beta) && sc->omega != 0.0 && rr != 0.0)) {
-      sc->restart = 1;
-      sc->rho = n2;
-    }
+    sc->beta = beta;
+    const bool broke = !(isfinite(beta) && omega != 0.0 && rr != 0.0);
+    sc->restart = broke ? 1 : 0;
+    sc->rho = broke ? n2 : rr;
   }
 }
 
@@ -600,7 +627,7 @@ __global__ void __launch_bounds__(kBlock) k64p_xr(Geo g, PrecVecsT<double> v, do
     acc[1] = fma(r1, v.r0[row], acc[1]);
   }
   double out[2];
-  if (grid_sum<2>(acc, part, &sc->cnt[3], out) && lin_tid() == 0) finish_prec64(sc, out[0], out[1]);
+  if (grid_sum<2>(acc, part, &sc->cnt[3], out)) finish_prec64(sc, out[0], out[1]);
 }
 
 // ---- FP32 iteration, vectorised: four consecutive k cells per thread (nzc % 4 == 0) ----
@@ -881,7 +908,7 @@ __global__ void __launch_bounds__(kBlock) k32pv_xr(Geo g, PrecVecs v, double *pa
     st4(v.r1 + row, r1);
   }
   double acc[2] = {n2.get(), rr.get()}, out[2];
-  if (grid_sum<2>(acc, part, &sc->cnt[3], out) && lin_tid() == 0) finish_iteration<true>(sc, out[0], out[1]);
+  if (grid_sum<2>(acc, part, &sc->cnt[3], out)) finish_iteration<true>(sc, out[0], out[1]);
 }
 
 // ---- FP32 stencil kernels on a bulk-copy (TMA) pipeline ----
@@ -1259,8 +1286,8 @@ __global__ void __launch_bounds__(kBlock) k32v_xr(Geo g, Vec32 v, double *part, 
     st4(r1v + row, r1);
   }
   double acc[2] = {n2.get(), rr.get()}, out[2];
-  if (grid_sum<2>(acc, part, &sc->cnt[3], out) && lin_tid() == 0) {
-    sc->par ^= 1;  // this iteration's p and ap become the previous ones
+  if (grid_sum<2>(acc, part, &sc->cnt[3], out)) {
+    if (lin_tid() == 0) sc->par = parity ^ 1;  // this iteration's p and ap become the previous ones
     finish_iteration<true>(sc, out[0], out[1]);
   }
 }
@@ -1284,20 +1311,25 @@ int fp32_pointwise_blocks_per_sm() {
 // iteration; the FP32 sweeps of the MIXED mode fuse the p update into the SpMV (two
 // kernels, 10 words per cell).
 __device__ __forceinline__ void finish_cg64(SolverScal *sc, double n2) {
-  const double relres = sqrt(n2) / sc->norm0;
+  if (lin_tid() >= 32) return;
+  const double tol = sc->tol;
+  const int iter = sc->iter, maxit = sc->maxit;
+  double relres, beta, unused;
+  div3(sqrt(n2), sc->norm0, n2, sc->rho, n2, sc->rho, relres, beta, unused);
+  if (lin_tid() != 0) return;
   sc->relres = relres;
-  if (relres < sc->tol) {
+  if (relres < tol) {
     sc->done = 1;
   } else if (!isfinite(relres)) {
     sc->done = 1;
     sc->status = CFDGB_ENAN;
-  } else if (sc->iter >= sc->maxit) {
+  } else if (iter >= maxit) {
     sc->done = 1;
     sc->status = CFDGB_ENOCONV;
   } else {
-    sc->beta = n2 / sc->rho;
+    sc->beta = beta;
     sc->rho = n2;
-    sc->iter += 1;
+    sc->iter = iter + 1;
   }
 }
 
@@ -1355,7 +1387,7 @@ __global__ void __launch_bounds__(kBlock) k64cg_xr(Geo g, KrylovVecs<double> v, 
     a[0] += r * r;
   }
   double out[1];
-  if (grid_sum<1>(a, part, &sc->cnt[3], out) && lin_tid() == 0) finish_cg64(sc, out[0]);
+  if (grid_sum<1>(a, part, &sc->cnt[3], out)) finish_cg64(sc, out[0]);
 }
 // p = r + beta p
 __global__ void __launch_bounds__(kBlock) k64cg_p(Geo g, KrylovVecs<double> v, const SolverScal *sc) {
@@ -1369,33 +1401,34 @@ __global__ void __launch_bounds__(kBlock) k64cg_p(Geo g, KrylovVecs<double> v, c
 
 // FP32 sweep (MIXED): hand over to the FP64 refinement like the BiCGSTAB sweeps
 __device__ __forceinline__ void finish_cg32(SolverScal *sc, double n2) {
-  const double relres = sqrt(n2) / sc->norm0, rn = sqrt(n2);
+  if (lin_tid() >= 32) return;
+  const double tol = sc->tol, best = sc->best, delta = sc->delta, rmax = sc->rmax, rn = sqrt(n2);
+  const int iter = sc->iter, maxit = sc->maxit;
+  double relres, beta, unused;
+  div3(rn, sc->norm0, n2, sc->rho, n2, sc->rho, relres, beta, unused);
+  if (lin_tid() != 0) return;
   sc->relres = relres;
-  if (relres < sc->best) sc->best = relres;
+  if (relres < best) sc->best = relres;
   if (!isfinite(relres)) {
     sc->done = 1;
     sc->status = CFDGB_ENAN;
-  } else if (sc->iter > 16 && relres > 1e3 * sc->best) {
+  } else if (iter > 16 && relres > 1e3 * (relres < best ? relres : best)) {
     sc->done = 1;
     sc->status = CFDGB_ENOCONV;
-  } else if (sc->iter >= sc->maxit) {
+  } else if (iter >= maxit) {
     sc->done = 1;
     sc->status = CFDGB_ENOCONV;
-    sc->iter += 1;
-  } else if (relres < sc->tol || rn < sc->delta * sc->rmax) {
+    sc->iter = iter + 1;
+  } else if (relres < tol || rn < delta * rmax) {
     sc->done = 1;
     sc->status = kStatusRefine;
-    sc->iter += 1;
+    sc->iter = iter + 1;
   } else {
-    sc->beta = n2 / sc->rho;
+    sc->beta = beta;
     sc->rho = n2;
-    sc->restart = 0;
-    if (!isfinite(sc->beta)) {
-      sc->restart = 1;
-      sc->rho = n2;
-    }
-    sc->rmax = fmax(sc->rmax, rn);
-    sc->iter += 1;
+    sc->restart = isfinite(beta) ? 0 : 1;
+    sc->rmax = fmax(rmax, rn);
+    sc->iter = iter + 1;
   }
 }
 
@@ -1532,8 +1565,8 @@ __global__ void __launch_bounds__(kBlock) k32cg_xr(Geo g, Vec32 v, double *part,
     }
   }
   double acc[1] = {n2.get()}, out[1];
-  if (grid_sum<1>(acc, part, &sc->cnt[3], out) && lin_tid() == 0) {
-    sc->par ^= 1;
+  if (grid_sum<1>(acc, part, &sc->cnt[3], out)) {
+    if (lin_tid() == 0) sc->par = parity ^ 1;
     finish_cg32(sc, out[0]);
   }
 }
@@ -1659,6 +1692,7 @@ __global__ void __launch_bounds__(kBlock) k_refine_start32(Geo g, Stencil<double
     sc->rel0 = sc->relres;
     sc->snap_rel = sc->relres;  // x = 0, kept by the first x update
     sc->snap = 1;
+    sc->snap_iter = sc->iter;
     sc->done = 0;
     sc->status = 0;
     sc->restart = 1;
