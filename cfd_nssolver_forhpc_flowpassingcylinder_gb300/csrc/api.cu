@@ -404,15 +404,16 @@ double sor_omega_opt(const cfdgb_config *c) {
 }
 
 // The step kernels' divisors are the metric arrays and dt: the single correction of div_by
-// is proven only for certified divisors (div_certified); any other one, or a dt that an
-// adaptive rule chooses on the device, selects the double correction
-bool division_twice(const cfdgb_ctx *c) {
-  if (c->cfg.dt_mode != CFDGB_DT_FIXED || !div_certified(c->cfg.dt)) return true;
+// is proven only for certified divisors (div_certified); any other metric, or any other dt or
+// one that an adaptive rule chooses on the device, selects the double correction for its own
+// divisions
+bool metrics_twice(const cfdgb_ctx *c) {
   for (auto *v : {&c->Dx, &c->Dy, &c->Dz, &c->Dxs, &c->Dys, &c->Dzs})
     for (double d : *v)
       if (!div_certified(d)) return true;
   return false;
 }
+bool dt_twice(const cfdgb_ctx *c) { return c->cfg.dt_mode != CFDGB_DT_FIXED || !div_certified(c->cfg.dt); }
 
 int validate(const cfdgb_config *c) {
   if (!c) return fail(CFDGB_EINVAL, "null config");
@@ -1217,6 +1218,7 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, c->device) != cudaSuccess) return bail(fail(CFDGB_ECUDA, "device query"));
   c->nsm = prop.multiProcessorCount;
+  if (!convdiff_prepare()) return bail(fail(CFDGB_ECUDA, "kernel attributes"));
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(fail(CFDGB_ECUDA, "stream create"));
   // grid (structureGrid.hpp:336-367): uniform, X[0] = -2 dx, running sums
@@ -1291,6 +1293,15 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
     const std::vector<double> *DD[3] = {&c->Dx, &c->Dy, &c->Dz}, *DS[3] = {&c->Dxs, &c->Dys, &c->Dzs};
     for (int a = 0; a < 3; ++a)
       for (size_t q = 0; q < DD[a]->size(); ++q) rm.push_back(((*DS[a])[q] * 0.5) / (*DD[a])[q]);
+    for (int a = 0; a < 3; ++a) {  // QUICK's factors (Geo::qkx)
+      const auto &D = *DD[a], &S = *DS[a];
+      const size_t n = D.size();
+      auto at = [&](const std::vector<double> &m, size_t q) { return m[std::min(q, n - 1)]; };
+      for (size_t q = 0; q < n; ++q) rm.push_back(0.125 * at(D, q + 1) * at(D, q + 1) / S[q]);
+      for (size_t q = 0; q < n; ++q) rm.push_back(0.125 * at(D, q + 1) * at(D, q + 1) / at(S, q + 1));
+      for (size_t q = 0; q < n; ++q) rm.push_back(0.125 * S[q] * S[q] / D[q]);
+      for (size_t q = 0; q < n; ++q) rm.push_back(0.125 * S[q] * S[q] / at(D, q + 1));
+    }
     double *drm = nullptr;
     if ((rc = dalloc(c, &drm, rm.size()))) return bail(rc);
     if (cudaMemcpy(drm, rm.data(), rm.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1298,8 +1309,10 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
     g.rDx = drm; g.rDy = g.rDx + nx; g.rDz = g.rDy + ny;
     g.rDxs = g.rDz + nz; g.rDys = g.rDxs + nx; g.rDzs = g.rDys + ny;
     g.hfx = g.rDzs + nz; g.hfy = g.hfx + nx; g.hfz = g.hfy + ny;
+    g.qkx = g.hfz + nz; g.qky = g.qkx + 4 * nx; g.qkz = g.qky + 4 * ny;
   }
-  g.div2 = division_twice(c) ? 1 : 0;
+  g.div2 = metrics_twice(c) ? 1 : 0;
+  g.div2t = dt_twice(c) ? 1 : 0;
   g.uni = 1;
   for (auto *v : {&c->Dx, &c->Dy, &c->Dz, &c->Dxs, &c->Dys, &c->Dzs})
     for (double d : *v)
@@ -1349,7 +1362,7 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
   g.lgx = (cfg->nz + g.lbx - 1) / g.lbx;
   g.lgy = (cfg->ny + g.lby - 1) / g.lby;
   g.lgz = std::max(1, std::min(cfg->nx, c->nsm * 8 / std::max(1, g.lgx * g.lgy)));
-  int nblk3 = g.lgx * g.lgy * g.lgz;
+  int nblk3 = std::max(g.lgx * g.lgy * g.lgz, kConvdiffBlocks * c->nsm);
   // vectorised FP32 kernels: quads of four k cells per thread when nz % 4 == 0
   // (the stretched grid's MIXED sweeps run the scalar kernels, on its stored FP32 rows)
   // the flat pointwise kernels (every SM filled): the FP32 quad kernels and the MIXED
@@ -1834,7 +1847,7 @@ int cfdgb_set_dt(cfdgb_ctx *c, double dt) {
   if (!(dt > 0.0) || !std::isfinite(dt)) return fail(CFDGB_EINVAL, "dt must be positive");
   c->cfg.dt = dt;
   drop_step_graph(c);  // a graph holds the CFL rule's dt bound, taken from dt
-  c->g.div2 = division_twice(c) ? 1 : 0;  // dt is a divisor too
+  c->g.div2t = dt_twice(c) ? 1 : 0;  // dt is a divisor too
   if (c->cfg.time_order == 3 && c->ss)  // the constant-step history is of the old dt
     CK(cudaMemsetAsync(&c->ss->hist, 0, 2 * sizeof(int), c->stream));
   // the step kernels read dt from the step scalars

@@ -17,6 +17,7 @@
 namespace cfdgb {
 
 constexpr int kBlock = 256;  // threads per block of every grid-stride kernel
+constexpr int kConvdiffBlocks = 4;  // blocks per SM of k_convdiff_quick, at most (sizes the partials)
 
 // Geometry as the kernels see it.  Padded indices i,j,k run over [0, nx+4); interior
 // cells are [2, n+2).  Compact rows enumerate the interior with k fastest.
@@ -59,7 +60,15 @@ struct Geo {
   // per-index reciprocals RN(1/D), RN(1/Ds) of the metrics (padded lengths) for div_by, and
   // the DFIB face-fraction factors (Ds * 0.5) / D of updateUandF.hpp, each one IEEE division
   const double *rDx, *rDy, *rDz, *rDxs, *rDys, *rDzs, *hfx, *hfy, *hfz;
-  int div2;  // 1: div_by applies its correction twice (a divisor lacks the certificate)
+  // QUICK's factors at the upper face of index I, four rows per axis (padded lengths): the
+  // component's own axis for flow up and down, 0.125 D[I+1]^2 / Ds[I] and / Ds[I+1], and
+  // across, 0.125 Ds[I]^2 / D[I] and / D[I+1], each one IEEE division
+  const double *qkx, *qky, *qkz;
+  // 1: div_by applies its correction twice: div2 for the metrics (one of them lacks the
+  // certificate), div2t for dt (it lacks it, or an adaptive rule chooses it on the device).
+  // Apart, because a dt such as 0.002 without the certificate made every division by a
+  // certified spacing take five FP64 instructions instead of three
+  int div2, div2t;
   int uni;   // 1: every metric array holds one value (a uniform grid): per-axis factors hoist
 };
 
@@ -76,6 +85,19 @@ inline int k_block_width(int nz) {
     if (idle(nz, c) < idle(nz, w)) w = c;
   return w;
 }
+
+// Tests of a double on the integer pipe: a comparison with a floating-point zero, or a mask and
+// shift of its 64 bits that the compiler recognises as one, runs on the FP64 pipe (64 cycles a
+// warp and scheduler); the two halves taken apart do not.  positive: a > 0, also for a NaN
+// without the sign bit.
+__device__ __forceinline__ bool is_zero(double a) {
+  return ((__double2hiint(a) & 0x7fffffff) | __double2loint(a)) == 0;
+}
+__device__ __forceinline__ bool positive(double a) {
+  const int h = __double2hiint(a);
+  return h > 0 || (h == 0 && __double2loint(a) != 0);
+}
+__device__ __forceinline__ bool finite_int(double a) { return (__double2hiint(a) & 0x7fffffff) < 0x7ff00000; }
 
 // a / b correctly rounded, given y = RN(1/b), by Markstein's FMA correction.  Markstein's
 // theorem (P. Markstein, IBM J. Res. Develop. 34(1), 1990; J.-M. Muller et al., Handbook of
@@ -97,7 +119,7 @@ __device__ __forceinline__ double div_by(double a, double b, double y, bool two)
     r = fma(-q1, b, a);
     q1 = fma(r, y, q1);
   }
-  return a == 0.0 ? q : q1;
+  return is_zero(a) ? q : q1;
 }
 
 // Host: whether b's reciprocal y = RN(1/b) carries Markstein's certificate |b y - 1| < 2^-54

@@ -10,6 +10,8 @@ namespace cfdgb {
 // step_exact.cu (bit-exact FP64, reference operation order)
 // scheme: a cfdgb_scheme value; nut (compact, may be null): eddy viscosity added to nu.
 // Fused CFL reduction into sc.ss (none when sc.ss is null); dt from sc.dtp when set.
+// convdiff_prepare: the kernel attributes it needs, once per device before the first launch
+bool convdiff_prepare();
 void launch_convdiff_exact(cudaStream_t s, int nblk, const Geo &g, int scheme, double dt, double nu,
                            const double *nut, const double *u, const double *v, const double *w, double *us,
                            double *vs, double *ws, const StepCtl &sc);

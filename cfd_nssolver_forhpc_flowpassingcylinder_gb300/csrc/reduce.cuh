@@ -44,7 +44,7 @@ __device__ __forceinline__ double warp_sum1(double v) {
     if (t == 0) return 0.0;
     return __longlong_as_double(__double_as_longlong((double)t) + ((long long)((int)em - 1075 - kSumGuard) << 52));
   }
-  if (!__any_sync(0xffffffffu, (b << 1) != 0)) return 0.0;  // drag sums away from the body
+  if (!__any_sync(0xffffffffu, !is_zero(v))) return 0.0;  // drag sums away from the body
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   return v;
@@ -115,59 +115,66 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double *part, unsigned
   return true;
 }
 
-// Grid-wide maxima of NV values per thread, with the same last-block pattern as grid_sum
-// (minima: pass the negated values).  Maxima are exact, so the result does not depend on
-// the order either.
+// The larger of two doubles on the integer pipe (an FP64 comparison takes the FP64 pipe, see
+// warp_sum1): ordered 64-bit keys, a NaN never taken over a number (as fmax).
+__device__ __forceinline__ double max_int(double a, double b) {
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  const long long kx = x ^ ((x >> 63) & 0x7fffffffffffffffLL), ky = y ^ ((y >> 63) & 0x7fffffffffffffffLL);
+  const bool nan = (__double2hiint(b) & 0x7fffffff) >= 0x7ff80000;
+  return ky > kx && !nan ? b : a;
+}
+
+// Grid-wide maxima of NV values per thread (no NaN among them), with the same last-block
+// pattern as grid_sum (minima: pass the negated values).  Maxima are exact, so the result
+// does not depend on the order either.
 template <int NV>
-__device__ __forceinline__ bool grid_max(double (&v)[NV], double *part, unsigned *ticket, double (&out)[NV]) {
-  __shared__ double sh[NV][kBlock / 32];
-  __shared__ bool last;
-  __shared__ double res[NV];
+__device__ __forceinline__ void block_max(double (&v)[NV], double (*sh)[32]) {
   const int t = lin_tid(), lane = t & 31, wid = t >> 5;
+  const int nw = (int)(blockDim.x * blockDim.y * blockDim.z) >> 5;
 #pragma unroll
   for (int q = 0; q < NV; ++q)
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v[q] = fmax(v[q], __shfl_down_sync(0xffffffffu, v[q], off));
+    for (int off = 16; off > 0; off >>= 1) v[q] = max_int(v[q], __shfl_xor_sync(0xffffffffu, v[q], off));
+  __syncthreads();  // sh may still be read by a previous call
   if (lane == 0)
 #pragma unroll
     for (int q = 0; q < NV; ++q) sh[q][wid] = v[q];
   __syncthreads();
-  const int G = nblocks();
-  if (t == 0) {
+  if (wid == 0)
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
-      double m = sh[q][0];
-      for (int w = 1; w < kBlock / 32; ++w) m = fmax(m, sh[q][w]);
-      part[q * G + lin_bid()] = m;
+      v[q] = lane < nw ? sh[q][lane] : -INFINITY;
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) v[q] = max_int(v[q], __shfl_xor_sync(0xffffffffu, v[q], off));
     }
+}
+template <int NV>
+__device__ __forceinline__ bool grid_max(double (&v)[NV], double *part, unsigned *ticket, double (&out)[NV]) {
+  __shared__ double sh[NV][32];
+  __shared__ bool last;
+  __shared__ double res[NV];
+  block_max<NV>(v, sh);
+  const int G = nblocks(), t = lin_tid();
+  if (t == 0) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) part[q * G + lin_bid()] = v[q];
     __threadfence();
     last = (atomicAdd(ticket, 1u) == (unsigned)(G - 1));
   }
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  // the partials, strided over the block's threads, then over its warps (every thread of
-  // the block takes part: a one-thread loop over the partials held the grid for a long tail)
   const int nt = (int)(blockDim.x * blockDim.y * blockDim.z);
 #pragma unroll
   for (int q = 0; q < NV; ++q) {
     double m = -INFINITY;
-    for (int b = t; b < G; b += nt) m = fmax(m, __ldcg(part + q * G + b));
-    for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, off));
+    for (int b = t; b < G; b += nt) m = max_int(m, __ldcg(part + q * G + b));
     v[q] = m;
   }
-  __syncthreads();  // sh is reused below
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < NV; ++q) sh[q][wid] = v[q];
-  __syncthreads();
+  block_max<NV>(v, sh);
   if (t == 0) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double m = sh[q][0];
-      for (int w = 1; w < nt / 32; ++w) m = fmax(m, sh[q][w]);
-      res[q] = m;
-    }
+    for (int q = 0; q < NV; ++q) res[q] = v[q];
     *ticket = 0u;
   }
   __syncthreads();

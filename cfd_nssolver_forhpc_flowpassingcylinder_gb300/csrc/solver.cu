@@ -1723,9 +1723,11 @@ __global__ void __launch_bounds__(kBlock) k_sum32(Geo g, const float *__restrict
 // dropped.  e - mean in FP32, widened exactly, scaled by 2^k and signed in its bits: one
 // FP64 addition a cell.  Pointwise, quads as k_sum32.
 __device__ __forceinline__ double correction(float e, float m, long long shift, long long sign) {
-  const long long d = __double_as_longlong(f2d_int(e - m));
-  // a zero stays zero; any other value is an FP32 normal, far from the FP64 limits
-  return __longlong_as_double((d << 1) == 0 ? 0LL : (d + shift) ^ sign);
+  const float f = e - m;
+  const long long d = __double_as_longlong(f2d_int(f));
+  // a zero stays zero (tested in FP32: the test of d is one of the FP64 pipe's); any other
+  // value is an FP32 normal, far from the FP64 limits
+  return __longlong_as_double((__float_as_uint(f) & 0x7f800000u) == 0u ? 0LL : (d + shift) ^ sign);
 }
 __global__ void __launch_bounds__(kBlock) k_correct64(Geo g, double *__restrict__ x, const float *__restrict__ e,
                                                        int k, int neg, const StepScal *ss) {

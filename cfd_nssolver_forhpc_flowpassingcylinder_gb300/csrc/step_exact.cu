@@ -248,14 +248,224 @@ __global__ void __launch_bounds__(kBlock, 2) k_convdiff_exact(Geo g, double dt_a
   if (sc.ss) cfl_finish(cfl, dt, sc);
 }
 
+// The same for QUICK, with every face computed once.  The kernel is bound by the FP64 pipe
+// (one warp instruction per 64 cycles and scheduler, idle lanes included), so what counts is
+// the number of FP64 instructions a cell: the per-cell form above evaluates both faces of each
+// axis (every face twice), divides every difference up to four times and forms the QUICK
+// factors by division, about 1050 instructions; here
+//   - a block of (tk + 2) x (rows + 1) threads marches along x, a thread owning one (j, k)
+//     column: the x face of plane i is kept in registers as the lower face of plane i + 1;
+//   - the differences and the upper faces along y and z go through shared memory to the
+//     neighbouring threads (two buffers each, one barrier a plane: the next plane's
+//     differences are formed before the barrier that publishes this plane's faces).  The first
+//     row and the first lane of a row hold no cell and compute the faces below the tile, the
+//     last lane the difference above it;
+//   - the factors 0.125 D^2 / Ds come from tables (Geo::qk*, each IEEE division's result);
+// about 215 instructions a cell.  Every value is formed by the reference's operations in its
+// order, so the results are the same bits (a face's value, velocity and flux are the same
+// expression from both of its cells).  512x256x64: 16.6 -> 4.9 ms (85 % of the FP64 pipe).
+struct QuickPlan {
+  int tk, rows, xc;      // cells of a tile along k and j, planes a block marches over
+  int threads, gx, gy, gz;
+};
+
+// The upper QUICK face's flux on one axis: the value fc and the next one fp, the differences
+// s0 = d0 - dm around the value and s1 around the next one, the factors of the two flow
+// directions and the face velocity vel (own axis: the face's own mean).
+template <bool OWN>
+__device__ __forceinline__ double quick_flux(double mean, double s0, double s1, double kp, double kn, double vel) {
+  const bool up = positive(vel);
+  const double P = mean - (up ? kp : kn) * (up ? s0 : s1);
+  return OWN ? P * P : P * vel;
+}
+
+template <bool AB, bool TWO>
+__global__ void __launch_bounds__(512, 1) k_convdiff_quick(Geo g, QuickPlan pl, double dt_arg, double nu0,
+                                                           const double *__restrict__ nut,
+                                                           const double *__restrict__ u,
+                                                           const double *__restrict__ v,
+                                                           const double *__restrict__ w, double *__restrict__ us,
+                                                           double *__restrict__ vs, double *__restrict__ ws,
+                                                           StepCtl sc) {
+  extern __shared__ double qsm[];
+  const int T = blockDim.x, t = threadIdx.x, W = pl.tk + 2;
+  double *sd = qsm + t, *sf = qsm + 12 * T + t;  // differences and fluxes: [buffer][y, z of u, v, w][thread]
+  const double dt = step_dt(sc, dt_arg);
+  CflAcc cfl;
+  AbStep ab;
+  if (AB) ab.init(sc, dt);
+  const int tr = t / W, tc = t - tr * W;
+  const int j = 1 + blockIdx.y * pl.rows + tr, k = 1 + blockIdx.x * pl.tk + tc;
+  const bool row = tr <= pl.rows && j <= g.ny - 3;
+  const bool in = row && tc <= pl.tk && k <= g.nz - 3;
+  const bool yf = in && tc > 0, zf = in && tr > 0, cell = yf && zf;
+  const bool zd = row && tr > 0 && k <= g.nz - 2;  // the difference to the next cell along k
+  const bool jtop = tr == pl.rows || j == g.ny - 3;  // no thread above holds the next difference
+  const int sx = (int)g.sx, sy = (int)g.sy;  // offsets within a plane or two: below 2^31 entries
+  const int i0 = 2 + blockIdx.z * pl.xc, i1 = min(g.nx - 2, i0 + pl.xc);
+  const int nx = g.nx, ny = g.ny, nz = g.nz;
+  const double *qx = g.qkx, *qy = g.qky, *qz = g.qkz;  // rows: own axis up, down; across up, down
+  const int jj = row ? j : 2, kk = in || zd ? k : 2;
+  long long c = (long long)i0 * g.sx + (long long)jj * sy + kk;
+  const double hy = g.hfy[jj], hz = g.hfz[kk];
+  const double nudt0 = nu0 * dt;
+  auto over = [](double a, const double *D, const double *rD, int q) { return div_by(a, D[q], rD[q], TWO); };
+  const double *const ph[3] = {u, v, w};
+  // the spacings that divide a difference (to the next value) along an axis, own or across
+  const double *const Sx[3] = {g.Dx + 1, g.Dxs, g.Dxs}, *const rSx[3] = {g.rDx + 1, g.rDxs, g.rDxs};
+  const double *const Sy[3] = {g.Dys, g.Dy + 1, g.Dys}, *const rSy[3] = {g.rDys, g.rDy + 1, g.rDys};
+  const double *const Sz[3] = {g.Dzs, g.Dzs, g.Dz + 1}, *const rSz[3] = {g.rDzs, g.rDzs, g.rDz + 1};
+  // differences of plane cc along y and z, into buffer s
+  auto differences = [&](const double (&f)[3], long long cc, double *s) {
+    if (yf) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) s[a * T] = over(ph[a][cc + sy] - f[a], Sy[a], rSy[a], j);
+    }
+    if (zd) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) s[(3 + a) * T] = over(ph[a][cc + 1] - f[a], Sz[a], rSz[a], k);
+    }
+  };
+  // x faces: the value, the difference and the flux of the plane before, per component
+  double fu[3] = {0, 0, 0}, dx[3] = {0, 0, 0}, fx[3] = {0, 0, 0};
+  if (in || zd) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) fu[a] = ph[a][c];
+  }
+  if (cell) {  // the face below the first plane
+    const long long m = c - sx;
+    const int i = i0 - 1;
+    const double um = u[m];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double *f = ph[a] + m;
+      const double f0 = f[0], d0 = over(fu[a] - f0, Sx[a], rSx[a], i);
+      const double s0 = d0 - over(f0 - f[-sx], Sx[a], rSx[a], i - 1);
+      const double s1 = over(f[2 * sx] - fu[a], Sx[a], rSx[a], i + 1) - d0;
+      const double mean = 0.5 * (f0 + fu[a]), vel = a == 1 ? um + (u[m + sy] - um) * hy : um + (u[m + 1] - um) * hz;
+      fx[a] = a == 0 ? quick_flux<true>(mean, s0, s1, qx[i], qx[nx + i], mean)
+                     : quick_flux<false>(mean, s0, s1, qx[2 * nx + i], qx[3 * nx + i], vel);
+      dx[a] = d0;
+    }
+  }
+  differences(fu, c, sd);
+  __syncthreads();
+  for (int i = i0; i < i1; ++i, c += sx) {
+    double fn[3] = {0, 0, 0}, sy0[3], sz0[3];  // next plane's values; second differences along y and z
+    if (in || zd) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) fn[a] = ph[a][c + sx];
+    }
+    const double hx = g.hfx[i];
+    if (yf) {
+      const double vx = fu[1] + (fn[1] - fu[1]) * hx, vz = fu[1] + (v[c + 1] - fu[1]) * hz;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double fp = ph[a][c + sy], d0 = sd[a * T];
+        const double dm = tr > 0 ? sd[a * T - W] : over(fu[a] - ph[a][c - sy], Sy[a], rSy[a], j - 1);
+        const double dp = !jtop ? sd[a * T + W] : over(ph[a][c + 2 * sy] - fp, Sy[a], rSy[a], j + 1);
+        const double mean = 0.5 * (fu[a] + fp);
+        sy0[a] = d0 - dm;
+        sf[a * T] = a == 1 ? quick_flux<true>(mean, sy0[a], dp - d0, qy[j], qy[ny + j], mean)
+                           : quick_flux<false>(mean, sy0[a], dp - d0, qy[2 * ny + j], qy[3 * ny + j], a == 0 ? vx : vz);
+      }
+    }
+    if (zf) {
+      const double wx = fu[2] + (fn[2] - fu[2]) * hx, wy = fu[2] + (w[c + sy] - fu[2]) * hy;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const double fp = ph[a][c + 1], d0 = sd[(3 + a) * T], dp = sd[(3 + a) * T + 1];
+        const double dm = tc > 0 ? sd[(3 + a) * T - 1] : over(fu[a] - ph[a][c - 1], Sz[a], rSz[a], k - 1);
+        const double mean = 0.5 * (fu[a] + fp);
+        sz0[a] = d0 - dm;
+        sf[(3 + a) * T] =
+            a == 2 ? quick_flux<true>(mean, sz0[a], dp - d0, qz[k], qz[nz + k], mean)
+                   : quick_flux<false>(mean, sz0[a], dp - d0, qz[2 * nz + k], qz[3 * nz + k], a == 0 ? wx : wy);
+      }
+    }
+    double *const so = qsm + t + (((i - i0) & 1) ? 0 : 6 * T);  // the other buffer of differences
+    if (i + 1 < i1) differences(fn, c + sx, so);
+    __syncthreads();
+    if (cell) {
+      double nudt = nudt0;
+      if (nut) nudt = (nu0 + nut[((long long)(i - 2) * g.nyc + (j - 2)) * g.nzc + (k - 2)]) * dt;
+      double ccfl = 0.0;
+      const double uy = fu[0] + (u[c + sy] - fu[0]) * hy, uz = fu[0] + (u[c + 1] - fu[0]) * hz;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        // the x face; its third difference only in warps with flow from that side
+        const double d0 = over(fn[a] - fu[a], Sx[a], rSx[a], i), s0 = d0 - dx[a];
+        const double mean = 0.5 * (fu[a] + fn[a]), vel = a == 0 ? mean : a == 1 ? uy : uz;
+        double s1 = s0;
+        if (__any_sync(__activemask(), !positive(vel)))
+          s1 = over(ph[a][c + 2 * sx] - fn[a], Sx[a], rSx[a], i + 1) - d0;
+        const double F = a == 0 ? quick_flux<true>(mean, s0, s1, qx[i], qx[nx + i], vel)
+                                : quick_flux<false>(mean, s0, s1, qx[2 * nx + i], qx[3 * nx + i], vel);
+        const bool on = a == 0 ? i < nx - 3 : a == 1 ? j < ny - 3 : k < nz - 3 + g.pz;
+        if (on) {
+          // the spacings between the component's own faces, per axis
+          const double *ax = a == 0 ? g.Dxs : g.Dx, *rax = a == 0 ? g.rDxs : g.rDx;
+          const double *ay = a == 1 ? g.Dys : g.Dy, *ray = a == 1 ? g.rDys : g.rDy;
+          const double *az = a == 2 ? g.Dzs : g.Dz, *raz = a == 2 ? g.rDzs : g.rDz;
+          const double convection = -dt * (over(F - fx[a], ax, rax, i) + over(sf[a * T] - sf[a * T - W], ay, ray, j) +
+                                           over(sf[(3 + a) * T] - sf[(3 + a) * T - 1], az, raz, k));
+          const double difussion =
+              nudt * (over(s0, ax, rax, i) + over(sy0[a], ay, ray, j) + over(sz0[a], az, raz, k));
+          const double r = AB ? ab.value(a, c, fu[a], convection, difussion) : fu[a] + convection + difussion;
+          (a == 0 ? us : a == 1 ? vs : ws)[c] = r;
+          ccfl += a == 0 ? over(r, g.Dxs, g.rDxs, i) : a == 1 ? over(r, g.Dys, g.rDys, j) : over(r, g.Dzs, g.rDzs, k);
+          cfl.comp(a, r);
+        }
+        dx[a] = d0;
+        fx[a] = F;
+      }
+      cfl.cell(ccfl);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) fu[a] = fn[a];
+    sd = so;
+    sf = qsm + 12 * T + t + (((i - i0) & 1) ? 0 : 6 * T);
+  }
+  if (sc.ss) cfl_finish(cfl, dt, sc);
+}
+
+// Tiles of k_convdiff_quick: whole k lines up to 126 cells, as many rows as 512 threads hold,
+// and the number of x chunks (one plane's face of extra work each) that costs least in whole
+// waves of one block a multiprocessor.
+static QuickPlan quick_plan(const Geo &g, int nsm) {
+  QuickPlan p;
+  const int kt = (g.nzc + 125) / 126;
+  p.tk = (g.nzc + kt - 1) / kt;
+  const int rows = std::min(g.nyc, 512 / (p.tk + 2) - 1);
+  p.gy = (g.nyc + rows - 1) / rows;
+  p.rows = (g.nyc + p.gy - 1) / p.gy;
+  p.gx = (g.nzc + p.tk - 1) / p.tk;
+  p.threads = ((p.tk + 2) * (p.rows + 1) + 31) / 32 * 32;
+  double best = 1e300;
+  p.xc = g.nxc;
+  const int most = std::min(g.nxc, std::max(1, kConvdiffBlocks * nsm / (p.gx * p.gy)));
+  for (int n = 1; n <= most; ++n) {
+    const int xc = (g.nxc + n - 1) / n, nb = (g.nxc + xc - 1) / xc;
+    const double cost = std::ceil((double)nb * p.gx * p.gy / nsm) * (xc + 0.4);
+    if (cost < best) {
+      best = cost;
+      p.xc = xc;
+    }
+  }
+  p.gz = (g.nxc + p.xc - 1) / p.xc;
+  return p;
+}
+
 // inc/matrix/b_matrix.hpp:35-98: b = -(jp)(1/dt) div(u*), one-sided differences
+// TWO: div_by's double correction (a template, as the branch would be predicated: two more FP64
+// instructions a division)
+template <bool TWO>
 __global__ void __launch_bounds__(kBlock) k_rhs_exact(Geo g, double dt_arg, const double *dtp,
                                                       const double *__restrict__ us,
                                                       const double *__restrict__ vs,
                                                       const double *__restrict__ ws, int jacobi,
                                                       Stencil<double> st, double *__restrict__ b) {
   const double ddt = 1.0 / (dtp ? *dtp : dt_arg);
-  const bool two = g.div2 != 0;
   for (long long row = blockIdx.x * (long long)kBlock + threadIdx.x; row < g.ncell;
        row += (long long)gridDim.x * kBlock) {
     int i, j, k;
@@ -263,9 +473,9 @@ __global__ void __launch_bounds__(kBlock) k_rhs_exact(Geo g, double dt_arg, cons
     const long long ic = pidx(g, i, j, k);
     // periodic z: the bottom face of the first cell is the top face nz-3
     const long long zb = (g.pz && k == 2) ? ic + g.nzc - 1 : ic - 1;
-    const double div = div_by(us[ic] - us[ic - g.sx], g.Dx[i], g.rDx[i], two) +
-                       div_by(vs[ic] - vs[ic - g.sy], g.Dy[j], g.rDy[j], two) +
-                       div_by(ws[ic] - ws[zb], g.Dz[k], g.rDz[k], two);
+    const double div = div_by(us[ic] - us[ic - g.sx], g.Dx[i], g.rDx[i], TWO) +
+                       div_by(vs[ic] - vs[ic - g.sy], g.Dy[j], g.rDy[j], TWO) +
+                       div_by(ws[ic] - ws[zb], g.Dz[k], g.rDz[k], TWO);
     if (jacobi) {
       b[row] = -row_jp(g, st, i - 2, j - 2, k - 2, row) * ddt * div;
     } else {
@@ -374,6 +584,26 @@ __global__ void __launch_bounds__(kBlock) k_transform(Geo g, const double *__res
 // virtualF_Int (inc/dfib/virtualForceIntergrator.hpp:67-90) and, in the time step, with
 // the part of copyVel (inc/source/copyVel.hpp:4) that matters: the faces update_UandF
 // never writes keep the initial values (ui, vi, wi) they hold in the reference's T3.
+// One face: T2 = u* - dt dp / Ds, the solid fraction e between the two cells, the forced
+// value ec uS + (1 - e) T2 with uS = 0 and the force (nu3 - T2) / dt.  Away from the body
+// (eta zero on both sides, all but a few per mille of the faces) e is 0, the forced value T2
+// (a negative zero added to ec uS becomes positive) and the force zero: those faces skip the
+// FP64 work, the tests on the integer pipe.  A T2 that is not finite takes the general form, so
+// that the force carries it to the drag's NaN flag.
+__device__ __forceinline__ double uf_face(double T2, double ec, double en, double hf, double dt, double rdt, bool two,
+                                          double &force) {
+  if (is_zero(ec) && is_zero(en) && finite_int(T2)) {
+    force = 0.0;
+    return is_zero(T2) ? 0.0 : T2;
+  }
+  const double e = ec + (en - ec) * hf;
+  const double n3 = ec * 0.0 + (1.0 - e) * T2;
+  force = div_by(n3 - T2, dt, rdt, two);
+  return n3;
+}
+
+// 512x256x64: 1.06 -> 0.40 ms (FP64 pipe)
+template <bool TWO>
 __global__ void __launch_bounds__(kBlock) k_update_uf_exact(
     Geo g, double dt_arg, const double *dtp, int in_step /* step_end mode */, double lz, const double *__restrict__ eta,
     const double *__restrict__ p, const double *__restrict__ us, const double *__restrict__ vs,
@@ -381,9 +611,8 @@ __global__ void __launch_bounds__(kBlock) k_update_uf_exact(
     double *__restrict__ f, const double *__restrict__ ui, const double *__restrict__ vi,
     const double *__restrict__ wi, double *part, StepScal *ss) {
   const double dt = dtp ? *dtp : dt_arg;
-  const bool two = g.div2 != 0;
+  const bool twot = g.div2t != 0;
   const long long tot = (long long)g.nx * g.ny * g.nz;
-  const double uS = 0.0, vS = 0.0, wS = 0.0;
   const double rdt = 1.0 / dt;
   double acc[2] = {0.0, 0.0};
   for (long long row = blockIdx.x * (long long)kBlock + threadIdx.x; row < g.ncell;
@@ -391,41 +620,36 @@ __global__ void __launch_bounds__(kBlock) k_update_uf_exact(
     int i, j, k;
     row_ijk(g, row, i, j, k);
     const long long ic = pidx(g, i, j, k);
-    const double vol = g.Dx[i] * g.Dy[j] * g.Dz[k];
-    const double ec = eta[ic];
+    const double ec = eta[ic], pc = p[ic];
+    double fx = 0.0, fy = 0.0, fz = 0.0;
     if (i < g.nx - 3) {
       const long long icP = ic + g.sx;
-      const double T2u = us[ic] - div_by(dt * (p[icP] - p[ic]), g.Dxs[i], g.rDxs[i], two);
-      const double e = ec + (eta[icP] - ec) * g.hfx[i];
-      const double nu3 = ec * uS + (1.0 - e) * T2u;
-      const double fx = div_by(nu3 - T2u, dt, rdt, two);
-      u3[ic] = nu3;
+      const double T2u = us[ic] - div_by(dt * (p[icP] - pc), g.Dxs[i], g.rDxs[i], TWO);
+      u3[ic] = uf_face(T2u, ec, eta[icP], g.hfx[i], dt, rdt, twot, fx);
       if (f) f[ic] = fx;
-      acc[0] += fx * vol;
     } else if (ui) {
       u3[ic] = ui[ic];
     }
     if (j < g.ny - 3) {
       const long long icP = ic + g.sy;
-      const double T2v = vs[ic] - div_by(dt * (p[icP] - p[ic]), g.Dys[j], g.rDys[j], two);
-      const double e = ec + (eta[icP] - ec) * g.hfy[j];
-      const double nv3 = ec * vS + (1.0 - e) * T2v;
-      const double fy = div_by(nv3 - T2v, dt, rdt, two);
-      v3[ic] = nv3;
+      const double T2v = vs[ic] - div_by(dt * (p[icP] - pc), g.Dys[j], g.rDys[j], TWO);
+      v3[ic] = uf_face(T2v, ec, eta[icP], g.hfy[j], dt, rdt, twot, fy);
       if (f) f[ic + tot] = fy;
-      acc[1] += fy * vol;
     } else if (vi) {
       v3[ic] = vi[ic];
     }
     if (k < g.nz - 3 + g.pz) {  // periodic z: the top face, its upper cell the first one
       const long long icP = (g.pz && k == g.nz - 3) ? ic - (g.nzc - 1) : ic + 1;
-      const double T2w = ws[ic] - div_by(dt * (p[icP] - p[ic]), g.Dzs[k], g.rDzs[k], two);
-      const double e = ec + (eta[icP] - ec) * g.hfz[k];
-      const double nw3 = ec * wS + (1.0 - e) * T2w;
-      w3[ic] = nw3;
-      if (f) f[ic + 2 * tot] = div_by(nw3 - T2w, dt, rdt, two);
+      const double T2w = ws[ic] - div_by(dt * (p[icP] - pc), g.Dzs[k], g.rDzs[k], TWO);
+      w3[ic] = uf_face(T2w, ec, eta[icP], g.hfz[k], dt, rdt, twot, fz);
+      if (f) f[ic + 2 * tot] = fz;
     } else if (wi) {
       w3[ic] = wi[ic];
+    }
+    if (!is_zero(fx) || !is_zero(fy)) {
+      const double vol = g.Dx[i] * g.Dy[j] * g.Dz[k];
+      acc[0] += fx * vol;
+      acc[1] += fy * vol;
     }
   }
   double out[2];
@@ -722,6 +946,15 @@ __global__ void __launch_bounds__(kBlock) k_eta_extrude(Geo g, double *__restric
 }
 
 // ---- launchers ----
+constexpr size_t kQuickSmem = 24 * sizeof(double);  // shared memory of k_convdiff_quick per thread
+bool convdiff_prepare() {
+  const int most = (int)kQuickSmem * 512;  // above the default 48 KB
+  const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  return cudaFuncSetAttribute(k_convdiff_quick<false, false>, a, most) == cudaSuccess &&
+         cudaFuncSetAttribute(k_convdiff_quick<false, true>, a, most) == cudaSuccess &&
+         cudaFuncSetAttribute(k_convdiff_quick<true, false>, a, most) == cudaSuccess &&
+         cudaFuncSetAttribute(k_convdiff_quick<true, true>, a, most) == cudaSuccess;
+}
 template <bool AB>
 static void convdiff_exact(cudaStream_t s, int nblk, const Geo &g, int scheme, double dt, double nu, const double *nut,
                            const double *u, const double *v, const double *w, double *us, double *vs, double *ws,
@@ -730,8 +963,18 @@ static void convdiff_exact(cudaStream_t s, int nblk, const Geo &g, int scheme, d
     k_convdiff_exact<CFDGB_LUD, AB><<<nblk, kBlock, 0, s>>>(g, dt, nu, nut, u, v, w, us, vs, ws, sc);
   else if (scheme == CFDGB_UD)
     k_convdiff_exact<CFDGB_UD, AB><<<nblk, kBlock, 0, s>>>(g, dt, nu, nut, u, v, w, us, vs, ws, sc);
-  else
-    k_convdiff_exact<CFDGB_QUICK, AB><<<nblk, kBlock, 0, s>>>(g, dt, nu, nut, u, v, w, us, vs, ws, sc);
+  else {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const QuickPlan pl = quick_plan(g, nsm);
+    const size_t smem = kQuickSmem * (size_t)pl.threads;
+    const dim3 grid(pl.gx, pl.gy, pl.gz);
+    if (g.div2)
+      k_convdiff_quick<AB, true><<<grid, pl.threads, smem, s>>>(g, pl, dt, nu, nut, u, v, w, us, vs, ws, sc);
+    else
+      k_convdiff_quick<AB, false><<<grid, pl.threads, smem, s>>>(g, pl, dt, nu, nut, u, v, w, us, vs, ws, sc);
+  }
 }
 void launch_convdiff_exact(cudaStream_t s, int nblk, const Geo &g, int scheme, double dt, double nu,
                            const double *nut, const double *u, const double *v, const double *w, double *us,
@@ -747,7 +990,7 @@ void launch_smagorinsky(cudaStream_t s, int nblk, const Geo &g, const double *l2
 }
 void launch_rhs_exact(cudaStream_t s, int nblk, const Geo &g, double dt, const double *dtp, const double *us,
                       const double *vs, const double *ws, int jacobi, const Stencil<double> &st, double *b) {
-  k_rhs_exact<<<nblk, kBlock, 0, s>>>(g, dt, dtp, us, vs, ws, jacobi, st, b);
+  (g.div2 ? k_rhs_exact<true> : k_rhs_exact<false>)<<<nblk, kBlock, 0, s>>>(g, dt, dtp, us, vs, ws, jacobi, st, b);
 }
 void launch_spmv_exact(cudaStream_t s, int nblk, const Geo &g, const Stencil<double> &st, const double *x,
                        double *y) {
@@ -775,8 +1018,8 @@ void launch_update_uf_exact(cudaStream_t s, int nblk, const Geo &g, double dt, c
                             double lz, const double *eta, const double *p, const double *us, const double *vs,
                             const double *ws, double *u3, double *v3, double *w3, double *f, const double *ui,
                             const double *vi, const double *wi, double *part, StepScal *ss) {
-  k_update_uf_exact<<<nblk, kBlock, 0, s>>>(g, dt, dtp, step_mode, lz, eta, p, us, vs, ws, u3, v3, w3, f, ui, vi,
-                                            wi, part, ss);
+  (g.div2 ? k_update_uf_exact<true> : k_update_uf_exact<false>)<<<nblk, kBlock, 0, s>>>(
+      g, dt, dtp, step_mode, lz, eta, p, us, vs, ws, u3, v3, w3, f, ui, vi, wi, part, ss);
 }
 void launch_bc(cudaStream_t s, const Geo &g, double *u, double *v, double *w, double *p, double *us,
                double *vs, double *ws, int do_main, const double *inlet, int conv, double *part, StepScal *ss,

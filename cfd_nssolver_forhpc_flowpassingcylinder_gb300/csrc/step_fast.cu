@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kBlock) k_update_uf_fast(
     StepScal *ss) {
   const double dt = dtp ? *dtp : dt_arg;
   const double rdt = 1.0 / dt;
-  auto nonzero = [](double e) { return (__double_as_longlong(e) << 1) != 0; };  // +-0 is zero
+  auto nonzero = [](double e) { return !is_zero(e); };  // +-0 is zero
   // UNI: -dt / Ds per axis once per thread (a uniform grid: the same product at every index)
   double gx = 0.0, gy = 0.0, gz = 0.0;
   if (UNI) {

@@ -15,10 +15,10 @@ __device__ __forceinline__ double step_dt(const StepCtl &sc, double dt_arg) { re
 struct CflAcc {
   double m[7] = {-1e300, -1e10, -1e10, -1e10, -1e10, -1e10, -1e10};
   __device__ __forceinline__ void comp(int a, double x) {
-    m[1 + a] = fmax(m[1 + a], x);
-    m[4 + a] = fmax(m[4 + a], -x);
+    m[1 + a] = max_int(m[1 + a], x);
+    m[4 + a] = max_int(m[4 + a], __longlong_as_double(__double_as_longlong(x) ^ (1LL << 63)));  // -x
   }
-  __device__ __forceinline__ void cell(double c) { m[0] = fmax(m[0], c); }
+  __device__ __forceinline__ void cell(double c) { m[0] = max_int(m[0], c); }
 };
 
 // The next dt from this step's CFL extremes (thread 0 of the last block).
