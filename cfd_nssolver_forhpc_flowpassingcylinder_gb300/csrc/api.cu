@@ -497,7 +497,8 @@ int iter_kid(const cfdgb_ctx *c, bool fp32, int part) {
 // kernels one part launches (a V-cycle is many)
 int iter_part_launches(const cfdgb_ctx *c, bool fp32, int part) {
   const int k = iter_kid(c, fp32, part);
-  return k == K_MG ? mg_vcycle_launches(c->mg) : k == K_MG64 ? mg_vcycle_launches(c->mg64) : 1;
+  const int jac = c->cfg.solver == CFDGB_BICGSTAB_JACOBI;
+  return k == K_MG ? mg_vcycle_launches(c->mg, jac) : k == K_MG64 ? mg_vcycle_launches(c->mg64, jac) : 1;
 }
 // iterations per captured chunk: the preconditioned iteration is long and needs few
 int chunk_iters(const cfdgb_ctx *c, bool fp32) { return prec_iter(c, fp32) ? 2 : c->chunk_len; }
@@ -2001,7 +2002,7 @@ int adjoint_solve(cfdgb_ctx *c, const double *rhs, double tol, int *iters) {
     for (int m = 0; m < 8; ++m) {
       if (mg) {
         for (int part = 0; part < kPrecParts; ++part) {
-          L(c, kPrecKid64[part], part == 1 || part == 4 ? mg_vcycle_launches(c->mg64) : 1, [&] {
+          L(c, kPrecKid64[part], part == 1 || part == 4 ? mg_vcycle_launches(c->mg64, 0) : 1, [&] {
             if (part == 1) launch_mg_vcycle(c->stream, c->mg64, 0, (const double *)pv.p, pv.ph, c->sca);
             else if (part == 4) launch_mg_vcycle(c->stream, c->mg64, 0, (const double *)pv.s, pv.sh, c->sca);
             else launch_bicgp64_part(c->stream, part == 0 ? 0 : part == 2 ? 1 : part == 3 ? 2 : part == 5 ? 3 : 4,

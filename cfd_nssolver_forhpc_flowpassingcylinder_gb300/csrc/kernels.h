@@ -174,8 +174,8 @@ struct MgLevelT {
   int fx, fy, fz;          // cells of this level per cell of the next one, per axis (1, 2)
   T *x, *b;                // correction and right-hand side (levels >= 1)
   int bx, by, gx, gy, gz;  // launch geometry: bx along k, by along j, gz planes strided over i
-  int qgrid;               // 1: the quad smoother (FP32, nz % 4 == 0), 0: the scalar one
-  int qbx, qby, qgx, qgy, qgz;  // its launch: quads along x, rows along y, planes strided over z
+  int qgrid;               // 1: the quad smoother (FP32, nz % 4 == 0) or the pair passes (FP64, nz even), 0: neither
+  int qbx, qby, qgx, qgy, qgz;  // its launch: quads (FP64: pairs) along x, rows along y, planes strided over z
   int pz;                  // periodic z (every level; nz even or 1 on each)
   // 1: the level's V-cycle work runs as two marching kernels (k_mg_down4, k_mg_up4; FP32
   // quads, every axis halves, nz / 4 a power of two up to 16): a block of nz / 4 x (mty + 4)
@@ -208,7 +208,7 @@ bool mg_plan(int nx, int ny, int nz, double hx, double hy, double hz, int nsm, b
              bool pz = false);
 // kernels one V-cycle launches
 template <typename T>
-int mg_vcycle_launches(const MgPlanT<T> &mg);
+int mg_vcycle_launches(const MgPlanT<T> &mg, int jacobi);
 // the pseudo-inverse of the coarsest level's operator, row-major, when that level has at
 // most kMgDenseCells cells (the caller uploads it and sets mg.cinv)
 template <typename T>

@@ -418,6 +418,130 @@ __global__ void __launch_bounds__(kBlock) k_mg_prolong8(MgLevelT<T> F, MgLevelT<
   }
 }
 
+// ---- FP64 levels with an even nz (the FP64 hierarchy): one thread per pair of cells along k,
+// of which one has the pass's colour, so that no lane idles.  These passes are bound by the
+// FP64 pipe (one warp instruction per 64 cycles and scheduler, idle lanes included), so the
+// same V-cycle is formed with few FP64 operations:
+//   - a missing neighbour is a zero selected on the integer pipe, not a guarded addition;
+//   - Jacobi-scaled rows (b' = b / diag): x0 from zero is b' itself, so the first pass reads
+//     its colour-0 neighbours from b' and stores both colours, and later passes take
+//     b' + idg S instead of (diag b' + S) idg;
+//   - after the pre-smoothing the residual is zero on colour 1 and, on colour 0, just the
+//     weighted sum of the colour-1 neighbours (x0 = b / diag), so the restriction reads no b;
+//   - the prolongation is added on colour 0 only: the next pass overwrites colour 1.
+// About 19 FP64 instructions a cell and V-cycle against 85 (and half the lanes idle) in the
+// general kernels above, which the levels with an odd nz keep.  512x256x64: a V-cycle
+// 1.44 -> 0.44 ms.
+#define FOR_PAIRS(L)                                          \
+  const int kp = blockIdx.x * blockDim.x + threadIdx.x;       \
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;        \
+  const bool on_ = (kp < ((L).nz >> 1)) && (j < (L).ny);      \
+  for (int i = blockIdx.z; on_ && i < (L).nx; i += gridDim.z)
+
+// weighted sum of the neighbours' values (lnb: the three pair sums, then the weights)
+__device__ __forceinline__ double lnb64(const MgLevelT<double> &L, const double *x, int i, int j, int k, long long r,
+                                        double start) {
+  const long long sx = (long long)L.ny * L.nz;
+  const double xm = i > 0 ? x[r - sx] : 0.0, xp = i < L.nx - 1 ? x[r + sx] : 0.0;
+  const double ym = j > 0 ? x[r - L.nz] : 0.0, yp = j < L.ny - 1 ? x[r + L.nz] : 0.0;
+  const double zm = k > 0 ? x[r - 1] : (L.pz ? x[r + L.nz - 1] : 0.0);
+  const double zp = k < L.nz - 1 ? x[r + 1] : (L.pz ? x[r + 1 - L.nz] : 0.0);
+  return fma_rn(L.wz, zm + zp, fma_rn(L.wy, ym + yp, fma_rn(L.wx, xm + xp, start)));
+}
+
+// x = b / diag on colour 0 (from zero; unscaled rows)
+__global__ void __launch_bounds__(kBlock) k_mgp_scale(MgLevelT<double> L, const double *__restrict__ b,
+                                                      double *__restrict__ x, const SolverScal *sc) {
+  pdl_wait();
+  if (sc->done) return;
+  pdl_trigger();
+  FOR_PAIRS(L) {
+    const int k = 2 * kp + ((i + j) & 1);
+    const long long r = lrow(L, i, j, k);
+    x[r] = b[r] * linv(L, i, j, k);
+  }
+}
+
+// one colour from the other: x = (b + S) idg, or b' + idg S for Jacobi-scaled rows (JAC);
+// from_b: the other colour's values are b' and are stored too (the first pass on JAC rows)
+template <bool JAC>
+__global__ void __launch_bounds__(kBlock) k_mgp_colour(MgLevelT<double> L, int colour, int from_b,
+                                                       const double *__restrict__ b, double *x, const SolverScal *sc) {
+  pdl_wait();
+  if (sc->done) return;
+  pdl_trigger();
+  const double *nb = from_b ? b : x;
+  FOR_PAIRS(L) {
+    const int d = (i + j + colour) & 1, k = 2 * kp + d;
+    const long long r = lrow(L, i, j, k);
+    const double idg = linv(L, i, j, k);
+    x[r] = JAC ? fma_rn(lnb64(L, nb, i, j, k, r, 0.0), idg, b[r]) : lnb64(L, nb, i, j, k, r, b[r]) * idg;
+    if (from_b) x[r + 1 - 2 * d] = b[r + 1 - 2 * d];
+  }
+}
+
+// bc = average over the children of the residual: the colour-1 neighbours of the four
+// colour-0 children (every axis halves)
+__global__ void __launch_bounds__(kBlock) k_mgp_restrict(MgLevelT<double> F, MgLevelT<double> Cl,
+                                                         const double *__restrict__ x, double *__restrict__ bc,
+                                                         const SolverScal *sc) {
+  pdl_wait();
+  if (sc->done) return;
+  pdl_trigger();
+  const long long sx = (long long)F.ny * F.nz, sy = F.nz;
+  FOR_LEVEL(Cl) {
+    double a = 0.0, e = 0.0, f = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // children (0,0,0), (0,1,1), (1,0,1), (1,1,0)
+      const int da = q >> 1, de = q & 1, dc = da ^ de;
+      const int fi = 2 * i + da, fj = 2 * j + de, fk = 2 * k + dc;
+      const long long r = lrow(F, fi, fj, fk);
+      const double xm = fi > 0 ? x[r - sx] : 0.0, xp = fi < F.nx - 1 ? x[r + sx] : 0.0;
+      const double ym = fj > 0 ? x[r - sy] : 0.0, yp = fj < F.ny - 1 ? x[r + sy] : 0.0;
+      const double zm = fk > 0 ? x[r - 1] : (F.pz ? x[r + F.nz - 1] : 0.0);
+      const double zp = fk < F.nz - 1 ? x[r + 1] : (F.pz ? x[r + 1 - F.nz] : 0.0);
+      a = q == 0 ? xm + xp : a + (xm + xp);
+      e = q == 0 ? ym + yp : e + (ym + yp);
+      f = q == 0 ? zm + zp : f + (zm + zp);
+    }
+    bc[lrow(Cl, i, j, k)] = wsum(F, a, e, f) * 0.125;
+  }
+}
+
+// x += P xc on colour 0 (every axis halves): k_mg_prolong8's taps
+__global__ void __launch_bounds__(kBlock) k_mgp_prolong(MgLevelT<double> F, MgLevelT<double> Cl,
+                                                        const double *__restrict__ xc, double *__restrict__ x,
+                                                        const SolverScal *sc) {
+  pdl_wait();
+  if (sc->done) return;
+  pdl_trigger();
+  FOR_LEVEL(Cl) {
+    double cv[3][3][3];
+    const int ci[3] = {i > 0 ? i - 1 : i, i, i < Cl.nx - 1 ? i + 1 : i};
+    const int cj[3] = {j > 0 ? j - 1 : j, j, j < Cl.ny - 1 ? j + 1 : j};
+    const int ck[3] = {k > 0 ? k - 1 : (Cl.pz ? Cl.nz - 1 : k), k, k < Cl.nz - 1 ? k + 1 : (Cl.pz ? 0 : k)};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int e = 0; e < 3; ++e)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) cv[a][e][c] = xc[lrow(Cl, ci[a], cj[e], ck[c])];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int da = q >> 1, de = q & 1, dc = da ^ de;
+      const long long r = lrow(F, 2 * i + da, 2 * j + de, 2 * k + dc);
+      double v = x[r];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const int ta = (t >> 2) & 1, te = (t >> 1) & 1, tc = t & 1;
+        const double w = (ta ? 0.25 : 0.75) * (te ? 0.25 : 0.75) * (tc ? 0.25 : 0.75);
+        v = fma_rn(w, cv[ta ? 2 * da : 1][te ? 2 * de : 1][tc ? 2 * dc : 1], v);
+      }
+      x[r] = v;
+    }
+  }
+}
+
 // ---- a level whose every axis halves, FP32 quads (nz / 4 a power of two up to 16): its
 // V-cycle work in two marching kernels instead of six per-pass launches.  A block of
 // nz / 4 x (mty + 4) threads owns a band of mty rows and two halo rows on each side (a
@@ -904,6 +1028,19 @@ __device__ __forceinline__ void cell_ijk(const MgLevelT<T> &L, int q, int &i, in
 template <typename T>
 __device__ void blk_smooth(const MgLevelT<T> &L, int colour, int zero, const T *b, T *x) {
   const int n = L.nx * L.ny * L.nz;
+  if constexpr (sizeof(T) == sizeof(double)) {
+    if (L.nz % 2 == 0) {  // k_mgp_scale, k_mgp_colour
+      const int half = L.nz / 2, np = n / 2;
+      for (int p = threadIdx.x; p < np; p += blockDim.x) {
+        const unsigned r = udiv_inv((unsigned)p, L.dh_m, L.dh_l), ii = udiv_inv(r, L.dy_m, L.dy_l);
+        const int i = (int)ii, j = (int)r - i * L.ny, d = (i + j + colour) & 1;
+        const int k = 2 * (p - (int)r * half) + d, q = (int)r * L.nz + k;
+        x[q] = (zero ? b[q] : lnb64(L, x, i, j, k, q, b[q])) * linv(L, i, j, k);
+      }
+      __syncthreads();
+      return;
+    }
+  }
   if (L.nz % 2 == 0) {
     // the cells of a row pair up along k, one of each colour: a thread per pair updates the
     // one of the colour (and, from zero, clears the other)
@@ -936,10 +1073,23 @@ template <typename T>
 __device__ void blk_restrict(const MgLevelT<T> &F, const MgLevelT<T> &Cl, const T *bf, const T *xf, T *bc) {
   const T inv = T(1) / (T)(F.fx * F.fy * F.fz);
   const int n = Cl.nx * Cl.ny * Cl.nz;
+  const bool pairs = sizeof(T) == sizeof(double) && F.nz % 2 == 0;  // zero residual on colour 1 (k_mgp_restrict)
   for (int q = threadIdx.x; q < n; q += blockDim.x) {
     int i, j, k;
     cell_ijk(Cl, q, i, j, k);
     T sum = T(0);
+    if constexpr (sizeof(T) == sizeof(double)) {
+      if (pairs) {
+        for (int a = 0; a < F.fx; ++a)
+          for (int e = 0; e < F.fy; ++e)
+            for (int c = 0; c < F.fz; ++c) {
+              const int fi = i * F.fx + a, fj = j * F.fy + e, fk = k * F.fz + c;
+              if (!((fi + fj + fk) & 1)) sum = lnb64(F, xf, fi, fj, fk, lrow(F, fi, fj, fk), sum);
+            }
+        bc[q] = sum * inv;
+        continue;
+      }
+    }
     for (int a = 0; a < F.fx; ++a)
       for (int e = 0; e < F.fy; ++e)
         for (int c = 0; c < F.fz; ++c) {
@@ -959,6 +1109,7 @@ __device__ void blk_prolong(const MgLevelT<T> &F, const MgLevelT<T> &Cl, const T
   for (int q = threadIdx.x; q < n; q += blockDim.x) {
     int i, j, k;
     cell_ijk(F, q, i, j, k);
+    if (sizeof(T) == sizeof(double) && F.nz % 2 == 0 && ((i + j + k) & 1)) continue;  // overwritten next
     xf[q] += prolong_at(F, Cl, xc, i, j, k);
   }
   __syncthreads();
@@ -1020,9 +1171,11 @@ static void level_geometry(MgLevelT<T> &L, int nsm, bool quads) {
   L.gy = (L.ny + L.by - 1) / L.by;
   L.gz = std::max(1, std::min(L.nx, nsm * 8 / std::max(1, L.gx * L.gy)));
   // the quad smoother is FP32 (float4 loads): quads along x, rows along y, planes over z
-  L.qgrid = quads && sizeof(T) == sizeof(float) && L.nz % 4 == 0 ? 1 : 0;
+  // (FP64: the pair passes, pairs along x)
+  const bool pairs = sizeof(T) == sizeof(double) && L.nz % 2 == 0;
+  L.qgrid = (quads && sizeof(T) == sizeof(float) && L.nz % 4 == 0) || pairs ? 1 : 0;
   if (L.qgrid) {
-    const int nq = L.nz / 4;
+    const int nq = pairs ? L.nz / 2 : L.nz / 4;
     L.qbx = 1;
     while (L.qbx < nq && L.qbx < 32) L.qbx *= 2;
     L.qby = kBlock / L.qbx;
@@ -1069,7 +1222,7 @@ bool mg_plan(int nx, int ny, int nz, double hx, double hy, double hz, int nsm, b
     // the marching kernels: a band of 256 / (nz / 4) rows (at most ny), the segments sized so
     // that about two blocks per SM run
     const int nq = nz / 4;
-    if (L.qgrid && fx == 2 && fy == 2 && fz == 2 && nq <= 16 && (nq & (nq - 1)) == 0 && cells < (1LL << 31)) {
+    if (sizeof(T) == sizeof(float) && L.qgrid && fx == 2 && fy == 2 && fz == 2 && nq <= 16 && (nq & (nq - 1)) == 0 && cells < (1LL << 31)) {
       L.march = 1;
       L.mty = std::min(256 / nq, ny);
       L.mgy = (ny + L.mty - 1) / L.mty;
@@ -1100,12 +1253,14 @@ bool mg_plan(int nx, int ny, int nz, double hx, double hy, double hz, int nsm, b
 }
 
 // per level above the tail (or the coarsest): 2 smooths + restrict, prolong + 2 smooths, or
-// the two marching kernels; then one tail (or coarsest) kernel
+// the two marching kernels; then one tail (or coarsest) kernel.  The FP64 pair passes start
+// Jacobi-scaled rows (level 0) with one pass.
 template <typename T>
-int mg_vcycle_launches(const MgPlanT<T> &mg) {
+int mg_vcycle_launches(const MgPlanT<T> &mg, int jacobi) {
   const int m = mg.tail < mg.nlev ? mg.tail : mg.nlev - 1;
   int n = 1;
   for (int l = 0; l < m; ++l) n += mg.lev[l].march ? 2 : 6;
+  if (sizeof(T) == sizeof(double) && m > 0 && mg.lev[0].qgrid && jacobi) --n;
   return n;
 }
 
@@ -1199,6 +1354,14 @@ void launch_mg_vcycle(cudaStream_t s, const MgPlanT<T> &mg, int jacobi, const T 
     }
     launch_pdl(k_mg_smooth<T>, grid(l), block(l), 0, s, mg.lev[l], colour, zero, l == 0 ? jacobi : 0, B(l), X(l), sc);
   };
+  // a colour pass of the FP64 pair kernels
+  auto pair = [&](int l, int colour, int from_b) {
+    if constexpr (sizeof(T) == sizeof(double)) {
+      const MgLevelT<T> &F = mg.lev[l];
+      launch_pdl(l == 0 && jacobi ? k_mgp_colour<true> : k_mgp_colour<false>, dim3(F.qgx, F.qgy, F.qgz),
+                 dim3(F.qbx, F.qby, 1), 0, s, F, colour, from_b, B(l), X(l), sc);
+    }
+  };
   // pre-smoothing from zero and restriction to level l + 1.  (Both colour passes in one
   // kernel, each black cell recomputing its red neighbours' start values, was measured at
   // 80 us on the 512x256x64 level against 36 us for the two quad passes: not kept.)
@@ -1236,9 +1399,23 @@ void launch_mg_vcycle(cudaStream_t s, const MgPlanT<T> &mg, int jacobi, const T 
       return;
     }
     const int bs = l == 0 ? jacobi : 0;
+    const MgLevelT<T> &F = mg.lev[l];
+    if constexpr (sizeof(T) == sizeof(double)) {
+      if (F.qgrid) {
+        if (!bs)
+          launch_pdl(k_mgp_scale, dim3(F.qgx, F.qgy, F.qgz), dim3(F.qbx, F.qby, 1), 0, s, F, B(l), X(l), sc);
+        pair(l, 1, bs);
+        if (F.fx == 2 && F.fy == 2 && F.fz == 2)
+          launch_pdl(k_mgp_restrict, grid(l + 1), block(l + 1), 0, s, F, mg.lev[l + 1], (const T *)X(l),
+                     mg.lev[l + 1].b, sc);
+        else
+          launch_pdl(k_mg_restrict<T>, grid(l + 1), block(l + 1), 0, s, F, mg.lev[l + 1], bs, B(l), X(l),
+                     mg.lev[l + 1].b, sc);
+        return;
+      }
+    }
     smooth(l, 0, 1);
     smooth(l, 1, 0);
-    const MgLevelT<T> &F = mg.lev[l];
     if (F.fx == 2 && F.fy == 2 && F.fz == 2)
       launch_pdl(k_mg_restrict8<T>, grid(l + 1), block(l + 1), 0, s, F, mg.lev[l + 1], bs, B(l), X(l),
                  mg.lev[l + 1].b, sc);
@@ -1265,6 +1442,17 @@ void launch_mg_vcycle(cudaStream_t s, const MgPlanT<T> &mg, int jacobi, const T 
       march(l, true);
       continue;
     }
+    if constexpr (sizeof(T) == sizeof(double)) {
+      if (F.qgrid) {
+        if (F.fx == 2 && F.fy == 2 && F.fz == 2)
+          launch_pdl(k_mgp_prolong, grid(l + 1), block(l + 1), 0, s, F, mg.lev[l + 1], (const T *)X(l + 1), X(l), sc);
+        else
+          launch_pdl(k_mg_prolong<T>, grid(l), block(l), 0, s, F, mg.lev[l + 1], (const T *)X(l + 1), X(l), sc);
+        pair(l, 1, 0);
+        pair(l, 0, 0);
+        continue;
+      }
+    }
     if (F.fx == 2 && F.fy == 2 && F.fz == 2)
       launch_pdl(k_mg_prolong8<T>, grid(l + 1), block(l + 1), 0, s, F, mg.lev[l + 1], (const T *)X(l + 1), X(l), sc);
     else
@@ -1276,10 +1464,10 @@ void launch_mg_vcycle(cudaStream_t s, const MgPlanT<T> &mg, int jacobi, const T 
 
 template bool mg_plan<float>(int, int, int, double, double, double, int, bool, MgPlanT<float> *, bool);
 template bool mg_plan<double>(int, int, int, double, double, double, int, bool, MgPlanT<double> *, bool);
-template int mg_vcycle_launches<float>(const MgPlanT<float> &);
+template int mg_vcycle_launches<float>(const MgPlanT<float> &, int);
 template bool mg_dense_inverse<float>(const MgPlanT<float> &, std::vector<float> &);
 template bool mg_dense_inverse<double>(const MgPlanT<double> &, std::vector<double> &);
-template int mg_vcycle_launches<double>(const MgPlanT<double> &);
+template int mg_vcycle_launches<double>(const MgPlanT<double> &, int);
 template void mg_prepare<float>();
 template void mg_prepare<double>();
 template void launch_mg_vcycle<float>(cudaStream_t, const MgPlanT<float> &, int, const float *, float *,
