@@ -61,7 +61,7 @@ enum KId {
   K_RESID64, K_SETUP32, K_CORRECT64, K_TRANSFORM, K_UPDATE, K_BC, K_RBSOR, K_RNORM, K_NANRESET, K_ETA,
   K_CGQ64, K_CGXR64, K_CGP64, K_CGPQ32, K_CGXR32, K_CFL, K_LES,
   K_PP32, K_MG, K_PV32, K_PS32, K_PT32, K_PXR32, K_MIRROR,
-  K_PP64, K_MG64, K_PV64, K_PS64, K_PT64, K_PXR64, K_COUNT
+  K_PP64, K_MG64, K_PV64, K_PS64, K_PT64, K_PXR64, K_LOOP64, K_CGLOOP64, K_COUNT
 };
 const char *const kKernelNames[K_COUNT] = {
     "convection_diffusion", "rhs", "bicg_setup64", "bicg_ap64", "bicg_s64", "bicg_as64", "bicg_xr64",
@@ -69,7 +69,8 @@ const char *const kKernelNames[K_COUNT] = {
     "correct64", "transform", "update_uf", "bc", "rbsor_sweep", "residual_norm64", "nan_reset", "solid_fraction",
     "cg_q64", "cg_xr64", "cg_p64", "cg_pq32", "cg_xr32", "cfl", "smagorinsky",
     "bicgp_p32", "mg_vcycle", "bicgp_v32", "bicgp_s32", "bicgp_t32", "bicgp_xr32", "mirror32",
-    "bicgp_p64", "mg_vcycle64", "bicgp_v64", "bicgp_s64", "bicgp_t64", "bicgp_xr64"};
+    "bicgp_p64", "mg_vcycle64", "bicgp_v64", "bicgp_s64", "bicgp_t64", "bicgp_xr64",
+    "bicg_loop64", "cg_loop64"};
 
 // Scalars of one time step run as a graph, appended on the device (k_step_record)
 struct StepRec {
@@ -133,9 +134,11 @@ struct cfdgb_ctx {
   // chunk graphs of solver iterations
   cudaGraphExec_t chunk64 = nullptr, chunk32 = nullptr;
   int chunk_len = 16;
+  int loop_blocks = 0;  // blocks of the one-launch FP64 iterations (loop64_blocks); 0: a kernel a phase
   double omega = 0.0;  // SOR relaxation in use (cfg.omega, or the optimal one when that is 0)
   // test switch (environment CFDGB_TEST_WAIT_FAULT at create): the next MIXED solve makes one
-  // bounded wait of the FP32 bulk-copy pipeline run out, to exercise that failure path
+  // bounded wait of the FP32 bulk-copy pipeline run out, the next FP64 one a wait between the
+  // blocks of its one-launch iterations, to exercise that failure path
   bool test_wait_fault = false;
   // one CUDA graph per time step (FP64 Krylov solvers, after the first step, kernel timing
   // off): the whole step with its convergence loop as a conditional WHILE node; each step
@@ -484,12 +487,18 @@ const int kPrecKid64[kPrecParts] = {K_PP64, K_MG64, K_PV64, K_PS64, K_MG64, K_PT
 // the iteration of this precision is the multigrid-preconditioned one
 bool prec_iter(const cfdgb_ctx *c, bool fp32) { return fp32 ? c->use_mg : c->use_mg64; }
 
+// the FP64 Krylov iteration runs whole chunks in one cooperative launch
+bool loop_iter(const cfdgb_ctx *c, bool fp32) { return !fp32 && !c->use_mg64 && c->loop_blocks > 0; }
+
+// launch_iter_kernel's parts in one iteration (a whole chunk for the one-launch form)
 int iter_kernels(const cfdgb_ctx *c, bool fp32) {
+  if (loop_iter(c, fp32)) return 1;
   if (prec_iter(c, fp32)) return kPrecParts;
   if (c->cfg.solver == CFDGB_CG) return fp32 ? 2 : 3;
   return fp32 ? 3 : 5;
 }
 int iter_kid(const cfdgb_ctx *c, bool fp32, int part) {
+  if (loop_iter(c, fp32)) return c->cfg.solver == CFDGB_CG ? K_CGLOOP64 : K_LOOP64;
   if (prec_iter(c, fp32)) return (fp32 ? kPrecKid : kPrecKid64)[part];
   if (c->cfg.solver == CFDGB_CG) return (fp32 ? K_CGPQ32 : K_CGQ64) + part;
   return (fp32 ? K_PAP32 : K_AP64) + part;
@@ -500,10 +509,23 @@ int iter_part_launches(const cfdgb_ctx *c, bool fp32, int part) {
   const int jac = c->cfg.solver == CFDGB_BICGSTAB_JACOBI;
   return k == K_MG ? mg_vcycle_launches(c->mg, jac) : k == K_MG64 ? mg_vcycle_launches(c->mg64, jac) : 1;
 }
-// iterations per captured chunk: the preconditioned iteration is long and needs few
-int chunk_iters(const cfdgb_ctx *c, bool fp32) { return prec_iter(c, fp32) ? 2 : c->chunk_len; }
+// iterations per chunk, and how often a captured chunk repeats the parts: the preconditioned
+// iteration is long and needs few; the one-launch form is the chunk
+int chunk_iters(const cfdgb_ctx *c, bool fp32) {
+  if (loop_iter(c, fp32)) return loop64_iters(c->ncell);
+  return prec_iter(c, fp32) ? 2 : c->chunk_len;
+}
+int chunk_repeats(const cfdgb_ctx *c, bool fp32) { return loop_iter(c, fp32) ? 1 : chunk_iters(c, fp32); }
 void launch_iter_kernel(cfdgb_ctx *c, bool fp32, int part) {
   const bool jac = c->cfg.solver == CFDGB_BICGSTAB_JACOBI;
+  if (loop_iter(c, fp32)) {
+    if (c->cfg.solver == CFDGB_CG)
+      launch_cg64_loop(c->stream, c->g, c->spe64, c->k64, c->part, c->sc, c->loop_blocks, chunk_iters(c, false));
+    else
+      launch_bicg64_loop(c->stream, c->g, jac ? c->jac64 : c->spe64, c->k64, c->part, c->sc, c->loop_blocks,
+                         chunk_iters(c, false));
+    return;
+  }
   if (!fp32 && c->use_mg64) {
     PrecVecsT<double> v{c->k64.x, c->k64.r0, c->k64.r1, c->k64.p1, c->k64.ap, c->k64.s, c->k64.as, c->ph64, c->sh64,
                         nullptr};
@@ -545,7 +567,7 @@ void launch_iter_kernel(cfdgb_ctx *c, bool fp32, int part) {
 int capture_chunk(cfdgb_ctx *c, bool fp32) {
   cudaGraph_t graph;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  for (int m = 0; m < chunk_iters(c, fp32); ++m)
+  for (int m = 0; m < chunk_repeats(c, fp32); ++m)
     for (int part = 0; part < iter_kernels(c, fp32); ++part) launch_iter_kernel(c, fp32, part);
   CK(cudaStreamEndCapture(c->stream, &graph));
   cudaGraphExec_t exec;
@@ -569,6 +591,15 @@ int set_solver_params(cfdgb_ctx *c, SolverScal *dsc, double tol, int maxit) {
   return 0;
 }
 
+// the test switch (one shot): the next launch that waits on dsc makes a bounded wait run out
+int request_test_wait(cfdgb_ctx *c, SolverScal *dsc) {
+  if (!c->test_wait_fault) return 0;
+  static const int one = 1;
+  CK(cudaMemcpyAsync(&dsc->test_wait, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  c->test_wait_fault = false;
+  return 0;
+}
+
 // Iterate chunks until the device says done.  Returns the scalars in *out.  Each chunk
 // is a captured graph of chunk_len iterations; with kernel timing on, the same kernels
 // are launched one by one between event pairs instead, one iteration per poll, so that no
@@ -576,7 +607,7 @@ int set_solver_params(cfdgb_ctx *c, SolverScal *dsc, double tol, int maxit) {
 int run_chunks(cfdgb_ctx *c, bool fp32, SolverScal *out) {
   SolverScal *dsc = fp32 ? c->sc32 : c->sc;
   if (!c->timing && !(fp32 ? c->chunk32 : c->chunk64)) TRY(capture_chunk(c, fp32));
-  const int len = c->timing ? 1 : chunk_iters(c, fp32);
+  const int len = c->timing ? 1 : chunk_repeats(c, fp32);
   const long long max_chunks = (long long)c->cfg.maxit / len + 3;
   const int nk = iter_kernels(c, fp32);
   for (long long q = 0; q < max_chunks; ++q) {
@@ -599,8 +630,9 @@ int run_chunks(cfdgb_ctx *c, bool fp32, SolverScal *out) {
     if (trace >= 2)
       std::fprintf(stderr, "[cfdgb]     %s it %d relres %.4e\n", fp32 ? "fp32" : "fp64", c->h_sc->iter,
                    c->h_sc->relres);
-    if (fp32 && c->h_sc->fault)
-      return fail(CFDGB_ECUDA, "FP32 stencil pipeline: a bounded wait gave up (block stopped early)");
+    if (c->h_sc->fault)
+      return fail(CFDGB_ECUDA, fp32 ? "FP32 stencil pipeline: a bounded wait gave up (block stopped early)"
+                                    : "FP64 iteration: a bounded wait between blocks gave up");
     if (c->h_sc->done) {
       *out = *c->h_sc;
       return 0;
@@ -687,6 +719,7 @@ int solve_pressure(cfdgb_ctx *c, int *iters, int *outer, double *relres, int *st
   }
   if (c->cfg.precision == CFDGB_FP64) {
     TRY(set_solver_params(c, c->sc, c->cfg.tol, c->cfg.maxit));
+    if (loop_iter(c, false)) TRY(request_test_wait(c, c->sc));
     L(c, K_SETUP64, 1, [&] { launch_setup64(c, st64); });
     SolverScal r;
     TRY(run_chunks(c, false, &r));
@@ -738,11 +771,7 @@ int solve_mixed(cfdgb_ctx *c, double tol, int *iters, int *outer, double *relres
   }
   if (rel < tol) return 0;
   TRY(set_solver_params(c, c->sc32, tol, c->cfg.maxit));
-  if (c->test_wait_fault) {  // one shot
-    static const int one = 1;
-    CK(cudaMemcpyAsync(&c->sc32->test_wait, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    c->test_wait_fault = false;
-  }
+  TRY(request_test_wait(c, c->sc32));
   L(c, K_SETUP32, 1, [&] {
     launch_refine_start32(c->stream, c->g, st64, jacf, c->k32, c->p32, c->ap32, c->rf, c->ss, sweep_reduction(c), sweep_peak(c), 1,
                           c->part, c->sc32);
@@ -1025,7 +1054,7 @@ int capture_step_graph(cfdgb_ctx *c) {
   CK(cudaStreamSynchronize(c->stream));
   c->graph_fixed = 0;
   std::fill(std::begin(c->graph_fixed_kn), std::end(c->graph_fixed_kn), 0LL);
-  const int len = chunk_iters(c, false), nk = iter_kernels(c, false);
+  const int len = chunk_repeats(c, false), nk = iter_kernels(c, false);
   cudaGraph_t graph = nullptr;
   c->capturing = true;
   auto done = [&](cudaError_t e) -> int {
@@ -1069,7 +1098,7 @@ int capture_step_graph(cfdgb_ctx *c) {
   std::swap(c->stream, c->side);  // the iteration launchers enqueue on c->stream
   for (int m = 0; m < len; ++m)
     for (int part = 0; part < nk; ++part) launch_iter_kernel(c, false, part);
-  const int max_bodies = c->cfg.maxit / len + 4;
+  const int max_bodies = c->cfg.maxit / chunk_iters(c, false) + 4;
   k_loop_cond<<<1, 1, 0, c->stream>>>(h, c->sc, c->ring, max_bodies);
   std::swap(c->stream, c->side);
   cudaGraph_t body_out = nullptr;
@@ -1098,12 +1127,13 @@ int capture_step_graph(cfdgb_ctx *c) {
 // steps; fills stats[0..n) and returns the worst status
 int run_step_graphs(cfdgb_ctx *c, int n, cfdgb_step_stats *stats, int *worst) {
   if (!c->step_graph) TRY(capture_step_graph(c));
-  const int len = chunk_iters(c, false), nk = iter_kernels(c, false);
+  const int len = chunk_repeats(c, false), nk = iter_kernels(c, false);
   long long per_body = 1;  // k_loop_cond
   for (int part = 0; part < nk; ++part) per_body += (long long)iter_part_launches(c, false, part) * len;
   for (int done = 0; done < n;) {
     const int b = std::min(n - done, kRing);
     CK(cudaMemsetAsync(&c->ring->n, 0, sizeof(int), c->stream));
+    if (loop_iter(c, false)) TRY(request_test_wait(c, c->sc));
     for (int q = 0; q < b; ++q) CK(cudaGraphLaunch(c->step_graph, c->stream));
     CK(cudaMemcpyAsync(c->h_ring, c->ring, offsetof(StepRing, rec) + b * sizeof(StepRec), cudaMemcpyDeviceToHost,
                        c->stream));
@@ -1463,7 +1493,8 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
     }
     c->use_mg = true;
   }
-  if ((rc = dalloc(c, &c->part, 8 * (size_t)std::max(c->nblk, nblk3)))) return bail(rc);
+  if (cfg->solver != CFDGB_RBSOR && !std::getenv("CFDGB_NO_LOOP")) c->loop_blocks = loop64_blocks(c->ncell);
+  if ((rc = dalloc(c, &c->part, std::max(8 * (size_t)std::max(c->nblk, nblk3), loop64_part_doubles())))) return bail(rc);
   if ((rc = dalloc(c, &c->sc, 1)) || (rc = dalloc(c, &c->sc32, 1)) || (rc = dalloc(c, &c->ss, 1))) return bail(rc);
   cudaMemset(c->sc, 0, sizeof(SolverScal));
   cudaMemset(c->sc32, 0, sizeof(SolverScal));
@@ -1778,8 +1809,11 @@ int cfdgb_op_bicgstab(cfdgb_ctx *c, int solver, double tol, int maxit, const dou
   SolverScal r{};
   int rc = 0;
   for (long long q = 0; q < (long long)maxit / 8 + 3; ++q) {
-    for (int m = 0; m < 8; ++m)
-      for (int part = 0; part < 5; ++part) launch_bicg64_part(c->stream, part, c->g, st, c->k64, c->part, c->sc);
+    if (c->loop_blocks)
+      launch_bicg64_loop(c->stream, c->g, st, c->k64, c->part, c->sc, c->loop_blocks, loop64_iters(c->ncell));
+    else
+      for (int m = 0; m < 8; ++m)
+        for (int part = 0; part < 5; ++part) launch_bicg64_part(c->stream, part, c->g, st, c->k64, c->part, c->sc);
     CK(cudaMemcpyAsync(c->h_sc, c->sc, sizeof(SolverScal), cudaMemcpyDeviceToHost, c->stream));
     TRY(sync(c));
     if (c->h_sc->done) { r = *c->h_sc; break; }
@@ -1999,7 +2033,11 @@ int adjoint_solve(cfdgb_ctx *c, const double *rhs, double tol, int *iters) {
   const PrecVecsT<double> pv{c->ka.x, c->ka.r0, c->ka.r1, c->ka.p1, c->ka.ap, c->ka.s, c->ka.as, c->kapx[0],
                              c->kapx[1], nullptr};
   for (long long q = 0; q < (long long)c->cfg.maxit / 8 + 3; ++q) {
-    for (int m = 0; m < 8; ++m) {
+    if (!mg && c->loop_blocks)
+      L(c, K_LOOP64, 1, [&] {
+        launch_bicg64_loop(c->stream, c->g, c->spe64, c->ka, c->part, c->sca, c->loop_blocks, loop64_iters(c->ncell));
+      });
+    for (int m = 0; m < 8 && (mg || !c->loop_blocks); ++m) {
       if (mg) {
         for (int part = 0; part < kPrecParts; ++part) {
           L(c, kPrecKid64[part], part == 1 || part == 4 ? mg_vcycle_launches(c->mg64, 0) : 1, [&] {

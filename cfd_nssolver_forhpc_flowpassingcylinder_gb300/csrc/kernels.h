@@ -95,6 +95,21 @@ void launch_bicg_setup64(cudaStream_t s, int nblk, const Geo &g, const Stencil<d
 // FP64 iteration, kernel `part` 0..4 (ap, s, as, xr, p); each a no-op once sc->done is set
 void launch_bicg64_part(cudaStream_t s, int part, const Geo &g, const Stencil<double> &st, KrylovVecs<double> v,
                         double *part_buf, SolverScal *sc);
+// The same iteration and CG's, `iters` of them in one cooperative launch of `blocks` blocks
+// (loop64_blocks: 0 where the grid is larger than kLoopCells or the device cannot); part_buf
+// holds loop64_part_doubles() doubles.  A chunk is loop64_iters iterations, a millisecond or
+// a few, so that a solve stays interruptible between launches.
+// kLoopCells: one launch against a kernel a phase, us an iteration: 2.1 M cells 120.3 / 131.8
+// (BiCGSTAB), 59.1 / 64.9 (CG), 4.7 M 271.4 / 270.2 and 146.6 / 144.2, 8.4 M 462.7 / 450.8 and
+// 262.8 / 246.4 (the block a multiprocessor leaves HBM waiting): the line lies between.
+constexpr long long kLoopCells = 3LL << 20;
+int loop64_blocks(long long ncell);
+int loop64_iters(long long ncell);
+size_t loop64_part_doubles();
+void launch_bicg64_loop(cudaStream_t s, const Geo &g, const Stencil<double> &st, KrylovVecs<double> v,
+                        double *part_buf, SolverScal *sc, int blocks, int iters);
+void launch_cg64_loop(cudaStream_t s, const Geo &g, const Stencil<double> &st, KrylovVecs<double> v,
+                      double *part_buf, SolverScal *sc, int blocks, int iters);
 // FP32 iteration, kernel `part` 0..2 (p update + A p, s + A s, x and r1); p and ap are
 // double-buffered: p2[sc->par] holds the previous p, p2[sc->par ^ 1] receives the new one
 void launch_bicg32_part(cudaStream_t s, int part, const Geo &g, const Stencil<float> &st, KrylovVecs<float> v,

@@ -18,7 +18,7 @@
 //     solver scalars and reduction tickets it relies on before it starts, but two calls
 //     whose work overlaps on the GPU (different streams or threads at the same time) race
 //     on it and must not be issued;
-//   - the call polls the solver's convergence from the host every 8 iterations (a
+//   - the call polls the solver's convergence from the host every chunk of iterations (a
 //     device-to-host copy and a wait on `stream`), so `stream` must not be capturing into a
 //     CUDA graph: a capturing stream is rejected with CFDGB_EINVAL before any work;
 //   - the first call on a device looks up the array's device address with
@@ -174,12 +174,17 @@ extern "C" int cfdgb_poisson_solve_static(int nx, int ny, int nz, double dx, dou
   launch_bicg_setup64(s, 0, g, st, v, d_rhs, px1, px2, part, sc);
   SolverScal h{};
   bool done = false;
+  const int loop = loop64_blocks(n);  // chunks of iterations in one launch, as the context driver runs them
   for (long long q = 0; q < (long long)maxit / 8 + 3 && !done; ++q) {
-    for (int m = 0; m < 8; ++m)
-      for (int k = 0; k < 5; ++k) launch_bicg64_part(s, k, g, st, v, part, sc);
+    if (loop)
+      launch_bicg64_loop(s, g, st, v, part, sc, loop, loop64_iters(n));
+    else
+      for (int m = 0; m < 8; ++m)
+        for (int k = 0; k < 5; ++k) launch_bicg64_part(s, k, g, st, v, part, sc);
     if (cudaMemcpyAsync(&h, sc, sizeof(SolverScal), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
       return CFDGB_ECUDA;
+    if (h.fault) return CFDGB_ECUDA;  // a bounded wait between blocks gave up
     done = h.done != 0;
   }
   if (!done) return CFDGB_ECUDA;

@@ -16,6 +16,7 @@
 // iteration; the p update is fused into the next SpMV and s into its SpMV by
 // recomputing them at the stencil points (L1-resident), 17 instead of 19 words per cell.
 #include <algorithm>
+#include <atomic>
 
 #include "cfdgb_internal.cuh"
 #include "kernels.h"
@@ -1571,6 +1572,515 @@ __global__ void __launch_bounds__(kBlock) k32cg_xr(Geo g, Vec32 v, double *part,
   }
 }
 
+// ---- FP64 Krylov iterations in one cooperative launch ----
+// On grids up to a few million cells an iteration's kernels are short (2-20 us) and mostly
+// latency: each launch ramps up, reads its scalars through L2 and three of five end in a
+// reduction whose last block works alone.  Here one block a multiprocessor keeps a contiguous
+// range of cells for the whole chunk of iterations; the phases of an iteration (the five
+// kernels above, or CG's three) are separated by a grid barrier of one counter, and after a
+// reducing phase every block sums the block partials itself, in the same order, so the
+// scalars need no second round trip.  Same operations per cell as the kernels above; the dot
+// products are summed in this partition's order.
+// Measured, us an iteration, a kernel a phase -> one launch: BiCGSTAB 8 K cells 21.4 -> 11.9,
+// 131 K 31.1 -> 21.3, 1.05 M 75.9 -> 65.1 (the FP64 pipe's time is 41.7), 2.1 M 131.8 -> 120.3,
+// stretched 1.6 M 117.6 -> 94.7; CG 8 K 12.6 -> 8.4, 314 K 24.7 -> 17.1.
+// The barrier counts arrivals (sc->cnt[6], back to zero through sc->cnt[7] when the last block
+// leaves).  A wait is bounded: one that gives up sets sc->fault and CFDGB_ECUDA, the block
+// leaves, and so do the others, each after its own bounded wait.  (Polling all blocks' sums,
+// each word tagged with the reduction's number, instead of the counter: 152 x 152 polled words
+// slow the stores they wait for, 96x48x4 12.7 -> 23.7 us an iteration: not kept.)
+constexpr int kLoopBlock = 512;
+constexpr int kLoopMaxBlocks = 512;  // sums of the blocks, read by one thread each
+constexpr long long kLoopWaitCycles = 1LL << 32;  // ~2 s
+constexpr int kLoopSlots = 5;        // values reduced in an iteration
+
+struct LoopScal {
+  double rho, alpha, omega, beta, relres;
+  int iter, done, status, restart, bad;
+};
+
+struct LoopGrid {
+  SolverScal *sc;
+  double *part;     // [slot][kLoopMaxBlocks]
+  unsigned target;  // arrivals that complete the next barrier
+  long long limit;  // cycles a wait may take
+  __device__ __forceinline__ bool sync(LoopScal &L) {
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sc->cnt[6]) : "memory");
+      const long long t0 = clock64();
+      for (;;) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&sc->cnt[6]) : "memory");
+        if ((int)(v - target) >= 0) break;
+        if (clock64() - t0 > limit) {
+          L.bad = 1;
+          break;
+        }
+      }
+    }
+    __syncthreads();
+    return L.bad == 0;
+  }
+  // sums of v over the grid (slots s..), with a barrier; warp 0 calls fin(sums) in all its lanes,
+  // which leaves the scalars in L
+  template <int NV, class Fin>
+  __device__ __forceinline__ bool reduce(LoopScal &L, double (&v)[NV], int s, Fin &&fin) {
+    __shared__ double sh[NV][kLoopMaxBlocks / 32];
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = (int)(gridDim.x + 31) >> 5;
+    block_sum<NV>(v);
+    if (t == 0)
+#pragma unroll
+      for (int q = 0; q < NV; ++q) part[(s + q) * kLoopMaxBlocks + blockIdx.x] = v[q];
+    if (!sync(L)) return false;
+    if (wid < nw) {
+      double o[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) o[q] = t < (int)gridDim.x ? __ldcg(part + (s + q) * kLoopMaxBlocks + t) : 0.0;
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        const double x = warp_sum1(o[q]);
+        if (lane == 0) sh[q][wid] = x;
+      }
+    }
+    __syncthreads();
+    if (wid == 0) {
+      double out[NV];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) out[q] = warp_sum1(lane < nw ? sh[q][lane] : 0.0);
+      fin(out);
+    }
+    __syncthreads();
+    return true;
+  }
+};
+
+// The test request (sc->test_wait, set only by the host's test switch): block 0 waits for one
+// arrival that never comes, every block with a short limit, so that the waits run out
+__device__ __forceinline__ LoopGrid loop_grid(SolverScal *sc, double *part) {
+  const int test = sc->test_wait;
+  return LoopGrid{sc, part, test && blockIdx.x == 0 ? 1u : 0u, test ? kTestWaitCycles : kLoopWaitCycles};
+}
+// scalars in, and out by block 0 when every block has left the loop's last barrier
+__device__ __forceinline__ void loop_begin(LoopScal &L, const SolverScal *sc) {
+  if (threadIdx.x == 0) {
+    L.rho = sc->rho;
+    L.alpha = sc->alpha;
+    L.omega = sc->omega;
+    L.beta = sc->beta;
+    L.relres = sc->relres;
+    L.iter = sc->iter;
+    L.done = sc->done;
+    L.status = sc->status;
+    L.restart = sc->restart;
+    L.bad = 0;
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ void loop_end(const LoopScal &L, const LoopGrid &G) {
+  SolverScal *const sc = G.sc;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  if (L.bad) {
+    atomicExch(&sc->fault, 1);
+    sc->status = CFDGB_ECUDA;
+    sc->done = 1;
+    sc->test_wait = 0;
+  } else if (blockIdx.x == 0) {
+    sc->rho = L.rho;
+    sc->alpha = L.alpha;
+    sc->omega = L.omega;
+    sc->beta = L.beta;
+    sc->relres = L.relres;
+    sc->iter = L.iter;
+    sc->done = L.done;
+    sc->status = L.status;
+    sc->restart = L.restart;
+  }
+  __threadfence();
+  if (atomicAdd(&sc->cnt[7], 1u) == gridDim.x - 1) {  // every block is past its last wait
+    sc->cnt[6] = 0u;
+    sc->cnt[7] = 0u;
+  }
+}
+
+// finish_iteration<false> on the loop's scalars (warp 0)
+__device__ __forceinline__ void loop_finish(LoopScal &L, double norm0, double tol, double thr, int maxit, int timestep,
+                                            double n2, double rr) {
+  const double rho_old = L.rho;
+  double relres, ao, rq;
+  div3(sqrt(n2), norm0, L.alpha, L.omega, rr, rho_old, relres, ao, rq);
+  if (threadIdx.x != 0) return;
+  L.relres = relres;
+  if (relres < tol) {
+    L.done = 1;
+  } else if (L.iter >= maxit) {
+    L.done = 1;
+    L.status = CFDGB_ENOCONV;
+  } else {
+    L.rho = rr;
+    L.beta = ao * rq;
+    L.restart = !(timestep < 10 || fabs(rho_old) > thr);
+    L.iter += 1;
+  }
+}
+
+// The cells of a block: a contiguous range, the threads strided through it.  load(row) reads a
+// cell's values and use(row, values) consumes them; the next cell's loads are issued before
+// this one's arithmetic (a block a multiprocessor has too few warps to hide L2's latency with).
+template <class Load, class Use>
+__device__ __forceinline__ void loop_cells(long long lo, long long hi, Load &&load, Use &&use) {
+  long long row = lo + threadIdx.x;
+  if (row >= hi) return;
+  auto cur = load(row);
+  for (;;) {
+    const long long next = row + kLoopBlock;
+    if (next >= hi) break;
+    auto nxt = load(next);
+    use(row, cur);
+    cur = nxt;
+    row = next;
+  }
+  use(row, cur);
+}
+template <int N>
+struct LoopVals {
+  double v[N];
+};
+
+// The operator at a row: the neighbours' values in the order of stencil_apply's terms (zero
+// where there is none), the centre, and what the row's entries need.  MODE 0: a uniform grid
+// (class table).  The stretched grid takes its entries from the per-axis factors and one stored
+// value a row (jp, or SPE's diagonal) instead of the seven stored entries, which were 56 bytes
+// a cell and application: MODE 1, Jacobi-scaled rows, f_c - jp sum(factor f_nb) (the diagonal
+// dj jp is 1 to within half an ulp, as jp = RN(1/dj)); MODE 2, SPE rows.
+struct LoopStencil {
+  double f[6], c, d, z;
+  int ic, jc, kc;
+};
+template <int MODE>
+__device__ __forceinline__ LoopStencil loop_load(const Geo &g, const double *f, const double *z, long long row) {
+  LoopStencil S;
+  row_cijk(row, g.nyc, g.nzc, S.ic, S.jc, S.kc);
+  const long long nyz = (long long)g.nyc * g.nzc, zm = z_minus(g, S.kc, row), zp = z_plus(g, S.kc, row);
+  S.f[0] = S.ic > 0 ? f[row - nyz] : 0.0;
+  S.f[1] = S.jc > 0 ? f[row - g.nzc] : 0.0;
+  S.f[2] = zm >= 0 ? f[zm] : 0.0;
+  S.f[3] = zp >= 0 ? f[zp] : 0.0;
+  S.f[4] = S.jc < g.nyc - 1 ? f[row + g.nzc] : 0.0;
+  S.f[5] = S.ic < g.nxc - 1 ? f[row + nyz] : 0.0;
+  S.c = f[row];
+  if (z) S.z = z[row];
+  if (MODE == 1) S.d = g.jpv[row];
+  if (MODE == 2) S.d = g.cof[0][3 * g.ncell + row];
+  return S;
+}
+template <int MODE>
+__device__ __forceinline__ double loop_apply(const Geo &g, const Stencil<double> &st, const LoopStencil &S) {
+  if (MODE == 0) {
+    const double *c = st.c[cls_of(g, S.ic, S.jc, S.kc)];
+    double y = c[0] * S.f[0];
+    y = fma(c[1], S.f[1], y);
+    y = fma(c[2], S.f[2], y);
+    y = fma(c[3], S.c, y);
+    y = fma(c[4], S.f[3], y);
+    y = fma(c[5], S.f[4], y);
+    return fma(c[6], S.f[5], y);
+  }
+  const double *ym = MODE == 1 ? g.fym : g.fyp, *yp = MODE == 1 ? g.fyp : g.fym;  // SPE_sparseMatrix.hpp:79,83
+  double y = g.fxm[S.ic] * S.f[0];
+  y = fma(ym[S.jc], S.f[1], y);
+  y = fma(g.fzm[S.kc], S.f[2], y);
+  y = fma(g.fzp[S.kc], S.f[3], y);
+  y = fma(yp[S.jc], S.f[4], y);
+  y = fma(g.fxp[S.ic], S.f[5], y);
+  return MODE == 1 ? fma(-S.d, y, S.c) : fma(S.d, S.c, -y);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(kLoopBlock, 1) k64_bicg_loop(Geo g, Stencil<double> st, KrylovVecs<double> v,
+                                                               double *part, SolverScal *sc, int iters, int chunk) {
+  __shared__ LoopScal L;
+  loop_begin(L, sc);
+  if (L.done) return;  // the same in every block: sc is written only after the last barrier
+  LoopGrid G = loop_grid(sc, part);
+  const double norm0 = sc->norm0, tol = sc->tol, thr = sc->restart_thr;
+  const int maxit = sc->maxit, timestep = sc->timestep;
+  const long long lo = min(g.ncell, (long long)blockIdx.x * chunk), hi = min(g.ncell, lo + chunk);
+  double *x = v.x, *r0 = v.r0, *r1 = v.r1, *p1 = v.p1, *s = v.s, *ap = v.ap, *as = v.as;
+  for (int it = 0; it < iters; ++it) {
+    {  // ap = A p1, alpha
+      double a[1] = {0.0};
+      loop_cells(
+          lo, hi, [&](long long row) { return loop_load<MODE>(g, p1, r0, row); },
+          [&](long long row, const LoopStencil &S) {
+            const double y = loop_apply<MODE>(g, st, S);
+            ap[row] = y;
+            a[0] = fma(y, S.z, a[0]);
+          });
+      if (!G.reduce<1>(L, a, 0, [&](const double (&o)[1]) {
+            const double al = L.rho / o[0];
+            if (threadIdx.x == 0) L.alpha = al;
+          }))
+        break;
+    }
+    const double al = L.alpha;
+    loop_cells(
+        lo, hi, [&](long long row) { return LoopVals<2>{{r1[row], ap[row]}}; },
+        [&](long long row, const LoopVals<2> &q) { s[row] = fma(-al, q.v[1], q.v[0]); });
+    if (!G.sync(L)) break;
+    {  // as = A s, omega
+      double a[2] = {0.0, 0.0};
+      loop_cells(
+          lo, hi, [&](long long row) { return loop_load<MODE>(g, s, nullptr, row); },
+          [&](long long row, const LoopStencil &S) {
+            const double y = loop_apply<MODE>(g, st, S);
+            as[row] = y;
+            a[0] = fma(y, S.c, a[0]);
+            a[1] = fma(y, y, a[1]);
+          });
+      if (!G.reduce<2>(L, a, 1, [&](const double (&o)[2]) {
+            const double w = o[0] / o[1];
+            if (threadIdx.x == 0) L.omega = w;
+          }))
+        break;
+    }
+    const double w = L.omega;
+    {  // x, r1, stop test and beta
+      double a[2] = {0.0, 0.0};
+      loop_cells(
+          lo, hi, [&](long long row) { return LoopVals<5>{{s[row], as[row], p1[row], x[row], r0[row]}}; },
+          [&](long long row, const LoopVals<5> &q) {
+            const double r = fma(-w, q.v[1], q.v[0]);
+            x[row] = fma(w, q.v[0], fma(al, q.v[2], q.v[3]));
+            r1[row] = r;
+            a[0] = fma(r, r, a[0]);
+            a[1] = fma(r, q.v[4], a[1]);
+          });
+      if (!G.reduce<2>(L, a, 3, [&](const double (&o)[2]) {
+            loop_finish(L, norm0, tol, thr, maxit, timestep, o[0], o[1]);
+          }))
+        break;
+    }
+    if (L.done) break;
+    const double be = L.beta;
+    const bool rst = L.restart != 0;
+    loop_cells(
+        lo, hi, [&](long long row) { return LoopVals<3>{{r1[row], ap[row], p1[row]}}; },
+        [&](long long row, const LoopVals<3> &q) {
+          p1[row] = rst ? q.v[0] : fma(be, fma(-w, q.v[1], q.v[2]), q.v[0]);
+          if (rst) r0[row] = q.v[0];
+        });
+    if (!G.sync(L)) break;
+  }
+  loop_end(L, G);
+}
+
+// CG's stop test and beta (finish_cg64) on the loop's scalars (warp 0)
+__device__ __forceinline__ void loop_finish_cg(LoopScal &L, double norm0, double tol, int maxit, double n2) {
+  double relres, beta, unused;
+  div3(sqrt(n2), norm0, n2, L.rho, n2, L.rho, relres, beta, unused);
+  if (threadIdx.x != 0) return;
+  L.relres = relres;
+  if (relres < tol) {
+    L.done = 1;
+  } else if (!isfinite(relres)) {
+    L.done = 1;
+    L.status = CFDGB_ENAN;
+  } else if (L.iter >= maxit) {
+    L.done = 1;
+    L.status = CFDGB_ENOCONV;
+  } else {
+    L.beta = beta;
+    L.rho = n2;
+    L.iter += 1;
+  }
+}
+
+__global__ void __launch_bounds__(kLoopBlock, 1) k64cg_loop(Geo g, Stencil<double> st, KrylovVecs<double> v,
+                                                            double *part, SolverScal *sc, int iters, int chunk) {
+  __shared__ LoopScal L;
+  loop_begin(L, sc);
+  if (L.done) return;
+  LoopGrid G = loop_grid(sc, part);
+  const double norm0 = sc->norm0, tol = sc->tol;
+  const int maxit = sc->maxit;
+  const long long lo = min(g.ncell, (long long)blockIdx.x * chunk), hi = min(g.ncell, lo + chunk);
+  double *x = v.x, *r1 = v.r1, *p1 = v.p1, *q1 = v.ap;
+  for (int it = 0; it < iters; ++it) {
+    {  // q = A p, alpha
+      double a[1] = {0.0};
+      loop_cells(
+          lo, hi, [&](long long row) { return loop_load<0>(g, p1, nullptr, row); },
+          [&](long long row, const LoopStencil &S) {
+            const double y = loop_apply<0>(g, st, S);
+            q1[row] = y;
+            a[0] = fma(y, S.c, a[0]);
+          });
+      if (!G.reduce<1>(L, a, 0, [&](const double (&o)[1]) {
+            const double al = L.rho / o[0];
+            if (threadIdx.x == 0) L.alpha = al;
+          }))
+        break;
+    }
+    const double al = L.alpha;
+    {  // x, r, stop test and beta
+      double a[1] = {0.0};
+      loop_cells(
+          lo, hi, [&](long long row) { return LoopVals<4>{{p1[row], q1[row], x[row], r1[row]}}; },
+          [&](long long row, const LoopVals<4> &q) {
+            x[row] = fma(al, q.v[0], q.v[2]);
+            const double r = fma(-al, q.v[1], q.v[3]);
+            r1[row] = r;
+            a[0] = fma(r, r, a[0]);
+          });
+      if (!G.reduce<1>(L, a, 1, [&](const double (&o)[1]) { loop_finish_cg(L, norm0, tol, maxit, o[0]); })) break;
+    }
+    if (L.done) break;
+    const double be = L.beta;
+    loop_cells(
+        lo, hi, [&](long long row) { return LoopVals<2>{{p1[row], r1[row]}}; },
+        [&](long long row, const LoopVals<2> &q) { p1[row] = fma(be, q.v[0], q.v[1]); });
+    if (!G.sync(L)) break;
+  }
+  loop_end(L, G);
+}
+
+// The neighbours of a cell in the order of stencil_apply's terms: -x, -y, -z, +z, +y, +x
+// (row -1 where there is none) and the row's coefficients
+struct LoopRow {
+  int nb[6];
+  double c[7];
+};
+__device__ __forceinline__ LoopRow loop_row(const Geo &g, const Stencil<double> &st, int row) {
+  LoopRow R;
+  int ic, jc, kc;
+  row_cijk(row, g.nyc, g.nzc, ic, jc, kc);
+  const int nyz = g.nyc * g.nzc;
+  R.nb[0] = ic > 0 ? row - nyz : -1;
+  R.nb[1] = jc > 0 ? row - g.nzc : -1;
+  R.nb[2] = (int)z_minus(g, kc, row);
+  R.nb[3] = (int)z_plus(g, kc, row);
+  R.nb[4] = jc < g.nyc - 1 ? row + g.nzc : -1;
+  R.nb[5] = ic < g.nxc - 1 ? row + nyz : -1;
+#pragma unroll
+  for (int q = 0; q < 7; ++q)
+    R.c[q] = g.nonuni ? g.cof[st.jac][q * g.ncell + row] : st.c[cls_of(g, ic, jc, kc)][q];
+  return R;
+}
+// A f from the centre and the neighbours' values (zero where there is none)
+__device__ __forceinline__ double loop_row_apply(const LoopRow &R, const double (&f)[6], double fc) {
+  double y = R.c[0] * f[0];
+  y = fma(R.c[1], f[1], y);
+  y = fma(R.c[2], f[2], y);
+  y = fma(R.c[3], fc, y);
+  y = fma(R.c[4], f[3], y);
+  y = fma(R.c[5], f[4], y);
+  return fma(R.c[6], f[5], y);
+}
+
+// One cell a thread (grids up to the device's threads in this form): the thread's own values
+// stay in registers for the whole chunk, and p and s are also formed at the six neighbours from
+// the published r1 and A p, so that an iteration has three barriers instead of five.
+__global__ void __launch_bounds__(kLoopBlock, 1) k64_bicg_loop1(Geo g, Stencil<double> st, KrylovVecs<double> v,
+                                                                double *part, SolverScal *sc, int iters, int chunk) {
+  __shared__ LoopScal L;
+  loop_begin(L, sc);
+  if (L.done) return;
+  LoopGrid G = loop_grid(sc, part);
+  const double norm0 = sc->norm0, tol = sc->tol, thr = sc->restart_thr;
+  const int maxit = sc->maxit, timestep = sc->timestep;
+  const int row = blockIdx.x * chunk + threadIdx.x;
+  const bool on = (int)threadIdx.x < chunk && row < g.ncell;
+  LoopRow R{};
+  double x = 0, r0 = 0, r1 = 0, p = 0, ap = 0;
+  double rn[6] = {0, 0, 0, 0, 0, 0}, pn[6] = {0, 0, 0, 0, 0, 0};  // r1 and p at the neighbours
+  if (on) {
+    R = loop_row(g, st, row);
+    x = v.x[row];
+    r0 = v.r0[row];
+    r1 = v.r1[row];
+    p = v.p1[row];
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+      if (R.nb[q] >= 0) {
+        rn[q] = v.r1[R.nb[q]];
+        pn[q] = v.p1[R.nb[q]];
+      }
+  }
+  for (int it = 0; it < iters; ++it) {
+    {  // A p, published (its neighbours read the last one two barriers ago)
+      double a[1] = {0.0};
+      if (on) {
+        ap = loop_row_apply(R, pn, p);
+        v.ap[row] = ap;
+        a[0] = ap * r0;
+      }
+      if (!G.reduce<1>(L, a, 0, [&](const double (&o)[1]) {
+            const double al = L.rho / o[0];
+            if (threadIdx.x == 0) L.alpha = al;
+          }))
+        break;
+    }
+    const double al = L.alpha;
+    double sv = 0, as = 0, an[6] = {0, 0, 0, 0, 0, 0};
+    {
+      double a[2] = {0.0, 0.0};
+      if (on) {
+        double sn[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) an[q] = R.nb[q] >= 0 ? __ldcg(v.ap + R.nb[q]) : 0.0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) sn[q] = fma(-al, an[q], rn[q]);
+        sv = fma(-al, ap, r1);
+        as = loop_row_apply(R, sn, sv);
+        a[0] = as * sv;
+        a[1] = as * as;
+      }
+      if (!G.reduce<2>(L, a, 1, [&](const double (&o)[2]) {
+            const double w = o[0] / o[1];
+            if (threadIdx.x == 0) L.omega = w;
+          }))
+        break;
+    }
+    const double w = L.omega;
+    {
+      double a[2] = {0.0, 0.0};
+      if (on) {
+        x = fma(w, sv, fma(al, p, x));
+        r1 = fma(-w, as, sv);
+        v.r1[row] = r1;  // published: its neighbours read the last one two barriers ago
+        a[0] = r1 * r1;
+        a[1] = r1 * r0;
+      }
+      if (!G.reduce<2>(L, a, 3, [&](const double (&o)[2]) {
+            loop_finish(L, norm0, tol, thr, maxit, timestep, o[0], o[1]);
+          }))
+        break;
+    }
+    if (L.done) break;
+    const double be = L.beta;
+    const bool rst = L.restart != 0;
+    if (on) {  // p here and at the neighbours
+      p = rst ? r1 : fma(be, fma(-w, ap, p), r1);
+      if (rst) r0 = r1;
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        if (R.nb[q] >= 0) {
+          rn[q] = __ldcg(v.r1 + R.nb[q]);
+          pn[q] = rst ? rn[q] : fma(be, fma(-w, an[q], pn[q]), rn[q]);
+        }
+    }
+  }
+  if (on) {
+    v.x[row] = x;
+    v.r0[row] = r0;
+    v.p1[row] = p;
+  }
+  loop_end(L, G);
+}
+
 // bicgstabRe2.hpp:133-153: at the cap, NaN/Inf entries come from the previous solution;
 // if more than 10 % were bad, the whole vector comes from the one before.
 __global__ void __launch_bounds__(kBlock) k_nan_replace(Geo g, double *x, const double *px1, double *part,
@@ -1891,6 +2401,61 @@ void launch_bicg64_part(cudaStream_t s, int part, const Geo &g, const Stencil<do
     case 3: k64_xr<<<cgrid(g), cblock(g), 0, s>>>(g, v, part_buf, sc); break;
     default: k64_p<<<cgrid(g), cblock(g), 0, s>>>(g, v, sc); break;
   }
+}
+
+int loop64_blocks(long long ncell) {
+  if (ncell > kLoopCells) return 0;
+  // per device: 0 not asked yet, else blocks + 1 (a fact of the device and this build)
+  constexpr int kDevices = 64;
+  static std::atomic<int> known[kDevices];
+  int dev = 0, nsm = 0, coop = 0, a = 0, b = 0, c = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return 0;
+  if (const int k = known[dev].load()) return k - 1;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k64_bicg_loop<0>, kLoopBlock, 0) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k64cg_loop, kLoopBlock, 0) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k64_bicg_loop1, kLoopBlock, 0) != cudaSuccess)
+    return 0;
+  const int blocks = coop && a > 0 && b > 0 && c > 0 ? std::min(nsm, kLoopMaxBlocks) : 0;
+  known[dev].store(blocks + 1);
+  return blocks;
+}
+int loop64_iters(long long ncell) {
+  const long long n = (1LL << 26) / (ncell > 0 ? ncell : 1);
+  return (int)(n < 16 ? 16 : (n > 256 ? 256 : n));
+}
+size_t loop64_part_doubles() { return (size_t)kLoopSlots * kLoopMaxBlocks; }
+
+static void launch_loop(cudaStream_t s, bool cg, const Geo &g, const Stencil<double> &st, KrylovVecs<double> v,
+                        double *part_buf, SolverScal *sc, int blocks, int iters) {
+  // whole warps of cells a block, and no more blocks than hold any
+  const long long chunk = ((g.ncell + blocks - 1) / blocks + 31) / 32 * 32;
+  const int nb = (int)((g.ncell + chunk - 1) / chunk);
+  const bool one = !cg && chunk <= kLoopBlock;  // a cell a thread; and a thread for each block's sum
+  auto kernel = cg        ? k64cg_loop
+                : one     ? k64_bicg_loop1
+                : !g.nonuni ? k64_bicg_loop<0>
+                : st.jac  ? k64_bicg_loop<1>
+                          : k64_bicg_loop<2>;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nb);
+  cfg.blockDim = dim3(one ? std::max((int)chunk, (nb + 31) / 32 * 32) : kLoopBlock);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, g, st, v, part_buf, sc, iters, (int)chunk);
+}
+void launch_bicg64_loop(cudaStream_t s, const Geo &g, const Stencil<double> &st, KrylovVecs<double> v,
+                        double *part_buf, SolverScal *sc, int blocks, int iters) {
+  launch_loop(s, false, g, st, v, part_buf, sc, blocks, iters);
+}
+void launch_cg64_loop(cudaStream_t s, const Geo &g, const Stencil<double> &st, KrylovVecs<double> v,
+                      double *part_buf, SolverScal *sc, int blocks, int iters) {
+  launch_loop(s, true, g, st, v, part_buf, sc, blocks, iters);
 }
 
 void launch_bicg32_part(cudaStream_t s, int part, const Geo &g, const Stencil<float> &st,

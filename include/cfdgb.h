@@ -269,7 +269,7 @@ int cfdgb_backward(cfdgb_ctx *ctx, double *dJ_dinlet, double *dJ_deta);
  * GPU that loads the library (17,039,616 bytes, about 17.0 MB: 8 vectors of 2 MiB, block
  * partials and scalars) and shared by all calls, so at most 2^18 = 262,144 unknowns (larger
  * grids: CFDGB_EINVAL), and calls whose work overlaps on the GPU race.  The call polls the
- * solver's convergence from the host, waiting on `stream` every 8 iterations, so a stream
+ * solver's convergence from the host, waiting on `stream` between chunks of iterations, so a stream
  * that is capturing into a CUDA graph is rejected (CFDGB_EINVAL).  The first call on a
  * device looks up the array's device address. */
 int cfdgb_poisson_solve_static(int nx, int ny, int nz, double dx, double dy, double dz, int solver, double tol,
