@@ -177,6 +177,12 @@ struct cfdgb_ctx {
   std::vector<SolverScal> ck_sc;
   std::vector<int> ck_loop;
   std::vector<double *> win;  // 3 padded buffers per window step: u, v, w
+  // cfdgb_forward or cfdgb_backward is running: MIXED solves keep the residual's FMA chain.  The
+  // solid-fraction gradient takes differences of the window's pressure as rounded to FP32, so
+  // other last bits of the solution (its free constant, known to 1e-8 only) move that gradient by
+  // up to 8e-8 of its largest value (14 random inlets on 256x128x32, the integer residual
+  // against the FMA chain): both of its passes and its forward run take one form
+  bool in_adjoint = false;
   std::vector<float *> winp;  // the window steps' pressure, padded, rounded to FP32
   // the adjoint's transposed solve preconditioned by an FP64 V-cycle (contexts with the
   // multigrid preconditioner; built on the first backward)
@@ -752,8 +758,9 @@ int solve_mixed(cfdgb_ctx *c, double tol, int *iters, int *outer, double *relres
   static const bool trace = std::getenv("CFDGB_TRACE") != nullptr;
   const int jacf = jac ? 1 : 0;
   auto residual = [&](int flags, double *rel) -> int {
-    L(c, K_RESID64, 1, [&] {
-      launch_residual64(c->stream, c->nblk, c->g, st64, jacf, c->b, c->x, c->rf, c->part, c->ss, c->sc32, flags);
+    L(c, K_RESID64, residual64_launches(c->g, flags, c->in_adjoint), [&] {
+      launch_residual64(c->stream, c->nsm, c->g, st64, jac ? c->jac32 : c->spe32, jacf, c->b, c->x, c->rf,
+                        c->part, c->ss, c->sc32, flags, c->in_adjoint);
     });
     CK(cudaMemcpyAsync(c->h_ss, c->ss, sizeof(StepScal), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -1315,6 +1322,7 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
   g.nx = nx; g.ny = ny; g.nz = nz;
   g.sx = (long long)ny * nz; g.sy = nz;
   g.ncell = c->ncell;
+  g.hx = c->Dx[2]; g.hy = c->Dy[2]; g.hz = c->Dz[2];
   g.Dx = c->metric; g.Dy = g.Dx + nx; g.Dz = g.Dy + ny;
   g.Dxs = g.Dz + nz; g.Dys = g.Dxs + nx; g.Dzs = g.Dys + ny;
   {  // reciprocals of the metrics and the DFIB face factors, one IEEE division each
@@ -2064,6 +2072,11 @@ int adjoint_solve(cfdgb_ctx *c, const double *rhs, double tol, int *iters) {
 
 }  // namespace
 
+struct InAdjoint {
+  cfdgb_ctx *c;
+  explicit InAdjoint(cfdgb_ctx *ctx) : c(ctx) { c->in_adjoint = true; }
+  ~InAdjoint() { c->in_adjoint = false; }
+};
 int cfdgb_forward(cfdgb_ctx *c, const cfdgb_objective *obj, double *J) {
   if (!c || !obj) return fail(CFDGB_EINVAL, "null argument");
   if (c->cfg.solver == CFDGB_RBSOR)  // the replay and the transposed solve are the Krylov solvers'
@@ -2082,6 +2095,7 @@ int cfdgb_forward(cfdgb_ctx *c, const cfdgb_objective *obj, double *J) {
   if (obj->nsteps < 1 || obj->first < 1 || obj->last < obj->first || obj->last > obj->nsteps || obj->ckpt_every < 1)
     return fail(CFDGB_EINVAL, "bad objective window");
   if (!c->have_fields || c->loop != 0) return fail(CFDGB_ESTATE, "cfdgb_init_fields must come right before");
+  InAdjoint mark(c);
   c->obj = *obj;
   c->fwd_done = false;
   const int K = obj->ckpt_every, nck = (obj->nsteps + K - 1) / K;
@@ -2123,6 +2137,7 @@ int cfdgb_forward(cfdgb_ctx *c, const cfdgb_objective *obj, double *J) {
 int cfdgb_backward(cfdgb_ctx *c, double *dJ_dinlet, double *dJ_deta) {
   if (!c) return fail(CFDGB_EINVAL, "null context");
   if (!c->fwd_done) return fail(CFDGB_ESTATE, "cfdgb_forward must come first");
+  InAdjoint mark(c);
   const cfdgb_objective &obj = c->obj;
   const int K = obj.ckpt_every, nck = (obj.nsteps + K - 1) / K;
   const size_t np = c->npad;

@@ -69,6 +69,7 @@ struct Geo {
   // Apart, because a dt such as 0.002 without the certificate made every division by a
   // certified spacing take five FP64 instructions instead of three
   int div2, div2t;
+  double hx, hy, hz;  // the uniform grid's spacings
   int uni;   // 1: every metric array holds one value (a uniform grid): per-axis factors hoist
 };
 
@@ -143,15 +144,17 @@ __host__ __device__ __forceinline__ double sweep_scale(double r) {
 }
 
 __device__ __forceinline__ float d2f_int(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
-  const unsigned long long a = b & 0x7fffffffffffffffULL;
-  if ((a >> 52) == 0x7ffULL) return __uint_as_float(sign | 0x7f800000u | ((a << 12) ? 0x400000u : 0u));
-  const unsigned long long r = a + 0x0fffffffULL + ((a >> 29) & 1ULL);  // drop 29 bits: nearest, even
-  const int e = (int)(r >> 52) - 896;                                     // FP32 exponent field
-  if (e <= 0) return __uint_as_float(sign);
-  if (e >= 255) return __uint_as_float(sign | 0x7f800000u);
-  return __uint_as_float(sign | ((unsigned)e << 23) | (unsigned)((r >> 29) & 0x7fffffULL));
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), sign = hi & 0x80000000u;
+  const int e = (int)((hi >> 20) & 0x7ffu) - 896;  // FP32 exponent field
+  if ((unsigned)e >= 255u) {  // below the normal FP32 range, beyond it, Inf or NaN
+    if (e < 0) return __uint_as_float(sign);
+    const bool nan = e == 0x7ff - 896 && ((hi & 0xfffffu) | lo) != 0u;
+    return __uint_as_float(sign | 0x7f800000u | (nan ? 0x400000u : 0u));
+  }
+  const unsigned m = ((hi & 0xfffffu) << 3) | (lo >> 29);
+  // drop 29 bits: nearest, even (a carry out of the mantissa raises the exponent, up to Inf)
+  const int f = (int)((unsigned)e << 23) + (int)m + (int)(((lo & 0x1fffffffu) + 0x0fffffffu + (m & 1u)) >> 29);
+  return __uint_as_float(f < 0x00800000 ? sign : sign | (unsigned)f);
 }
 
 // float -> double, exact, by integer operations (FP32 subnormals, never met here, read as zero)
@@ -161,6 +164,28 @@ __device__ __forceinline__ double f2d_int(float x) {
   if (e == 0u) return __hiloint2double((int)(b & 0x80000000u), 0);
   const unsigned eh = e == 0xffu ? 0x7ffu : e + 896u;
   return __hiloint2double((int)((b & 0x80000000u) | (eh << 20) | ((b >> 3) & 0xfffffu)), (int)(b << 29));
+}
+
+// a double to a 64-bit integer in units of 2^(em - 1082), em >= its exponent field (truncated;
+// |q| < 2^60), by integer operations
+__device__ __forceinline__ long long d2fix(double x, int em) {
+  const int hi = __double2hiint(x);
+  const unsigned long long m =
+      ((unsigned long long)(unsigned)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(x);
+  const int s = min(em - ((hi >> 20) & 0x7ff), 63);  // zeros and subnormals: em >= 200, nothing is left
+  const long long q = (long long)((m << 7) >> s), n = (long long)(hi >> 31);
+  return (q ^ n) - n;
+}
+// a 64-bit integer below 2^62, times 2^shift, to the nearest double by integer operations (the
+// result is a normal number or zero)
+__device__ __forceinline__ double fix2d(long long t, int shift) {
+  if (t == 0) return 0.0;
+  unsigned long long a = (unsigned long long)(t < 0 ? -t : t);
+  const int lz = __clzll((long long)a);
+  a = (a << lz) >> 1;  // bit 62 the leading one
+  a = (a + 0x1ffu + ((a >> 10) & 1u)) >> 10;
+  const unsigned long long b = ((unsigned long long)(1085 - lz + shift) << 52) + a;
+  return __longlong_as_double((long long)(b | ((unsigned long long)t & 0x8000000000000000ULL)));
 }
 
 // compact row -> padded (i,j,k).  Grids below 2^31 cells divide in 32 bits: a 64-bit
@@ -367,7 +392,8 @@ struct StepScal {
   double oflux;    // convective outflow: the outlet correction (net boundary flux / outlet area)
   int hist;        // Adams-Bashforth: increments stored by the steps since init (at most 2)
   int hslot;       // Adams-Bashforth order 3: the history slot that holds the last increment
-  int nan_flag, pad;
+  int nan_flag;
+  unsigned xexp;   // MIXED: the largest exponent field of the solution x (k_residual_fx), 0: unknown
   unsigned cnt[10];
 };
 
