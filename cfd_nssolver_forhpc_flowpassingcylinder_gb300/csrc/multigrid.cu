@@ -16,6 +16,7 @@
 // has stopped.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -542,406 +543,386 @@ __global__ void __launch_bounds__(kBlock) k_mgp_prolong(MgLevelT<double> F, MgLe
   }
 }
 
-// ---- a level whose every axis halves, FP32 quads (nz / 4 a power of two up to 16): its
-// V-cycle work in two marching kernels instead of six per-pass launches.  A block of
-// nz / 4 x (mty + 4) threads owns a band of mty rows and two halo rows on each side (a
-// thread: one quad of one row) and marches along x over a segment of msx planes and two halo
-// planes on each side.  A thread keeps its planes in registers (rings of three, rotated by
-// unrolling); each stage's plane passes through shared memory for the y neighbours (three
-// buffers per stage, so one barrier a plane; rows outside the level hold zeros there) and
-// the z neighbours across quads by shuffles.  The arithmetic runs on cell pairs (FP32x2).
-//   k_mg_down4: the pre-smoothing from zero (colour 0: b / diag; colour 1 from those), the
-//     residual and its restriction to the next level's b.  The level's x is not stored: the
-//     only part of it read later, colour 0's, is b / diag again.
-//   k_mg_up4: colour 0 = b / diag + P xc, then the colour-1 and colour-0 passes of the
+// ---- a level whose every axis halves, FP32, nz / 4 up to kMgMarchQuads: its V-cycle work in
+// two marching kernels instead of six per-pass launches.  A block of nz / 4 x (mty / 2 + 2)
+// threads owns a band of mty rows and two halo rows on each side (a thread: one quad along k of
+// two rows, j even and j + 1) and marches along x over a segment of msx planes and two halo
+// planes on each side.  The cells of one colour in a quad are a pair: the even or the odd ones,
+// by the row's parity (E, O below), known at compile time since the rows are j even and odd and
+// the planes are unrolled.  The x and y neighbours of one colour's pair are the other colour's
+// pairs of the planes and rows beside it, its z neighbours that pair itself and the same
+// shifted by one, so every colour pass is FP32x2 arithmetic on the cells of its colour only.
+// A thread's own planes stay in registers (rings of three); the neighbours' rows and quads come
+// from shared memory, two buffers a colour and one barrier a plane:
+//   step p: colour 0 of plane p, colour 1 of plane p - 1, the last stage of plane p - 2, from
+//   the neighbours' pairs of the planes that the step before wrote.
+//   k_mg_down: the pre-smoothing from zero (colour 0: b / diag; colour 1 from those), the
+//     residual (colour 1's from its update's own neighbour sum) and its restriction to the
+//     next level's b.  The level's x is not stored: the only part of it read later, colour
+//     0's, is b / diag again.
+//   k_mg_up: colour 0 = b / diag + P xc, then the colour-1 and colour-0 passes of the
 //     post-smoothing; x stored.
-// Neighbours beyond a wall enter as zeros (the registers of planes and the shared rows
-// outside the level hold zeros).  Each value is otherwise formed by the rounded sequence of
-// k_mg_smooth4, k_mg_restrict8 or k_mg_prolong8 (the pair operations round each component
-// as the scalar ones do), so a V-cycle gives the per-pass kernels' result (equal as
+// Neighbours beyond a wall enter as zeros.  Each value is otherwise formed by the rounded
+// sequence of k_mg_smooth4, k_mg_restrict8 or k_mg_prolong8 (the pair operations round each
+// component as the scalar ones do), so a V-cycle gives the per-pass kernels' result (equal as
 // numbers: a sum of two zeros may differ in sign).
-constexpr int kMgMarchThreads = 320;
+constexpr int kMgMarchThreads = 512;
+constexpr int kMgMarchQuads = 128;  // at least four row pairs a block
 
 __device__ __forceinline__ float2 pr(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 bc2(float a) { return make_float2(a, a); }
+// a product that enters a sum: scalar, since the compiler contracts a pair product that feeds a
+// pair sum into one FFMA2 (results different from the per-pass kernels' rounded product)
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return pr(mul_rn(a.x, b.x), mul_rn(a.y, b.y)); }
+// (scalar: the prolongation's operands are not aligned register pairs)
+__device__ __forceinline__ float2 fma2s(float2 a, float2 b, float2 c) {
+  return pr(fma_rn(a.x, b.x, c.x), fma_rn(a.y, b.y, c.y));
+}
 // wsum of two cells
 __device__ __forceinline__ float2 wsum2(const MgLevel &L, float2 a, float2 e, float2 f) {
   return __ffma2_rn(bc2(L.wz), f, __ffma2_rn(bc2(L.wy), e, __fmul2_rn(bc2(L.wx), a)));
 }
 
-// a thread's row and quad, and what does not change along the march
-struct MarchRow {
-  unsigned mask;      // the lanes of this warp that exist
-  int left, right;    // lanes of the quads before and after this one in its row (wrapping)
-  int q, tj, j, k0;
-  bool jin, jm, jp;   // the row exists; its neighbours along y exist
-  bool zl, zr;        // the quad has a z neighbour before / after it (or across the wrap)
-  float wycy;         // wy cy (exact: cy in 0..2)
-  float2 wz01, wz23;  // wz cz of the quad's cells (exact)
-  int cy3, cz0, cz3;  // 3 cy; cz of the end cells (the middle ones have cz = 2)
-  // 1/diag of the quad's cells on a plane with 9 cx = c9
-  __device__ __forceinline__ float2 idg01(const MgLevel &L, int c9) const {
-    return pr(L.idg[c9 + cy3 + cz0], L.idg[c9 + cy3 + 2]);
+// 1/diag (x, y) and the diagonal (z, w) of a quad's even or odd cells, in shared memory by
+// [one x neighbour or two][y neighbours, 3: a row beyond the level (1/diag 0: colour 1 is zero
+// there)][z neighbour before][after][even, odd]; one entry serves all threads of a kind (as
+// registers, with a branch at the first and last plane: 17 % slower on 512x256x64)
+struct MarchDiag {
+  float4 v[2][4][2][2][2];
+};
+__device__ __forceinline__ void march_diag(const MgLevel &L, MarchDiag &D) {
+  for (int t = threadIdx.x; t < 64; t += blockDim.x) {
+    const int odd = t & 1, zr = (t >> 1) & 1, zl = (t >> 2) & 1, cy = (t >> 3) & 3, cx = 1 + (t >> 5);
+    float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (cy < 3) {
+      const int c = 9 * cx + 3 * cy, c0 = odd ? 2 : 1 + zl, c1 = odd ? 1 + zr : 2;
+      const float dxy = add_rn(L.wx * (float)cx, L.wy * (float)cy);  // the products are exact
+      d = make_float4(L.idg[c + c0], L.idg[c + c1], add_rn(dxy, L.wz * (float)c0), add_rn(dxy, L.wz * (float)c1));
+    }
+    (&D.v[0][0][0][0][0])[t] = d;
   }
-  __device__ __forceinline__ float2 idg23(const MgLevel &L, int c9) const {
-    return pr(L.idg[c9 + cy3 + 2], L.idg[c9 + cy3 + cz3]);
+}
+
+// a thread's rows and quad, and what does not change along the march
+struct MarchRows {
+  int q, ty, j;       // j: the even row (-2: below the level)
+  bool in, band;      // the rows exist; and belong to the band
+  bool zl, zr;        // the quad has a z neighbour before / after it (or across the wrap)
+  int im, ip, il, ir; // threads of the rows below and above, of the quads before and after
+  int d[2];           // the rows' entries of MarchDiag (even cells, one x neighbour)
+  // row r's even (odd = 0) or odd cells on plane i
+  __device__ __forceinline__ float4 diag(const MgLevel &L, const MarchDiag &D, int r, int odd, int i) const {
+    return (&D.v[0][0][0][0][0])[d[r] + (i > 0 && i < L.nx - 1 ? 32 : 0) + odd];  // (a march has nx >= 2)
   }
 };
 
-template <int NQ>
-__device__ __forceinline__ MarchRow march_row(const MgLevel &L) {
-  MarchRow R;
-  const int w0 = threadIdx.x & ~31, n = min(32, (int)blockDim.x - w0);
-  R.mask = n >= 32 ? 0xffffffffu : ((1u << n) - 1u);
-  R.q = threadIdx.x % NQ;
-  R.tj = threadIdx.x / NQ;
-  R.k0 = 4 * R.q;
-  const int row0 = (threadIdx.x & 31) - R.q;  // a row's NQ lanes lie in one warp (NQ divides 32)
-  R.left = row0 + ((R.q - 1) & (NQ - 1));
-  R.right = row0 + ((R.q + 1) & (NQ - 1));
-  R.j = blockIdx.y * L.mty - 2 + R.tj;
-  R.jin = R.j >= 0 && R.j < L.ny;
-  R.jm = R.j > 0;
-  R.jp = R.j < L.ny - 1;
+__device__ __forceinline__ MarchRows march_rows(const MgLevel &L) {
+  MarchRows R;
+  const int nq = L.nz >> 2, tid = threadIdx.x, rows = blockDim.x / nq;
+  R.ty = tid / nq;
+  R.q = tid - R.ty * nq;
+  R.j = blockIdx.y * L.mty - 2 + 2 * R.ty;
+  R.in = R.j >= 0 && R.j < L.ny;  // ny is even: both rows or neither
+  R.band = R.in && R.ty >= 1 && R.ty < rows - 1;
   R.zl = R.q > 0 || L.pz;
-  R.zr = R.q < NQ - 1 || L.pz;
-  const int cy = (int)R.jm + (int)R.jp;
-  R.wycy = L.wy * (float)cy;
-  R.cy3 = 3 * cy;
-  R.cz0 = zcount(L, R.k0);
-  R.cz3 = zcount(L, R.k0 + 3);
-  R.wz01 = pr(L.wz * (float)R.cz0, 2.f * L.wz);
-  R.wz23 = pr(2.f * L.wz, L.wz * (float)R.cz3);
+  R.zr = R.q < nq - 1 || L.pz;
+  // (the outer halo rows' missing neighbours: any value, used by no row that is)
+  R.im = R.ty > 0 ? tid - nq : tid;
+  R.ip = R.ty < rows - 1 ? tid + nq : tid;
+  R.il = R.q > 0 ? tid - 1 : tid + nq - 1;
+  R.ir = R.q < nq - 1 ? tid + 1 : tid + 1 - nq;
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+    R.d[r] = 8 * (R.in ? (R.j + r > 0) + (R.j + r < L.ny - 1) : 3) + 4 * (int)R.zl + 2 * (int)R.zr;
   return R;
 }
 
-__device__ __forceinline__ void unq(const float4 v, float (&o)[4]) {
-  o[0] = v.x;
-  o[1] = v.y;
-  o[2] = v.z;
-  o[3] = v.w;
+// the pairs beside a colour's cells along z: own, the other colour's pair of the quad; nb, the
+// one that lies beyond the quad (odd: the cells are the odd ones, else the even ones)
+__device__ __forceinline__ float2 march_z(int odd, float2 own, float nb) {
+  return odd ? __fadd2_rn(own, pr(own.y, nb)) : __fadd2_rn(pr(nb, own.x), own);
 }
-__device__ __forceinline__ float4 mkq(const float (&o)[4]) { return make_float4(o[0], o[1], o[2], o[3]); }
-
-// wx cx + wy cy of plane i (the diagonal less its z part) and 9 cx
-__device__ __forceinline__ float march_dxy(const MgLevel &L, const MarchRow &R, int i, int &c9) {
-  const int cx = (int)(i > 0) + (int)(i < L.nx - 1);
-  c9 = 9 * cx;
-  return fma_rn(L.wx, (float)cx, R.wycy);
+// that value: the last cell of the quad before or the first of the one after, zero beyond a wall
+__device__ __forceinline__ float march_zn(const MarchRows &R, int odd, const float2 *s) {
+  return odd ? (R.zr ? s[R.ir].x : 0.f) : (R.zl ? s[R.il].y : 0.f);
 }
+__device__ __forceinline__ float2 lo2(float4 v) { return pr(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return pr(v.z, v.w); }
+__device__ __forceinline__ float2 neg2(float2 v) { return pr(-v.x, -v.y); }
 
-// the z neighbours of a quad's end cells from the neighbouring lanes (every lane calls it)
-__device__ __forceinline__ void march_kz(const MarchRow &R, const float (&v)[4], float &kl, float &kr) {
-  const float l = __shfl_sync(R.mask, v[3], R.left), r = __shfl_sync(R.mask, v[0], R.right);
-  kl = R.zl ? l : 0.f;
-  kr = R.zr ? r : 0.f;
-}
-
-// b of a quad's cell pairs, times the diagonal for Jacobi-scaled rows (BS).  The product
-// stays scalar: its FP32x2 form gave results different from the per-pass kernels on the
-// Jacobi-scaled runs (measured; the pair operations alone round as the scalar ones do, and
-// the cause was not found), the scalar form gives identical ones.
-template <bool BS>
-__device__ __forceinline__ void march_bb(const MarchRow &R, float dxy, const float (&bv)[4], float2 &b01,
-                                         float2 &b23) {
-  if (BS) {
-    b01 = pr(mul_rn(bv[0], dxy + R.wz01.x), mul_rn(bv[1], dxy + R.wz01.y));
-    b23 = pr(mul_rn(bv[2], dxy + R.wz23.x), mul_rn(bv[3], dxy + R.wz23.y));
-  } else {
-    b01 = pr(bv[0], bv[1]);
-    b23 = pr(bv[2], bv[3]);
+// the march over planes p = is - 2 .. ie + 1, six at a time: the planes' parity and the places
+// in the rings of three are compile-time
+#define CFDGB_MARCH_PLANES(STEP)                             \
+  for (int p = is - 2;;) {                                   \
+    STEP(p, std::integral_constant<int, 0>{});               \
+    if (++p > ie + 1) break;                                 \
+    STEP(p, std::integral_constant<int, 1>{});               \
+    if (++p > ie + 1) break;                                 \
+    STEP(p, std::integral_constant<int, 2>{});               \
+    if (++p > ie + 1) break;                                 \
+    STEP(p, std::integral_constant<int, 3>{});               \
+    if (++p > ie + 1) break;                                 \
+    STEP(p, std::integral_constant<int, 4>{});               \
+    if (++p > ie + 1) break;                                 \
+    STEP(p, std::integral_constant<int, 5>{});               \
+    if (++p > ie + 1) break;                                 \
+    six();                                                   \
   }
-}
 
-// colour 0 of a quad after the pre-smoothing from zero (k_mg_smooth4's zero pass): b / diag
-// on colour 0, zero on colour 1
 template <bool BS>
-__device__ __forceinline__ void march_zero(const MgLevel &L, const MarchRow &R, float dxy, int c9, int t0,
-                                           const float (&bv)[4], float (&o)[4]) {
-  float2 b01, b23;
-  march_bb<BS>(R, dxy, bv, b01, b23);
-  const float2 v01 = __fmul2_rn(b01, R.idg01(L, c9)), v23 = __fmul2_rn(b23, R.idg23(L, c9));
-  o[0] = t0 ? 0.f : v01.x;
-  o[1] = t0 ? v01.y : 0.f;
-  o[2] = t0 ? 0.f : v23.x;
-  o[3] = t0 ? v23.y : 0.f;
-}
-
-// One colour pass of k_mg_smooth4 on a quad (its non-zero form): the cells of colour t0's
-// parity (t0: the first such cell) from the neighbours' values, the others kept.  xm, xp:
-// the quad on the planes before and after; ym, yp: rows j -1, j + 1; kl, kr: the cells
-// beyond the quad's ends.
-template <bool BS>
-__device__ __forceinline__ void march_pass(const MgLevel &L, const MarchRow &R, float dxy, int c9, int t0,
-                                           const float (&bv)[4], const float (&xv)[4], const float (&xm)[4],
-                                           const float (&xp)[4], const float4 ym, const float4 yp, float kl, float kr,
-                                           float (&o)[4]) {
-  float2 b01, b23;
-  march_bb<BS>(R, dxy, bv, b01, b23);
-  const float2 s01 = wsum2(L, __fadd2_rn(pr(xm[0], xm[1]), pr(xp[0], xp[1])), __fadd2_rn(pr(ym.x, ym.y), pr(yp.x, yp.y)),
-                           __fadd2_rn(pr(kl, xv[0]), pr(xv[1], xv[2])));
-  const float2 s23 = wsum2(L, __fadd2_rn(pr(xm[2], xm[3]), pr(xp[2], xp[3])), __fadd2_rn(pr(ym.z, ym.w), pr(yp.z, yp.w)),
-                           __fadd2_rn(pr(xv[1], xv[2]), pr(xv[3], kr)));
-  const float2 v01 = __fmul2_rn(__fadd2_rn(b01, s01), R.idg01(L, c9));
-  const float2 v23 = __fmul2_rn(__fadd2_rn(b23, s23), R.idg23(L, c9));
-  o[0] = t0 ? xv[0] : v01.x;
-  o[1] = t0 ? v01.y : xv[1];
-  o[2] = t0 ? xv[2] : v23.x;
-  o[3] = t0 ? v23.y : xv[3];
-}
-
-template <int NQ, bool BS>
-__global__ void __launch_bounds__(kMgMarchThreads, 2)
-    k_mg_down4(MgLevel F, MgLevel Cl, const float *__restrict__ b, float *__restrict__ bc, const SolverScal *sc) {
+__global__ void __launch_bounds__(kMgMarchThreads)
+    k_mg_down(MgLevel F, MgLevel Cl, const float *__restrict__ b, float *__restrict__ bc, const SolverScal *sc) {
   pdl_wait();
   if (sc->done) return;
   pdl_trigger();
-  constexpr int NZ = 4 * NQ;
-  const int RY = F.mty + 4, PL = RY * NQ;
-  extern __shared__ float4 msm[];
-  float4 *const sa = msm + threadIdx.x, *const sb = msm + 3 * PL + threadIdx.x;  // colour 0 / both
-  const MarchRow R = march_row<NQ>(F);
+  // the pairs of both rows of every thread: [buffer][row][thread]
+  __shared__ float2 s0[2][2][kMgMarchThreads], s1[2][2][kMgMarchThreads];
+  __shared__ MarchDiag D;
+  const int tid = threadIdx.x;
+  const MarchRows R = march_rows(F);
+  march_diag(F, D);
+  __syncthreads();
   const int is = blockIdx.x * F.msx, ie = min(F.nx, is + F.msx);
-  const bool blk = R.jin && R.tj >= 1 && R.tj < RY - 1;  // colour 1: the band and one halo row
-  const bool res = R.jin && R.tj >= 2 && R.tj < RY - 2;  // residual: the band
-  const bool even = !(R.j & 1);
-  const int sx = F.ny * NZ, o = (R.jin ? R.j : 0) * NZ + R.k0;  // 32-bit: under 2^31 cells
-  auto ldb = [&](int p) -> float4 {
-    return R.jin && p >= 0 && p < F.nx ? __ldg(reinterpret_cast<const float4 *>(b + (o + p * sx)))
-                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int sx = F.ny * F.nz, o = (R.in ? R.j : 0) * F.nz + 4 * R.q;  // 32-bit: under 2^31 cells
+  auto ldb = [&](int p, int r) -> float4 {
+    return R.in && p >= 0 && p < F.nx ? __ldg(reinterpret_cast<const float4 *>(b + (o + r * F.nz + p * sx)))
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
   };
-  float4 bn1 = ldb(is - 2), bn2 = ldb(is - 1);
-  float bA[4] = {}, bB[4] = {}, bC[4] = {};  // b of planes p, p-1, p-2 (rotating)
-  float xA[4] = {}, xB[4] = {}, xC[4] = {};  // colour 0 from zero, planes p, p-1, p-2
-  float fA[4] = {}, fB[4] = {}, fC[4] = {};  // both colours, planes p-1, p-2, p-3
-  float sA = 0.f, sB = 0.f;  // the restriction sums of the quad's two coarse cells (even rows)
-  // s0, s1, s2: the shared slots of planes p, p - 1, p - 2
-  auto step = [&](int p, float(&b0)[4], float(&b1)[4], float(&b2)[4], float(&x0)[4], float(&x1)[4],
-                  float(&x2)[4], float(&f1)[4], float(&f2)[4], float(&f3)[4], int s0, int s1, int s2) {
-    // plane p: b, and colour 0 from zero (zeros outside the level)
-    unq(bn1, b0);
-    bn1 = bn2;
-    bn2 = ldb(p + 2);
-    {
-      int c9;
-      const float dxy = march_dxy(F, R, p, c9);
-      march_zero<BS>(F, R, dxy, c9, (p + R.j) & 1, b0, x0);
-      sa[s0 * PL] = mkq(x0);
-    }
-    __syncthreads();
-    {  // plane p - 1: colour 1 from colour 0
-      const int i = p - 1;
-      float kl, kr;
-      march_kz(R, x1, kl, kr);
-      if (blk && i >= 0 && i < F.nx) {
-        int c9;
-        const float dxy = march_dxy(F, R, i, c9);
-        const float4 *s = sa + s1 * PL;
-        march_pass<BS>(F, R, dxy, c9, (i + R.j + 1) & 1, b1, x1, x2, x0, s[-NQ], s[NQ], kl, kr, f1);
-      } else {
+  float4 bn[2][2];  // b of the next two planes
+  float2 b0[3][2], b1[3][2], c0[3][2], c1[3][2], r1[3][2];  // b, x of each colour, colour 1's residual
 #pragma unroll
-        for (int c = 0; c < 4; ++c) f1[c] = x1[c];
+  for (int r = 0; r < 2; ++r) {
+    bn[0][r] = ldb(is - 2, r);
+    bn[1][r] = ldb(is - 1, r);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) b0[t][r] = b1[t][r] = c0[t][r] = c1[t][r] = r1[t][r] = pr(0.f, 0.f);
+  }
+  float2 S = pr(0.f, 0.f);  // the restriction sums of the quad's two coarse cells
+  auto step = [&](int p, auto u) {
+    constexpr int U = decltype(u)::value, P = U % 3, Q = (U + 2) % 3, T = (U + 1) % 3, W = U & 1;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {  // plane p: b, and colour 0 from zero (zeros outside the level)
+      const int par = W ^ r;
+      const float4 v = bn[W][r], d = R.diag(F, D, r, par, p);
+      bn[W][r] = ldb(p + 2, r);
+      b0[P][r] = par ? pr(v.y, v.w) : pr(v.x, v.z);
+      b1[P][r] = par ? pr(v.x, v.z) : pr(v.y, v.w);
+      if (BS) {  // Jacobi-scaled rows
+        b0[P][r] = mul2(b0[P][r], hi2(d));
+        b1[P][r] = mul2(b1[P][r], hi2(R.diag(F, D, r, 1 - par, p)));
       }
-      sb[s1 * PL] = mkq(f1);
+      c0[P][r] = mul2(b0[P][r], lo2(d));
     }
-    {  // plane p - 2: the residual b - A x, restricted (k_mg_restrict8's sums)
-      const int i = p - 2;
-      float kl, kr;
-      march_kz(R, f2, kl, kr);
-      const bool act = res && i >= is && i < ie;
-      float2 r01 = make_float2(0.f, 0.f), r23 = r01;
-      if (act) {
-        int c9;
-        const float dxy = march_dxy(F, R, i, c9);
-        const float4 *s = sb + s2 * PL;
-        const float4 ym = s[-NQ], yp = s[NQ];
-        float2 b01, b23;
-        march_bb<BS>(R, dxy, b2, b01, b23);
-        const float2 d01 = __fadd2_rn(bc2(dxy), R.wz01), d23 = __fadd2_rn(bc2(dxy), R.wz23);  // ldiag
-        const float2 s01 = wsum2(F, __fadd2_rn(pr(f3[0], f3[1]), pr(f1[0], f1[1])),
-                                 __fadd2_rn(pr(ym.x, ym.y), pr(yp.x, yp.y)), __fadd2_rn(pr(kl, f2[0]), pr(f2[1], f2[2])));
-        const float2 s23 = wsum2(F, __fadd2_rn(pr(f3[2], f3[3]), pr(f1[2], f1[3])),
-                                 __fadd2_rn(pr(ym.z, ym.w), pr(yp.z, yp.w)), __fadd2_rn(pr(f2[1], f2[2]), pr(f2[3], kr)));
-        r01 = __fadd2_rn(__ffma2_rn(pr(-d01.x, -d01.y), pr(f2[0], f2[1]), b01), s01);
-        r23 = __fadd2_rn(__ffma2_rn(pr(-d23.x, -d23.y), pr(f2[2], f2[3]), b23), s23);
-      }
-      // children (a, e, c) of a coarse cell summed in k_mg_restrict8's order: the odd row's
-      // residuals by shuffle
-      const float o0 = __shfl_down_sync(R.mask, r01.x, NQ), o1 = __shfl_down_sync(R.mask, r01.y, NQ);
-      const float o2 = __shfl_down_sync(R.mask, r23.x, NQ), o3 = __shfl_down_sync(R.mask, r23.y, NQ);
-      if (act && even) {
-        if (!(i & 1)) {
-          sA = 0.f;
-          sB = 0.f;
+    {  // plane p - 1: colour 1 from colour 0, and its residual from the same neighbour sum
+      const int i = p - 1;
+      if (i >= 0 && i < F.nx) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int odd = W ^ r;  // the row's colour-0 cells on plane i are the other ones
+          const float2 a = __fadd2_rn(c0[T][r], c0[P][r]);
+          const float2 e = __fadd2_rn(r ? c0[Q][0] : s0[1 - W][1][R.im], r ? s0[1 - W][0][R.ip] : c0[Q][1]);
+          const float2 w = wsum2(F, a, e, march_z(odd, c0[Q][r], march_zn(R, odd, s0[1 - W][r])));
+          const float4 d = R.diag(F, D, r, odd, i);
+          c1[Q][r] = mul2(__fadd2_rn(b1[Q][r], w), lo2(d));
+          r1[Q][r] = __fadd2_rn(__ffma2_rn(neg2(hi2(d)), c1[Q][r], b1[Q][r]), w);
         }
-        sA = add_rn(add_rn(add_rn(add_rn(sA, r01.x), r01.y), o0), o1);
-        sB = add_rn(add_rn(add_rn(add_rn(sB, r23.x), r23.y), o2), o3);
-        if (i & 1) {
+      } else {
+        c1[Q][0] = c1[Q][1] = pr(0.f, 0.f);
+      }
+    }
+    {  // plane p - 2: colour 0's residual, and the restriction (k_mg_restrict8's sums)
+      const int i = p - 2;
+      if (i >= is) {
+        if (!W) S = pr(0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int odd = W ^ r;
+          const float2 a = __fadd2_rn(c1[P][r], c1[Q][r]);
+          const float2 e = __fadd2_rn(r ? c1[T][0] : s1[W][1][R.im], r ? s1[W][0][R.ip] : c1[T][1]);
+          const float2 w = wsum2(F, a, e, march_z(odd, c1[T][r], march_zn(R, odd, s1[W][r])));
+          const float2 d = hi2(R.diag(F, D, r, odd, i));
+          const float2 r0 = __fadd2_rn(__ffma2_rn(neg2(d), c0[T][r], b0[T][r]), w);
+          S = __fadd2_rn(__fadd2_rn(S, odd ? r1[T][r] : r0), odd ? r0 : r1[T][r]);
+        }
+        if (W && R.band) {
           const float inv = 1.f / 8.f;
           *reinterpret_cast<float2 *>(bc + lrow(Cl, i >> 1, R.j >> 1, 2 * R.q)) =
-              make_float2(mul_rn(sA, inv), mul_rn(sB, inv));
+              make_float2(mul_rn(S.x, inv), mul_rn(S.y, inv));
         }
       }
     }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      s0[W][r][tid] = c0[P][r];
+      s1[1 - W][r][tid] = c1[Q][r];
+    }
+    __syncthreads();
   };
-  for (int p = is - 2;;) {
-    step(p, bA, bC, bB, xA, xC, xB, fA, fC, fB, 0, 2, 1);
-    if (++p > ie + 1) break;
-    step(p, bB, bA, bC, xB, xA, xC, fB, fA, fC, 1, 0, 2);
-    if (++p > ie + 1) break;
-    step(p, bC, bB, bA, xC, xB, xA, fC, fB, fA, 2, 1, 0);
-    if (++p > ie + 1) break;
-  }
+  auto six = [] {};
+  CFDGB_MARCH_PLANES(step)
 }
 
-// a coarse plane's values for a quad's prolongation: rows pj, nj (the parent row and the
-// neighbour on the child's side) x coarse z 2q - 1, 2q, 2q + 1, 2q + 2, the ends the parent
-// beyond a wall or wrapped (k_mg_prolong8's taps); raw: the float2 pairs of the two rows
-__device__ __forceinline__ void march_zext(const MarchRow &R, float4 raw, float (&o)[2][4]) {
-  const float l0 = __shfl_sync(R.mask, raw.y, R.left), l1 = __shfl_sync(R.mask, raw.w, R.left);
-  const float r0 = __shfl_sync(R.mask, raw.x, R.right), r1 = __shfl_sync(R.mask, raw.z, R.right);
-  o[0][0] = R.zl ? l0 : raw.x;
-  o[0][1] = raw.x;
-  o[0][2] = raw.y;
-  o[0][3] = R.zr ? r0 : raw.y;
-  o[1][0] = R.zl ? l1 : raw.z;
-  o[1][1] = raw.z;
-  o[1][2] = raw.w;
-  o[1][3] = R.zr ? r1 : raw.w;
-}
-
-template <int NQ, bool BS>
-__global__ void __launch_bounds__(kMgMarchThreads, 2)
-    k_mg_up4(MgLevel F, MgLevel Cl, const float *__restrict__ b, const float *__restrict__ xc, float *__restrict__ x,
-             const SolverScal *sc) {
+template <bool BS>
+__global__ void __launch_bounds__(kMgMarchThreads)
+    k_mg_up(MgLevel F, MgLevel Cl, const float *__restrict__ b, const float *__restrict__ xc, float *__restrict__ x,
+            const SolverScal *sc) {
   pdl_wait();
   if (sc->done) return;
   pdl_trigger();
-  constexpr int NZ = 4 * NQ;
-  const int RY = F.mty + 4, PL = RY * NQ;
-  extern __shared__ float4 msm[];
-  float4 *const sa = msm + threadIdx.x, *const sb = msm + 3 * PL + threadIdx.x;  // colour 0 / both
-  const MarchRow R = march_row<NQ>(F);
+  __shared__ float2 s0[2][2][kMgMarchThreads], s1[2][2][kMgMarchThreads];
+  __shared__ float2 sc_[kMgMarchThreads + 2 * kMgMarchQuads];  // a coarse plane: the rows' parents, one row more on each side
+  __shared__ MarchDiag D;
+  const int tid = threadIdx.x, nq = F.nz >> 2;
+  const MarchRows R = march_rows(F);
+  march_diag(F, D);
   const int is = blockIdx.x * F.msx, ie = min(F.nx, is + F.msx);
-  const bool one = R.jin && R.tj >= 1 && R.tj < RY - 1;   // colour 1: the band and one halo row
-  const bool zero = R.jin && R.tj >= 2 && R.tj < RY - 2;  // colour 0, stored: the band
-  // 32-bit offsets: a marching level has fewer than 2^31 cells (mg_plan)
-  const int sx = F.ny * NZ, o = (R.jin ? R.j : 0) * NZ + R.k0;
-  auto ldb = [&](int p) -> float4 {
-    return R.jin && p >= 0 && p < F.nx ? __ldg(reinterpret_cast<const float4 *>(b + (o + p * sx)))
-                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int sx = F.ny * F.nz, o = (R.in ? R.j : 0) * F.nz + 4 * R.q;  // 32-bit: under 2^31 cells
+  auto ldb = [&](int p, int r) -> float4 {
+    return R.in && p >= 0 && p < F.nx ? __ldg(reinterpret_cast<const float4 *>(b + (o + r * F.nz + p * sx)))
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
   };
-  // prolongation taps along y: the parent row and the neighbour on the child's side
-  const int jc = min(max(R.j, 0), F.ny - 1), pj = jc >> 1;
-  const int nj = (jc & 1) ? min(pj + 1, Cl.ny - 1) : max(pj - 1, 0);
-  const int co = pj * Cl.nz + 2 * R.q, cd = (nj - pj) * Cl.nz, csx = Cl.ny * Cl.nz;
-  auto ldc = [&](int m) -> float4 {  // coarse plane m (clamped to the level), rows pj and nj
-    const int r = min(max(m, 0), Cl.nx - 1) * csx + co;
-    const float2 u = __ldg(reinterpret_cast<const float2 *>(xc + r));
-    const float2 v = __ldg(reinterpret_cast<const float2 *>(xc + (r + cd)));
-    return make_float4(u.x, u.y, v.x, v.y);
+  // the parents of the thread's rows (a coarse row, clamped to the level) and, in the first and
+  // last rows of threads, the coarse row before and after
+  const int pj = R.j >> 1, csx = Cl.ny * Cl.nz, c2 = 2 * R.q;
+  const bool first = R.ty == 0, last = tid + nq >= (int)blockDim.x;
+  const int co = min(max(pj, 0), Cl.ny - 1) * Cl.nz + c2;
+  const int cx = min(max(first ? pj - 1 : pj + 1, 0), Cl.ny - 1) * Cl.nz + c2;
+  float2 n0, n1 = pr(0.f, 0.f);  // the next coarse plane on its way
+  auto ldc = [&](int m) {
+    const int t = min(max(m, 0), Cl.nx - 1) * csx;
+    n0 = __ldg(reinterpret_cast<const float2 *>(xc + (t + co)));
+    if (first || last) n1 = __ldg(reinterpret_cast<const float2 *>(xc + (t + cx)));
   };
-  // coarse planes m - 1 and m around the parent plane m = p / 2 of the fine plane p (raw
-  // pairs, extended at each use), and m + 1 in flight during the parent's first child (is - 2
-  // is even: the march starts on a first child)
-  const int m0 = (is - 2) >> 1;
-  float4 ca = ldc(m0 - 1), cb = ldc(m0), cn = cb;
-  float4 bn1 = ldb(is - 2), bn2 = ldb(is - 1);
-  float bA[4] = {}, bB[4] = {}, bC[4] = {};  // b of planes p, p-1, p-2 (rotating)
-  // the earlier planes of both stages are read back from this thread's own shared slots
-  // (registers are this kernel's limit); zeros before the march, as the planes before it
+  auto putc = [&] {
+    sc_[tid + nq] = n0;
+    if (first) sc_[tid] = n1;
+    if (last) sc_[tid + 2 * nq] = n1;
+  };
+  // a coarse plane's values for the quad: rows pj, pj - 1, pj + 1 x coarse z 2q - 1 .. 2q + 2, the
+  // ends the parent beyond a wall or wrapped (k_mg_prolong8's taps)
+  const float *const cf = reinterpret_cast<const float *>(sc_);
+  const int kl = R.zl ? 2 * R.il + 1 : 2 * tid, kr = R.zr ? 2 * R.ir : 2 * tid + 1;
+  auto getc = [&](float (&v)[3][4]) {
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    sa[q * PL] = make_float4(0.f, 0.f, 0.f, 0.f);
-    sb[q * PL] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  auto step = [&](int p, float(&b0)[4], float(&b1)[4], float(&b2)[4], int s0, int s1, int s2) {
-    const bool odd = p & 1;
-    float x0[4], x1[4], x2[4], y1[4], y2[4], y3[4];  // colour 0 + P xc of p, p-1, p-2; after colour 1, p-1..p-3
-    // plane p: colour 0 = b / diag + P xc (k_mg_prolong8: parent first on every axis)
-    unq(bn1, b0);
-    bn1 = bn2;
-    bn2 = ldb(p + 2);
-    {
-      int c9;
-      const float dxy = march_dxy(F, R, p, c9);
-      const int t0 = (p + R.j) & 1;
-      march_zero<BS>(F, R, dxy, c9, t0, b0, x0);
-      // cells (0, 1) and (2, 3): z taps parent (1, 1), (2, 2), child's side (0, 2), (1, 3);
-      // the parent plane (a = 0), then the plane on the child's side
-      const float wa[2] = {0.75f, 0.25f};
-      float2 v01 = make_float2(0.f, 0.f), v23 = v01;
-#pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        float cv[2][4];
-        march_zext(R, a == 0 ? cb : (odd ? cn : ca), cv);
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const float2 w = bc2(wa[a] * wa[e] * wa[t]);
-            v01 = __ffma2_rn(w, t == 0 ? pr(cv[e][1], cv[e][1]) : pr(cv[e][0], cv[e][2]), v01);
-            v23 = __ffma2_rn(w, t == 0 ? pr(cv[e][2], cv[e][2]) : pr(cv[e][1], cv[e][3]), v23);
-          }
-      }
-      const float2 s01 = __fadd2_rn(pr(x0[0], x0[1]), v01), s23 = __fadd2_rn(pr(x0[2], x0[3]), v23);
-      // outside the level: zeros, as the neighbours beyond a wall
-      const bool in = R.jin && p >= 0 && p < F.nx;
-      x0[0] = in && !t0 ? s01.x : 0.f;
-      x0[1] = in && t0 ? s01.y : 0.f;
-      x0[2] = in && !t0 ? s23.x : 0.f;
-      x0[3] = in && t0 ? s23.y : 0.f;
-      sa[s0 * PL] = mkq(x0);
-      if (odd) {  // the next plane has the next parent
-        ca = cb;
-        cb = cn;
-      } else {
-        cn = ldc((p >> 1) + 1);
-      }
+    for (int t = 0; t < 3; ++t) {
+      const int d = t == 0 ? nq : (t == 1 ? 0 : 2 * nq);
+      const float2 c = sc_[tid + d];
+      v[t][0] = cf[kl + 2 * d];
+      v[t][1] = c.x;
+      v[t][2] = c.y;
+      v[t][3] = cf[kr + 2 * d];
     }
-    __syncthreads();
-    unq(sa[s1 * PL], x1);
-    unq(sa[s2 * PL], x2);
-    unq(sb[s2 * PL], y2);
-    unq(sb[s0 * PL], y3);  // plane p - 3 (the slot that takes plane p in the next step)
+  };
+  // (is - 2 is even: the march starts on a first child.)  cv[0], cv[1]: the coarse planes m - 1
+  // and m of the parent plane m = p / 2, m + 1 replacing m - 1 on the second child
+  const int m0 = (is - 2) >> 1;
+  float cv[2][3][4];
+  ldc(m0 - 1);
+  putc();
+  __syncthreads();
+  getc(cv[0]);
+  ldc(m0);
+  __syncthreads();
+  putc();
+  __syncthreads();
+  getc(cv[1]);
+  ldc(m0 + 1);
+  __syncthreads();
+  float4 bn[2][2];  // b of the next two planes
+  float2 b0[3][2], b1[3][2], c0[3][2], c1[3][2];  // b and x of each colour
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    bn[0][r] = ldb(is - 2, r);
+    bn[1][r] = ldb(is - 1, r);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) b0[t][r] = b1[t][r] = c0[t][r] = c1[t][r] = pr(0.f, 0.f);
+  }
+  auto step = [&](int p, auto u) {
+    constexpr int U = decltype(u)::value, P = U % 3, Q = (U + 2) % 3, T = (U + 1) % 3, W = U & 1;
+    constexpr int M = 1 - (U / 2) % 2;  // cv[M]: the parent plane
+    if (W) {
+      getc(cv[1 - M]);
+    } else {
+      putc();  // plane m + 1, read on the second child
+      ldc((p >> 1) + 2);
+    }
+    const bool plane = p >= 0 && p < F.nx;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {  // plane p: colour 0 = b / diag + P xc (k_mg_prolong8: parent first on every axis)
+      const int par = W ^ r;
+      const float4 v = bn[W][r], d = R.diag(F, D, r, par, p);
+      bn[W][r] = ldb(p + 2, r);
+      b0[P][r] = par ? pr(v.y, v.w) : pr(v.x, v.z);
+      b1[P][r] = par ? pr(v.x, v.z) : pr(v.y, v.w);
+      if (BS) {  // Jacobi-scaled rows
+        b0[P][r] = mul2(b0[P][r], hi2(d));
+        b1[P][r] = mul2(b1[P][r], hi2(R.diag(F, D, r, 1 - par, p)));
+      }
+      const float wt[2] = {0.75f, 0.25f};
+      float2 t = pr(0.f, 0.f);
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float *c = cv[a ? 1 - M : M][e ? 1 + r : 0];
+          const float2 w0 = bc2(wt[a] * wt[e] * wt[0]), w1 = bc2(wt[a] * wt[e] * wt[1]);
+          t = a + e == 0 ? mul2(w0, pr(c[1], c[2])) : fma2s(w0, pr(c[1], c[2]), t);
+          t = fma2s(w1, par ? pr(c[2], c[3]) : pr(c[0], c[1]), t);
+        }
+      t = __fadd2_rn(mul2(b0[P][r], lo2(d)), t);
+      c0[P][r] = R.in && plane ? t : pr(0.f, 0.f);
+    }
     {  // plane p - 1: colour 1 of the post-smoothing
       const int i = p - 1;
-      float kl, kr;
-      march_kz(R, x1, kl, kr);
-      if (one && i >= 0 && i < F.nx) {
-        int c9;
-        const float dxy = march_dxy(F, R, i, c9);
-        const float4 *s = sa + s1 * PL;
-        march_pass<BS>(F, R, dxy, c9, (i + R.j + 1) & 1, b1, x1, x2, x0, s[-NQ], s[NQ], kl, kr, y1);
-      } else {
+      if (i >= 0 && i < F.nx) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) y1[c] = x1[c];
+        for (int r = 0; r < 2; ++r) {
+          const int odd = W ^ r;
+          const float2 a = __fadd2_rn(c0[T][r], c0[P][r]);
+          const float2 e = __fadd2_rn(r ? c0[Q][0] : s0[1 - W][1][R.im], r ? s0[1 - W][0][R.ip] : c0[Q][1]);
+          const float2 w = wsum2(F, a, e, march_z(odd, c0[Q][r], march_zn(R, odd, s0[1 - W][r])));
+          c1[Q][r] = mul2(__fadd2_rn(b1[Q][r], w), lo2(R.diag(F, D, r, odd, i)));
+        }
+      } else {
+        c1[Q][0] = c1[Q][1] = pr(0.f, 0.f);
       }
-      sb[s1 * PL] = mkq(y1);
     }
     {  // plane p - 2: colour 0, stored
       const int i = p - 2;
-      float kl, kr;
-      march_kz(R, y2, kl, kr);
-      if (zero && i >= is && i < ie) {
-        int c9;
-        const float dxy = march_dxy(F, R, i, c9);
-        const float4 *s = sb + s2 * PL;
-        float ov[4];
-        march_pass<BS>(F, R, dxy, c9, (i + R.j) & 1, b2, y2, y3, y1, s[-NQ], s[NQ], kl, kr, ov);
-        *reinterpret_cast<float4 *>(x + (o + i * sx)) = mkq(ov);
+      if (i >= is) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int odd = W ^ r;
+          const float2 a = __fadd2_rn(c1[P][r], c1[Q][r]);
+          const float2 e = __fadd2_rn(r ? c1[T][0] : s1[W][1][R.im], r ? s1[W][0][R.ip] : c1[T][1]);
+          const float2 w = wsum2(F, a, e, march_z(odd, c1[T][r], march_zn(R, odd, s1[W][r])));
+          const float2 v = mul2(__fadd2_rn(b0[T][r], w), lo2(R.diag(F, D, r, odd, i)));
+          const float2 ev = odd ? c1[T][r] : v, ov = odd ? v : c1[T][r];
+          if (R.band)
+            *reinterpret_cast<float4 *>(x + (o + r * F.nz + i * sx)) = make_float4(ev.x, ov.x, ev.y, ov.y);
+        }
       }
     }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      s0[W][r][tid] = c0[P][r];
+      s1[1 - W][r][tid] = c1[Q][r];
+    }
+    __syncthreads();
   };
-  for (int p = is - 2;;) {
-    step(p, bA, bC, bB, 0, 2, 1);
-    if (++p > ie + 1) break;
-    step(p, bB, bA, bC, 1, 0, 2);
-    if (++p > ie + 1) break;
-    step(p, bC, bB, bA, 2, 1, 0);
-    if (++p > ie + 1) break;
-  }
+  auto six = [&] {  // three parents: the two coarse planes change places
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float v = cv[0][t][c];
+        cv[0][t][c] = cv[1][t][c];
+        cv[1][t][c] = v;
+      }
+  };
+  CFDGB_MARCH_PLANES(step)
 }
+#undef CFDGB_MARCH_PLANES
 
 // coarsest level: x = 0, then `sweeps` red-black sweeps in shared memory, one block
 // x = M b on the coarsest level with the precomputed pseudo-inverse M (n x n, row-major):
@@ -1185,6 +1166,36 @@ static void level_geometry(MgLevelT<T> &L, int nsm, bool quads) {
   }
 }
 
+// The marching kernels' bands and segments: the fewest units of time over the waves of blocks,
+// each of msx planes, four halo planes and a start-up of about one, a plane costing a fixed part
+// (the barrier and the latencies of one thread's chain) and one per thread of the
+// multiprocessor: 0.74 us at 384 threads, 0.83 at 448 and 0.94 at 512 on 512x256x64.  Two blocks
+// of up to 256 threads share one (128 registers a thread).  512x256x64: 29 x 5 blocks of 448 threads, one wave.
+template <typename T>
+static void march_geometry(MgLevelT<T> &L, int nsm) {
+  const int nq = L.nz / 4, rows = L.ny / 2, most = kMgMarchThreads / nq - 2;
+  const int b0 = (rows + most - 1) / most;
+  double best = 0.0;
+  for (int bands = b0; bands <= std::min(rows, 4 * b0); ++bands) {
+    const int pairs = (rows + bands - 1) / bands, t = nq * (pairs + 2), per = t <= kMgMarchThreads / 2 ? 2 : 1;
+    const int mgy = (rows + pairs - 1) / pairs;
+    if (t < 64 && bands > b0) break;
+    for (int segs = 1; segs <= L.nx / 2; ++segs) {
+      const int msx = 2 * ((L.nx / 2 + segs - 1) / segs), mgx = (L.nx + msx - 1) / msx;
+      const long long blocks = (long long)mgx * mgy, sm = (long long)per * nsm, waves = (blocks + sm - 1) / sm;
+      const double on = (double)std::min<long long>(per, (blocks + nsm - 1) / nsm);  // blocks of a multiprocessor
+      const double cost = (double)waves * (msx + 5) * (250.0 + on * t);
+      if (best > 0.0 && cost >= best) continue;
+      best = cost;
+      L.mty = 2 * pairs;
+      L.mgy = mgy;
+      L.msx = msx;
+      L.mgx = mgx;
+    }
+  }
+  L.march = 1;
+}
+
 template <typename T>
 bool mg_plan(int nx, int ny, int nz, double hx, double hy, double hz, int nsm, bool quads, MgPlanT<T> *mg,
              bool pz) {
@@ -1219,17 +1230,9 @@ bool mg_plan(int nx, int ny, int nz, double hx, double hy, double hz, int nsm, b
     L.fx = fx;
     L.fy = fy;
     L.fz = fz;
-    // the marching kernels: a band of 256 / (nz / 4) rows (at most ny), the segments sized so
-    // that about two blocks per SM run
-    const int nq = nz / 4;
-    if (sizeof(T) == sizeof(float) && L.qgrid && fx == 2 && fy == 2 && fz == 2 && nq <= 16 && (nq & (nq - 1)) == 0 && cells < (1LL << 31)) {
-      L.march = 1;
-      L.mty = std::min(256 / nq, ny);
-      L.mgy = (ny + L.mty - 1) / L.mty;
-      const long long want = 2LL * nsm;
-      L.msx = 2 * (int)std::max(1LL, ((long long)nx * L.mgy + 2 * want - 1) / (2 * want));
-      L.mgx = (nx + L.msx - 1) / L.msx;
-    }
+    if (sizeof(T) == sizeof(float) && L.qgrid && fx == 2 && fy == 2 && fz == 2 && nz / 4 <= kMgMarchQuads &&
+        cells < (1LL << 31))
+      march_geometry(L, nsm);
     nx /= fx;
     ny /= fy;
     nz /= fz;
@@ -1365,32 +1368,16 @@ void launch_mg_vcycle(cudaStream_t s, const MgPlanT<T> &mg, int jacobi, const T 
   // pre-smoothing from zero and restriction to level l + 1.  (Both colour passes in one
   // kernel, each black cell recomputing its red neighbours' start values, was measured at
   // 80 us on the 512x256x64 level against 36 us for the two quad passes: not kept.)
-  // the marching kernels of a level (FP32 only; nz / 4 a power of two up to 16)
+  // the marching kernels of a level (FP32 only)
   auto march = [&](int l, bool up) {
     if constexpr (sizeof(T) == sizeof(float)) {
       const MgLevelT<T> &F = mg.lev[l], &Cl = mg.lev[l + 1];
-      const int bs = l == 0 ? jacobi : 0, nq = F.nz / 4;
-      const dim3 grid(F.mgx, F.mgy), block(nq * (F.mty + 4));
-      const size_t smem = 6 * sizeof(float4) * (size_t)block.x;
-#define CFDGB_MARCH(NQ)                                                                                      \
-  case NQ:                                                                                                 \
-    if (up && bs)                                                                                          \
-      launch_pdl(k_mg_up4<NQ, true>, grid, block, smem, s, F, Cl, B(l), (const T *)X(l + 1), X(l), sc);     \
-    else if (up)                                                                                           \
-      launch_pdl(k_mg_up4<NQ, false>, grid, block, smem, s, F, Cl, B(l), (const T *)X(l + 1), X(l), sc);    \
-    else if (bs)                                                                                           \
-      launch_pdl(k_mg_down4<NQ, true>, grid, block, smem, s, F, Cl, B(l), Cl.b, sc);                        \
-    else                                                                                                   \
-      launch_pdl(k_mg_down4<NQ, false>, grid, block, smem, s, F, Cl, B(l), Cl.b, sc);                       \
-    break;
-      switch (nq) {
-        CFDGB_MARCH(1)
-        CFDGB_MARCH(2)
-        CFDGB_MARCH(4)
-        CFDGB_MARCH(8)
-        CFDGB_MARCH(16)
-      }
-#undef CFDGB_MARCH
+      const bool bs = l == 0 && jacobi;
+      const dim3 grid(F.mgx, F.mgy), block(F.nz / 4 * (F.mty / 2 + 2));
+      if (up)
+        launch_pdl(bs ? k_mg_up<true> : k_mg_up<false>, grid, block, 0, s, F, Cl, B(l), (const T *)X(l + 1), X(l), sc);
+      else
+        launch_pdl(bs ? k_mg_down<true> : k_mg_down<false>, grid, block, 0, s, F, Cl, B(l), Cl.b, sc);
     }
   };
   auto down = [&](int l) {
