@@ -1195,6 +1195,14 @@ int upload_dense_coarse(cfdgb_ctx *c, MgPlanT<T> &mg) {
   TRY(dalloc(c, &d, M.size()));
   CK(cudaMemcpy(d, M.data(), M.size() * sizeof(T), cudaMemcpyHostToDevice));
   mg.cinv = d;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    const std::vector<int4> tab = mg_tail_table(mg);
+    if (tab.empty()) return 0;
+    int4 *t = nullptr;
+    TRY(dalloc(c, &t, tab.size()));
+    CK(cudaMemcpy(t, tab.data(), tab.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    mg.ttab = t;
+  }
   return 0;
 }
 
@@ -1493,6 +1501,7 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
       for (int l = 0; l < c->mg.nlev; ++l) c->mg.lev[l].march = 0;
     mg_prepare<float>();
     if ((rc = upload_dense_coarse(c, c->mg))) return bail(rc);
+    if (std::getenv("CFDGB_MG_PER_PASS")) c->mg.ttab = nullptr;  // (and the general tail)
     if ((rc = dalloc(c, &c->ph32, c->ncell)) || (rc = dalloc(c, &c->sh32, c->ncell))) return bail(rc);
     for (int l = 1; l < c->mg.nlev; ++l) {
       MgLevel &L = c->mg.lev[l];

@@ -194,9 +194,9 @@ struct MgLevelT {
   int qgrid;               // 1: the quad smoother (FP32, nz % 4 == 0) or the pair passes (FP64, nz even), 0: neither
   int qbx, qby, qgx, qgy, qgz;  // its launch: quads (FP64: pairs) along x, rows along y, planes strided over z
   int pz;                  // periodic z (every level; nz even or 1 on each)
-  // 1: the level's V-cycle work runs as two marching kernels (k_mg_down4, k_mg_up4; FP32
-  // quads, every axis halves, nz / 4 a power of two up to 16): a block of nz / 4 x (mty + 4)
-  // threads owns a band of mty rows and marches over a segment of msx planes; mgx x mgy blocks
+  // 1: the level's V-cycle work runs as two marching kernels (k_mg_down, k_mg_up; FP32 quads,
+  // every axis halves, nz / 4 up to 128): a block of nz / 4 x (mty / 2 + 2) threads owns a band of
+  // mty rows and marches over a segment of msx planes; mgx x mgy blocks
   int march, mty, msx, mgx, mgy;
   // division of a cell index by nz, ny and nz / 2 (the one-block kernels' cell loops): the
   // multiplier and shift of a division by an invariant integer (div_magic in multigrid.cu)
@@ -211,6 +211,7 @@ struct MgPlanT {
   int nlev;
   int coarse_sweeps;  // red-black sweeps of the coarsest solve
   int tail;           // levels tail..nlev-1 run in one block's shared memory (tail >= 1); nlev: none
+  const int4 *ttab;   // the one-block FP32 tail's table of cell pairs (device; mg_tail_table), or null: k_mg_tail
   const T *cinv;      // the coarsest level's dense pseudo-inverse (device), or null: red-black sweeps
   MgLevelT<T> lev[kMgMaxLevels];
 };
@@ -226,10 +227,13 @@ bool mg_plan(int nx, int ny, int nz, double hx, double hy, double hz, int nsm, b
 // kernels one V-cycle launches
 template <typename T>
 int mg_vcycle_launches(const MgPlanT<T> &mg, int jacobi);
-// the pseudo-inverse of the coarsest level's operator, row-major, when that level has at
+// the pseudo-inverse of the coarsest level's operator, by columns, when that level has at
 // most kMgDenseCells cells (the caller uploads it and sets mg.cinv)
 template <typename T>
 bool mg_dense_inverse(const MgPlanT<T> &mg, std::vector<T> &M);
+// the FP32 tail's table of cell pairs (the caller uploads it and sets mg.ttab, with mg.cinv), empty
+// where its kernel cannot run the hierarchy
+std::vector<int4> mg_tail_table(const MgPlan &mg);
 // kernel attributes the hierarchy needs (shared memory of the one-block kernels); once,
 // before the first V-cycle
 template <typename T>

@@ -16,6 +16,7 @@
 // has stopped.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -925,15 +926,27 @@ __global__ void __launch_bounds__(kMgMarchThreads)
 #undef CFDGB_MARCH_PLANES
 
 // coarsest level: x = 0, then `sweeps` red-black sweeps in shared memory, one block
-// x = M b on the coarsest level with the precomputed pseudo-inverse M (n x n, row-major):
-// one dot product of length n per cell (the block's shared copies of b, x)
+// x = M b on the coarsest level with the precomputed pseudo-inverse M (n x n, by columns, so that
+// the threads of neighbouring cells read neighbouring elements): one dot product of length n per
+// cell, its elements fetched sixteen at a time (the block's shared copies of b, x)
+template <typename T>
+__device__ __forceinline__ T dense_row(int n, const T *M, const T *bs, int q) {
+  T v = T(0);
+  int c = 0;
+  for (; c + 16 <= n; c += 16) {
+    T m[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) m[e] = M[(c + e) * n + q];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v = fma_rn(m[e], bs[c + e], v);
+  }
+  for (; c < n; ++c) v = fma_rn(M[c * n + q], bs[c], v);
+  return v;
+}
 template <typename T>
 __device__ void blk_dense(int n, const T *__restrict__ M, const T *bs, T *xs) {
   for (int q = threadIdx.x; q < n; q += blockDim.x) {
-    const T *row = M + (long long)q * n;
-    T v = T(0);
-    for (int c = 0; c < n; ++c) v += row[c] * bs[c];
-    xs[q] = v;
+    xs[q] = dense_row(n, M, bs, q);
   }
   __syncthreads();
 }
@@ -1143,6 +1156,316 @@ __global__ void __launch_bounds__(1024) k_mg_tail(MgPlanT<T> mg, int t, const So
   for (int q = threadIdx.x; q < nt; q += blockDim.x) mg.lev[t].x[q] = xs[t][q];
 }
 
+// The same tail for FP32 with a dense coarsest solve, built for latency: a phase of a small level
+// has a few operations a cell, so index arithmetic, serial loads and instruction fetches were
+// most of its time (512x256x64: a V-cycle 74 -> 62 us; 256x128x32: 43 -> 32; 120x40x12, with a
+// coarsest level of 225 cells: 37 -> 25).
+//   - A thread owns a pair of neighbours along an axis with an even extent (one cell of each
+//     colour; every level but the coarsest halves one).  The pairs' addresses come from a table
+//     made with the plan (mg_tail_table), copied to shared memory, as the coarsest level's
+//     inverse is, before the kernel waits for the one before it.
+//   - x is stored with a layer of ghost cells: zeros beyond walls, copies across a periodic z, so
+//     a neighbour sum is six unconditional loads.
+//   - The residuals go to a scratch copy of the level, one thread a pair, and the next level's
+//     threads add up their cells' children (k_mg_tail: eight residuals, one after the other, a
+//     thread).
+//   - The prolongation forms colour 0 only: the pass that follows overwrites colour 1.
+// Every value is formed by k_mg_tail's rounded sequence (lnb's sum as the compiler contracts it).
+constexpr int kTailSlots = 3;             // pairs a thread
+constexpr int kTailShared = 224 * 1024;  // bytes
+constexpr int kTailDiag = 28;             // entries of a level's table of diagonals (27, padded)
+static_assert(kTailSlots * 1024 * 2 >= tail_cells_max<float>(), "a thread's pairs");
+
+__host__ __device__ __forceinline__ int tail_padded(const MgLevel &L) { return (L.nx + 2) * (L.ny + 2) * (L.nz + 2); }
+__host__ __device__ __forceinline__ int tail_cells(const MgLevel &L) { return L.nx * L.ny * L.nz; }
+
+// shared memory in words: [pairs and coarsest cells][1/diag and diag][x, padded][b][the coarsest level's
+// b][scratch][inverse, the columns that fit]; the first two as in the table in global memory
+struct TailLayout {
+  int tab, x, b, d, s, m, cols, words;
+};
+static TailLayout tail_layout(const MgPlan &mg) {
+  TailLayout o;
+  int pairs = 0, px = 0;
+  for (int l = mg.tail; l < mg.nlev; ++l) {
+    px += tail_padded(mg.lev[l]);
+    if (l < mg.nlev - 1) pairs += tail_cells(mg.lev[l]) / 2;
+  }
+  const int nc = tail_cells(mg.lev[mg.nlev - 1]), all = kTailShared / 4;
+  o.tab = 4 * (pairs + nc);
+  o.x = o.tab + 2 * kTailDiag * (mg.nlev - 1 - mg.tail);
+  o.b = o.x + ((px + 1) & ~1);
+  o.d = (o.b + 2 * pairs + 3) & ~3;
+  o.s = o.d + kMgDenseCells;
+  o.m = (o.s + tail_padded(mg.lev[mg.tail]) + 3) & ~3;
+  o.cols = o.m >= all ? 0 : (all - o.m) / nc;
+  if (o.cols >= nc) o.cols = nc;
+  o.words = o.m + o.cols * nc;
+  return o;
+}
+
+__device__ __forceinline__ void tail_put(const MgLevel &L, float *X, int a, int wrap, float v) {
+  X[a] = v;
+  if (wrap) X[a + (wrap == 1 ? L.nz : -L.nz)] = v;
+}
+__device__ __forceinline__ float tail_nb(const MgLevel &L, const float *X, int a) {
+  const int PZ = L.nz + 2, PX = (L.ny + 2) * PZ;
+  const float x = add_rn(X[a - PX], X[a + PX]), y = add_rn(X[a - PZ], X[a + PZ]), z = add_rn(X[a - 1], X[a + 1]);
+  return fma_rn(L.wz, z, fma_rn(L.wx, x, mul_rn(L.wy, y)));
+}
+// the average of the residuals of a cell's children (k_mg_restrict's order), the first at s
+__device__ __forceinline__ float tail_children(const MgLevel &F, const float *s) {
+  const int PZ = F.nz + 2, PX = (F.ny + 2) * PZ;
+  float v = 0.f;
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (a < F.fx && e < F.fy && c < F.fz) v = add_rn(v, s[a * PX + e * PZ + c]);
+  return mul_rn(v, (F.fx == 2 ? 0.5f : 1.f) * (F.fy == 2 ? 0.5f : 1.f) * (F.fz == 2 ? 0.5f : 1.f));
+}
+
+// A pair's entry (int4): x: padded addresses of the cells of colour 0 and 1 (16 bits each); y: their
+// rows of the diagonal table (5 bits each), where a copy across the periodic wrap goes (2 bits
+// each: 1 after, 2 before), and colour 0's side taps along x, y, z (2 bits each: 1 after, 2
+// before, 0 the parent itself); z: both cells' rows of the level (the first level) or their first
+// children's addresses; w: the address of colour 0's parent.  The coarsest level's cells: x: padded
+// address, y: the copy across the wrap, z: the first child's address.
+__device__ __forceinline__ int lo16(int v) { return v & 0xffff; }
+__device__ __forceinline__ int hi16(int v) { return (int)((unsigned)v >> 16); }
+
+__global__ void __launch_bounds__(1024) k_mg_tail32(MgPlan mg, TailLayout o, const SolverScal *sc) {
+  extern __shared__ __align__(16) float tsm[];
+  const int tid = threadIdx.x, n = mg.nlev, t = mg.tail;
+  const MgLevel &C = mg.lev[n - 1];
+  const int nc = tail_cells(C);
+  const int4 *P = reinterpret_cast<const int4 *>(tsm);
+  const float2 *tb = reinterpret_cast<const float2 *>(tsm + o.tab);
+  float *X = tsm + o.x, *B = tsm + o.b;
+  float *const S = tsm + o.s, *const D = tsm + o.d;
+  {  // constants of the context: no need to wait for the kernel before
+    const unsigned d = (unsigned)__cvta_generic_to_shared(tsm);
+    for (int q = tid; q < o.x / 4; q += 1024)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d + 16 * q), "l"(mg.ttab + q) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const int nm = o.cols * nc, n4 = nm & ~3;
+    for (int q = 4 * tid; q < n4; q += 4096)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d + 4 * (o.m + q)), "l"(mg.cinv + q) : "memory");
+    if (tid < nm - n4) tsm[o.m + n4 + tid] = mg.cinv[n4 + tid];
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int q = o.x + tid; q < o.b; q += 1024) tsm[q] = 0.f;
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+  }
+  pdl_wait();
+  if (sc->done) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
+  pdl_trigger();
+  for (int l = t; l < n - 1; ++l) {
+    const MgLevel &L = mg.lev[l];
+    const int np = tail_cells(L) / 2;
+    int4 s[kTailSlots];
+    float b[kTailSlots][2], x0[kTailSlots], r1[kTailSlots];
+#pragma unroll
+    for (int u = 0; u < kTailSlots; ++u) {
+      const int p = tid + 1024 * u;
+      if (p >= np) break;
+      s[u] = P[p];
+      if (l == t) {
+        b[u][0] = L.b[lo16(s[u].z)];
+        b[u][1] = L.b[hi16(s[u].z)];
+      } else {
+        b[u][0] = tail_children(mg.lev[l - 1], S + lo16(s[u].z));
+        b[u][1] = tail_children(mg.lev[l - 1], S + hi16(s[u].z));
+      }
+      *reinterpret_cast<float2 *>(B + 2 * p) = make_float2(b[u][0], b[u][1]);
+      x0[u] = mul_rn(b[u][0], tb[s[u].y & 31].x);
+      tail_put(L, X, lo16(s[u].x), (s[u].y >> 10) & 3, x0[u]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kTailSlots; ++u) {
+      if (tid + 1024 * u >= np) break;
+      const float2 d = tb[(s[u].y >> 5) & 31];
+      const float w = tail_nb(L, X, hi16(s[u].x)), x1 = mul_rn(add_rn(b[u][1], w), d.x);
+      r1[u] = resid(b[u][1], d.y, x1, w);
+      tail_put(L, X, hi16(s[u].x), (s[u].y >> 12) & 3, x1);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kTailSlots; ++u) {
+      if (tid + 1024 * u >= np) break;
+      const int a = lo16(s[u].x);
+      S[a] = resid(b[u][0], tb[s[u].y & 31].y, x0[u], tail_nb(L, X, a));
+      S[hi16(s[u].x)] = r1[u];
+    }
+    __syncthreads();
+    X += tail_padded(L);
+    B += 2 * np;
+    P += np;
+    tb += kTailDiag;
+  }
+  {  // coarsest: the dense pseudo-inverse
+    const int4 s = tid < nc ? P[tid] : make_int4(0, 0, 0, 0);
+    if (tid < nc) D[tid] = tail_children(mg.lev[n - 2], S + s.z);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (tid < nc) {
+      // dense_row's sum; the first columns that did not fit are on their way meanwhile
+      float v = 0.f, g[16];
+      if (o.cols < nc) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) g[e] = o.cols + e < nc ? mg.cinv[(o.cols + e) * nc + tid] : 0.f;
+      }
+      const float *M = tsm + o.m + tid;
+      int c = 0;
+      for (; c + 16 <= o.cols; c += 16, M += 16 * nc) {
+        float m[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) m[e] = M[e * nc];
+#pragma unroll
+        for (int e = 0; e < 16; e += 4) {
+          const float4 b = *reinterpret_cast<const float4 *>(D + c + e);
+          v = fma_rn(m[e + 3], b.w, fma_rn(m[e + 2], b.z, fma_rn(m[e + 1], b.y, fma_rn(m[e], b.x, v))));
+        }
+      }
+      for (; c < o.cols; ++c, M += nc) v = fma_rn(*M, D[c], v);
+      if (o.cols < nc) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+          if (o.cols + e < nc) v = fma_rn(g[e], D[o.cols + e], v);
+        for (c = o.cols + 16; c < nc; ++c) v = fma_rn(mg.cinv[c * nc + tid], D[c], v);
+      }
+      tail_put(C, X, s.x, s.y, v);
+    }
+    __syncthreads();
+  }
+  for (int l = n - 2; l >= t; --l) {
+    const MgLevel &L = mg.lev[l], &Cl = mg.lev[l + 1];
+    const float *const Xc = X;
+    const int np = tail_cells(L) / 2, QZ = Cl.nz + 2, QX = (Cl.ny + 2) * QZ;
+    X -= tail_padded(L);
+    B -= 2 * np;
+    P -= np;
+    tb -= kTailDiag;
+    const float wi[2] = {L.fx == 2 ? 0.75f : 1.f, L.fx == 2 ? 0.25f : 0.f};
+    const float wj[2] = {L.fy == 2 ? 0.75f : 1.f, L.fy == 2 ? 0.25f : 0.f};
+    const float wk[2] = {L.fz == 2 ? 0.75f : 1.f, L.fz == 2 ? 0.25f : 0.f};
+    int4 s[kTailSlots];
+    float b[kTailSlots][2], x1[kTailSlots];
+#pragma unroll
+    for (int u = 0; u < kTailSlots; ++u) {  // colour 0 += P xc (prolong_at's taps in their order)
+      const int p = tid + 1024 * u;
+      if (p >= np) break;
+      s[u] = P[p];
+      const float2 v = *reinterpret_cast<const float2 *>(B + 2 * p);
+      b[u][0] = v.x;
+      b[u][1] = v.y;
+      auto side = [&](int sh, int d) {
+        const int c = (s[u].y >> sh) & 3;
+        return c == 0 ? 0 : (c == 1 ? d : -d);
+      };
+      const int ox = side(14, QX), oy = side(16, QZ), oz = side(18, 1);
+      float w = 0.f;
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int c = 0; c < 2; ++c)  // (a weight of zero adds zero times the parent)
+            w = fma_rn(wi[a] * wj[e] * wk[c], Xc[s[u].w + (a ? ox : 0) + (e ? oy : 0) + (c ? oz : 0)], w);
+      const int a0 = lo16(s[u].x);
+      tail_put(L, X, a0, (s[u].y >> 10) & 3, add_rn(X[a0], w));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kTailSlots; ++u) {
+      if (tid + 1024 * u >= np) break;
+      x1[u] = mul_rn(add_rn(b[u][1], tail_nb(L, X, hi16(s[u].x))), tb[(s[u].y >> 5) & 31].x);
+      tail_put(L, X, hi16(s[u].x), (s[u].y >> 12) & 3, x1[u]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kTailSlots; ++u) {
+      if (tid + 1024 * u >= np) break;
+      const int a = lo16(s[u].x);
+      const float v = mul_rn(add_rn(b[u][0], tail_nb(L, X, a)), tb[s[u].y & 31].x);
+      if (l > t) {
+        tail_put(L, X, a, (s[u].y >> 10) & 3, v);
+      } else {
+        L.x[lo16(s[u].z)] = v;
+        L.x[hi16(s[u].z)] = x1[u];
+      }
+    }
+    if (l > t) __syncthreads();
+  }
+}
+
+// The pairs' entries of k_mg_tail32 for levels tail..nlev-2, the coarsest level's cells and the
+// diagonals; empty:
+// it cannot run this hierarchy (no tail of two levels, a coarsest level without a dense inverse,
+// padded levels beyond the block's shared memory)
+std::vector<int4> mg_tail_table(const MgPlan &mg) {
+  std::vector<int4> tab;
+  const int n = mg.nlev, nc = tail_cells(mg.lev[n - 1]);
+  if (mg.tail >= n - 1 || nc > kMgDenseCells || 4ll * tail_layout(mg).m > kTailShared) return tab;
+  auto addr = [](const MgLevel &L, int i, int j, int k) { return ((i + 1) * (L.ny + 2) + j + 1) * (L.nz + 2) + k + 1; };
+  auto wrap = [](const MgLevel &L, int k) { return L.pz && L.nz > 1 ? (k == 0 ? 1 : (k == L.nz - 1 ? 2 : 0)) : 0; };
+  auto side = [](int i, int f, int m, bool per) {
+    const int d = (i & 1) ? 1 : -1, q = (i >> 1) + d;
+    return f == 1 || ((q < 0 || q >= m) && !(per && m > 1)) ? 0 : (d > 0 ? 1 : 2);  // periodic: the ghost holds it
+  };
+  auto ends = [](int i, int m) { return (i > 0) + (i < m - 1); };
+  for (int l = mg.tail; l < n; ++l) {
+    const MgLevel &L = mg.lev[l], &F = mg.lev[l - 1];
+    auto below = [&](int i, int j, int k) {  // the row of the level, or the first child's address
+      return l == mg.tail ? (i * L.ny + j) * L.nz + k : addr(F, F.fx * i, F.fy * j, F.fz * k);
+    };
+    const bool coarsest = l == n - 1;
+    const int di = !coarsest && L.nz % 2 && L.ny % 2, dk = !coarsest && L.nz % 2 == 0, dj = !coarsest && !di && !dk;
+    for (int i = 0; i < L.nx; i += 1 + di)
+      for (int j = 0; j < L.ny; j += 1 + dj)
+        for (int k = 0; k < L.nz; k += 1 + dk) {
+          if (coarsest) {
+            tab.push_back(make_int4(addr(L, i, j, k), wrap(L, k), below(i, j, k), 0));
+            continue;
+          }
+          int q[2][3] = {{i, j, k}, {i + di, j + dj, k + dk}};  // by colour
+          if ((i + j + k) & 1) std::swap(q[0], q[1]);
+          int4 e = make_int4(0, 0, 0, 0);
+          for (int c = 0; c < 2; ++c) {
+            const int *v = q[c];
+            const int z = L.pz ? (L.nz > 1 ? 2 : 0) : ends(v[2], L.nz);
+            e.x |= (int)((unsigned)addr(L, v[0], v[1], v[2]) << (16 * c));
+            e.y |= (9 * ends(v[0], L.nx) + 3 * ends(v[1], L.ny) + z) << (5 * c) | wrap(L, v[2]) << (10 + 2 * c);
+            e.z |= (int)((unsigned)below(v[0], v[1], v[2]) << (16 * c));
+          }
+          const MgLevel &Cl = mg.lev[l + 1];
+          const int *v = q[0];
+          e.y |= side(v[0], L.fx, Cl.nx, false) << 14 | side(v[1], L.fy, Cl.ny, false) << 16 |
+                 side(v[2], L.fz, Cl.nz, L.pz != 0) << 18;
+          e.w = addr(Cl, v[0] / L.fx, v[1] / L.fy, v[2] / L.fz);
+          tab.push_back(e);
+        }
+  }
+  for (int l = mg.tail; l < n - 1; ++l) {  // 1/diag and diag by row class
+    const MgLevel &L = mg.lev[l];
+    float2 d[kTailDiag] = {};
+    for (int c = 0; c < 27; ++c) {
+      const float dxy = L.wx * (float)(c / 9) + L.wy * (float)(c / 3 % 3);  // the products are exact
+      d[c] = make_float2(L.idg[c], dxy + L.wz * (float)(c % 3));
+    }
+    const size_t at = tab.size();
+    tab.resize(at + kTailDiag / 2);
+    std::memcpy(&tab[at], d, sizeof d);
+  }
+  return tab;
+}
+
 template <typename T>
 static void level_geometry(MgLevelT<T> &L, int nsm, bool quads) {
   L.bx = 1;
@@ -1176,7 +1499,7 @@ static void march_geometry(MgLevelT<T> &L, int nsm) {
   const int nq = L.nz / 4, rows = L.ny / 2, most = kMgMarchThreads / nq - 2;
   const int b0 = (rows + most - 1) / most;
   double best = 0.0;
-  for (int bands = b0; bands <= std::min(rows, 4 * b0); ++bands) {
+  for (int bands = b0; bands <= std::min(rows, b0 + 8); ++bands) {
     const int pairs = (rows + bands - 1) / bands, t = nq * (pairs + 2), per = t <= kMgMarchThreads / 2 ? 2 : 1;
     const int mgy = (rows + pairs - 1) / pairs;
     if (t < 64 && bands > b0) break;
@@ -1327,7 +1650,8 @@ bool mg_dense_inverse(const MgPlanT<T> &mg, std::vector<T> &M) {
     }
   }
   M.resize((size_t)n * n);
-  for (size_t q = 0; q < M.size(); ++q) M[q] = (T)(I[q] - 1.0 / n);
+  for (int r = 0; r < n; ++r)
+    for (int c = 0; c < n; ++c) M[(size_t)c * n + r] = (T)(I[(size_t)r * n + c] - 1.0 / n);
   return true;
 }
 
@@ -1337,6 +1661,8 @@ void mg_prepare() {
   cudaFuncSetAttribute(k_mg_coarse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)(2 * sizeof(T) * kMgSharedCells));
   cudaFuncSetAttribute(k_mg_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMgTailBytes);
+  if (sizeof(T) == sizeof(float))
+    cudaFuncSetAttribute(k_mg_tail32, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailShared);
 }
 
 template <typename T>
@@ -1414,9 +1740,16 @@ void launch_mg_vcycle(cudaStream_t s, const MgPlanT<T> &mg, int jacobi, const T 
   for (int l = 0; l + 1 < m; ++l) down(l);
   if (m < n) {
     down(m - 1);  // levels m-1 -> m as above, then the tail
-    size_t cells = 0;
+    size_t cells = 0, bytes = 0;
     for (int l = m; l < n; ++l) cells += (size_t)mg.lev[l].nx * mg.lev[l].ny * mg.lev[l].nz;
-    launch_pdl(k_mg_tail<T>, dim3(1), dim3(1024), 2 * sizeof(T) * cells, s, mg, m, sc);
+    if constexpr (sizeof(T) == sizeof(float)) {
+      if (mg.ttab) {
+        const TailLayout o = tail_layout(mg);
+        bytes = 4 * (size_t)o.words;
+        launch_pdl(k_mg_tail32, dim3(1), dim3(1024), bytes, s, mg, o, sc);
+      }
+    }
+    if (bytes == 0) launch_pdl(k_mg_tail<T>, dim3(1), dim3(1024), 2 * sizeof(T) * cells, s, mg, m, sc);
   } else {
     const MgLevelT<T> &C = mg.lev[n - 1];
     const size_t smem = 2 * sizeof(T) * (size_t)C.nx * C.ny * C.nz;
