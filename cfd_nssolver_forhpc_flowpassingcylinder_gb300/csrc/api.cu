@@ -61,7 +61,7 @@ enum KId {
   K_RESID64, K_SETUP32, K_CORRECT64, K_TRANSFORM, K_UPDATE, K_BC, K_RBSOR, K_RNORM, K_NANRESET, K_ETA,
   K_CGQ64, K_CGXR64, K_CGP64, K_CGPQ32, K_CGXR32, K_CFL, K_LES,
   K_PP32, K_MG, K_PV32, K_PS32, K_PT32, K_PXR32, K_MIRROR,
-  K_PP64, K_MG64, K_PV64, K_PS64, K_PT64, K_PXR64, K_LOOP64, K_CGLOOP64, K_COUNT
+  K_PP64, K_MG64, K_PV64, K_PS64, K_PT64, K_PXR64, K_LOOP64, K_CGLOOP64, K_CGLOOP32, K_COUNT
 };
 const char *const kKernelNames[K_COUNT] = {
     "convection_diffusion", "rhs", "bicg_setup64", "bicg_ap64", "bicg_s64", "bicg_as64", "bicg_xr64",
@@ -70,7 +70,7 @@ const char *const kKernelNames[K_COUNT] = {
     "cg_q64", "cg_xr64", "cg_p64", "cg_pq32", "cg_xr32", "cfl", "smagorinsky",
     "bicgp_p32", "mg_vcycle", "bicgp_v32", "bicgp_s32", "bicgp_t32", "bicgp_xr32", "mirror32",
     "bicgp_p64", "mg_vcycle64", "bicgp_v64", "bicgp_s64", "bicgp_t64", "bicgp_xr64",
-    "bicg_loop64", "cg_loop64"};
+    "bicg_loop64", "cg_loop64", "cg_loop32"};
 
 // Scalars of one time step run as a graph, appended on the device (k_step_record)
 struct StepRec {
@@ -134,6 +134,7 @@ struct cfdgb_ctx {
   // chunk graphs of solver iterations
   cudaGraphExec_t chunk64 = nullptr, chunk32 = nullptr;
   int chunk_len = 16;
+  bool loop32 = false;  // FP32 CG sweeps in one launch a chunk (cg32_loop_fits)
   int loop_blocks = 0;  // blocks of the one-launch FP64 iterations (loop64_blocks); 0: a kernel a phase
   double omega = 0.0;  // SOR relaxation in use (cfg.omega, or the optimal one when that is 0)
   // test switch (environment CFDGB_TEST_WAIT_FAULT at create): the next MIXED solve makes one
@@ -493,8 +494,10 @@ const int kPrecKid64[kPrecParts] = {K_PP64, K_MG64, K_PV64, K_PS64, K_MG64, K_PT
 // the iteration of this precision is the multigrid-preconditioned one
 bool prec_iter(const cfdgb_ctx *c, bool fp32) { return fp32 ? c->use_mg : c->use_mg64; }
 
-// the FP64 Krylov iteration runs whole chunks in one cooperative launch
-bool loop_iter(const cfdgb_ctx *c, bool fp32) { return !fp32 && !c->use_mg64 && c->loop_blocks > 0; }
+// the Krylov iteration runs whole chunks in one cooperative launch
+bool loop_iter(const cfdgb_ctx *c, bool fp32) {
+  return fp32 ? c->loop32 : !c->use_mg64 && c->loop_blocks > 0;
+}
 
 // launch_iter_kernel's parts in one iteration (a whole chunk for the one-launch form)
 int iter_kernels(const cfdgb_ctx *c, bool fp32) {
@@ -504,7 +507,7 @@ int iter_kernels(const cfdgb_ctx *c, bool fp32) {
   return fp32 ? 3 : 5;
 }
 int iter_kid(const cfdgb_ctx *c, bool fp32, int part) {
-  if (loop_iter(c, fp32)) return c->cfg.solver == CFDGB_CG ? K_CGLOOP64 : K_LOOP64;
+  if (loop_iter(c, fp32)) return fp32 ? K_CGLOOP32 : c->cfg.solver == CFDGB_CG ? K_CGLOOP64 : K_LOOP64;
   if (prec_iter(c, fp32)) return (fp32 ? kPrecKid : kPrecKid64)[part];
   if (c->cfg.solver == CFDGB_CG) return (fp32 ? K_CGPQ32 : K_CGQ64) + part;
   return (fp32 ? K_PAP32 : K_AP64) + part;
@@ -518,14 +521,16 @@ int iter_part_launches(const cfdgb_ctx *c, bool fp32, int part) {
 // iterations per chunk, and how often a captured chunk repeats the parts: the preconditioned
 // iteration is long and needs few; the one-launch form is the chunk
 int chunk_iters(const cfdgb_ctx *c, bool fp32) {
-  if (loop_iter(c, fp32)) return loop64_iters(c->ncell);
+  if (loop_iter(c, fp32)) return fp32 ? kCg32LoopIters : loop64_iters(c->ncell);
   return prec_iter(c, fp32) ? 2 : c->chunk_len;
 }
 int chunk_repeats(const cfdgb_ctx *c, bool fp32) { return loop_iter(c, fp32) ? 1 : chunk_iters(c, fp32); }
 void launch_iter_kernel(cfdgb_ctx *c, bool fp32, int part) {
   const bool jac = c->cfg.solver == CFDGB_BICGSTAB_JACOBI;
   if (loop_iter(c, fp32)) {
-    if (c->cfg.solver == CFDGB_CG)
+    if (fp32)
+      launch_cg32_loop(c->stream, c->g, c->spe32, c->k32, c->p32, c->ap32, c->part, c->sc32, c->nsm);
+    else if (c->cfg.solver == CFDGB_CG)
       launch_cg64_loop(c->stream, c->g, c->spe64, c->k64, c->part, c->sc, c->loop_blocks, chunk_iters(c, false));
     else
       launch_bicg64_loop(c->stream, c->g, jac ? c->jac64 : c->spe64, c->k64, c->part, c->sc, c->loop_blocks,
@@ -637,8 +642,8 @@ int run_chunks(cfdgb_ctx *c, bool fp32, SolverScal *out) {
       std::fprintf(stderr, "[cfdgb]     %s it %d relres %.4e\n", fp32 ? "fp32" : "fp64", c->h_sc->iter,
                    c->h_sc->relres);
     if (c->h_sc->fault)
-      return fail(CFDGB_ECUDA, fp32 ? "FP32 stencil pipeline: a bounded wait gave up (block stopped early)"
-                                    : "FP64 iteration: a bounded wait between blocks gave up");
+      return fail(CFDGB_ECUDA, loop_iter(c, fp32) ? "Krylov iteration: a bounded wait between blocks gave up"
+                                                  : "FP32 stencil pipeline: a bounded wait gave up (block stopped early)");
     if (c->h_sc->done) {
       *out = *c->h_sc;
       return 0;
@@ -1511,6 +1516,8 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
     c->use_mg = true;
   }
   if (cfg->solver != CFDGB_RBSOR && !std::getenv("CFDGB_NO_LOOP")) c->loop_blocks = loop64_blocks(c->ncell);
+  if (cfg->solver == CFDGB_CG && cfg->precision == CFDGB_MIXED && !c->use_mg && !std::getenv("CFDGB_NO_LOOP"))
+    c->loop32 = cg32_loop_fits(g, c->spe32, c->nsm);
   if ((rc = dalloc(c, &c->part, std::max(8 * (size_t)std::max(c->nblk, nblk3), loop64_part_doubles())))) return bail(rc);
   if ((rc = dalloc(c, &c->sc, 1)) || (rc = dalloc(c, &c->sc32, 1)) || (rc = dalloc(c, &c->ss, 1))) return bail(rc);
   cudaMemset(c->sc, 0, sizeof(SolverScal));

@@ -104,6 +104,13 @@ void launch_bicg64_part(cudaStream_t s, int part, const Geo &g, const Stencil<do
 // 262.8 / 246.4 (the block a multiprocessor leaves HBM waiting): the line lies between.
 constexpr long long kLoopCells = 3LL << 20;
 int loop64_blocks(long long ncell);
+// FP32 CG sweeps in one cooperative launch a chunk of kCg32LoopIters iterations, where the grid's
+// state fits the multiprocessors (cg32_loop_fits: uniform grids, up to 2.4 M cells on 152 of them);
+// the launch ends early when the sweep does
+constexpr int kCg32LoopIters = 256;
+bool cg32_loop_fits(const Geo &g, const Stencil<float> &st, int nsm);
+void launch_cg32_loop(cudaStream_t s, const Geo &g, const Stencil<float> &st, KrylovVecs<float> v, float *const p2[2],
+                      float *const ap2[2], double *part_buf, SolverScal *sc, int nsm);
 int loop64_iters(long long ncell);
 size_t loop64_part_doubles();
 void launch_bicg64_loop(cudaStream_t s, const Geo &g, const Stencil<double> &st, KrylovVecs<double> v,

@@ -1595,7 +1595,7 @@ constexpr long long kLoopWaitCycles = 1LL << 32;  // ~2 s
 constexpr int kLoopSlots = 5;        // values reduced in an iteration
 
 struct LoopScal {
-  double rho, alpha, omega, beta, relres;
+  double rho, alpha, omega, beta, relres, best, rmax;
   int iter, done, status, restart, bad;
 };
 
@@ -1604,55 +1604,71 @@ struct LoopGrid {
   double *part;     // [slot][kLoopMaxBlocks]
   unsigned target;  // arrivals that complete the next barrier
   long long limit;  // cycles a wait may take
+  // one thread: this block's arrival, and the wait for all (the block's stores come before, by the
+  // barrier that its threads passed)
+  __device__ __forceinline__ void arrive_wait(LoopScal &L) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sc->cnt[6]) : "memory");
+    const long long t0 = clock64();
+    for (;;) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&sc->cnt[6]) : "memory");
+      if ((int)(v - target) >= 0) break;
+      if (clock64() - t0 > limit) {
+        L.bad = 1;
+        break;
+      }
+    }
+  }
   __device__ __forceinline__ bool sync(LoopScal &L) {
     __syncthreads();
     target += gridDim.x;
-    if (threadIdx.x == 0) {
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sc->cnt[6]) : "memory");
-      const long long t0 = clock64();
-      for (;;) {
-        unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&sc->cnt[6]) : "memory");
-        if ((int)(v - target) >= 0) break;
-        if (clock64() - t0 > limit) {
-          L.bad = 1;
-          break;
-        }
-      }
-    }
+    if (threadIdx.x == 0) arrive_wait(L);
     __syncthreads();
     return L.bad == 0;
   }
   // sums of v over the grid (slots s..), with a barrier; warp 0 calls fin(sums) in all its lanes,
-  // which leaves the scalars in L
+  // which leaves the scalars in L.  Warp 0 alone adds up its block, arrives, waits and adds up the
+  // blocks, each of its lanes a few of them: two block barriers in all
   template <int NV, class Fin>
   __device__ __forceinline__ bool reduce(LoopScal &L, double (&v)[NV], int s, Fin &&fin) {
-    __shared__ double sh[NV][kLoopMaxBlocks / 32];
-    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nw = (int)(gridDim.x + 31) >> 5;
-    block_sum<NV>(v);
-    if (t == 0)
+    __shared__ double sh[NV][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
+    warp_sum<NV>(v);
+    if (lane == 0)
 #pragma unroll
-      for (int q = 0; q < NV; ++q) part[(s + q) * kLoopMaxBlocks + blockIdx.x] = v[q];
-    if (!sync(L)) return false;
-    if (wid < nw) {
-      double o[NV];
-#pragma unroll
-      for (int q = 0; q < NV; ++q) o[q] = t < (int)gridDim.x ? __ldcg(part + (s + q) * kLoopMaxBlocks + t) : 0.0;
-#pragma unroll
-      for (int q = 0; q < NV; ++q) {
-        const double x = warp_sum1(o[q]);
-        if (lane == 0) sh[q][wid] = x;
-      }
-    }
+      for (int q = 0; q < NV; ++q) sh[q][wid] = v[q];
+    target += gridDim.x;
     __syncthreads();
     if (wid == 0) {
-      double out[NV];
+      double o[NV];
 #pragma unroll
-      for (int q = 0; q < NV; ++q) out[q] = warp_sum1(lane < nw ? sh[q][lane] : 0.0);
-      fin(out);
+      for (int q = 0; q < NV; ++q) o[q] = warp_sum1(lane < nw ? sh[q][lane] : 0.0);
+      if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) part[(s + q) * kLoopMaxBlocks + blockIdx.x] = o[q];
+        arrive_wait(L);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < NV; ++q) o[q] = 0.0;
+      for (int b0 = 0; b0 < (int)gridDim.x; b0 += 160) {
+        double t[NV][5];
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+#pragma unroll
+          for (int e = 0; e < 5; ++e) {
+            const int b = b0 + 32 * e + lane;
+            t[q][e] = b < (int)gridDim.x ? __ldcg(part + (s + q) * kLoopMaxBlocks + b) : 0.0;
+          }
+#pragma unroll
+        for (int q = 0; q < NV; ++q) o[q] += (t[q][0] + (t[q][1] + t[q][2])) + (t[q][3] + t[q][4]);
+      }
+#pragma unroll
+      for (int q = 0; q < NV; ++q) o[q] = warp_sum1(o[q]);
+      if (L.bad == 0) fin(o);
     }
     __syncthreads();
-    return true;
+    return L.bad == 0;
   }
 };
 
@@ -1670,6 +1686,8 @@ __device__ __forceinline__ void loop_begin(LoopScal &L, const SolverScal *sc) {
     L.omega = sc->omega;
     L.beta = sc->beta;
     L.relres = sc->relres;
+    L.best = sc->best;
+    L.rmax = sc->rmax;
     L.iter = sc->iter;
     L.done = sc->done;
     L.status = sc->status;
@@ -1693,6 +1711,8 @@ __device__ __forceinline__ void loop_end(const LoopScal &L, const LoopGrid &G) {
     sc->omega = L.omega;
     sc->beta = L.beta;
     sc->relres = L.relres;
+    sc->best = L.best;
+    sc->rmax = L.rmax;
     sc->iter = L.iter;
     sc->done = L.done;
     sc->status = L.status;
@@ -1943,6 +1963,225 @@ __global__ void __launch_bounds__(kLoopBlock, 1) k64cg_loop(Geo g, Stencil<doubl
         lo, hi, [&](long long row) { return LoopVals<2>{{p1[row], r1[row]}}; },
         [&](long long row, const LoopVals<2> &q) { p1[row] = fma(be, q.v[0], q.v[1]); });
     if (!G.sync(L)) break;
+  }
+  loop_end(L, G);
+}
+
+// ---- FP32 CG sweeps in one cooperative launch, the state on chip ----
+// A block a multiprocessor keeps a contiguous range of cells for the whole chunk of iterations:
+// r and A p in registers, p in shared memory with the plane of cells before and after the range, x in
+// shared memory.  What the blocks exchange is r on the cells within a plane of a range's ends
+// (through L2): p there is formed again from it by every block that needs it.  So an iteration
+// has two grid barriers, both of them reductions, and moves a few megabytes instead of the ten
+// vector passes of k32cg*_pq and k32cg_xr.  Same operations per cell as those; the dot products
+// are summed in this partition's order.  A thread owns quads of cells along k where nz is a
+// multiple of four (V = 4), else single cells.  256x128x64: 21.5 -> 12.1 us an iteration (5.3 of
+// it the two reductions; 512 threads with x in registers as well: 12.3).
+constexpr int kCgLoopBlock = 1024;
+constexpr int kCgLoopCells = 16;                // cells a thread
+constexpr size_t kCgLoopShared = 224 * 1024;    // bytes
+
+template <int V>
+struct Cells {
+  float v[V];
+};
+template <int V>
+__device__ __forceinline__ Cells<V> cells_ld(const float *p) {
+  Cells<V> c;
+  if constexpr (V == 4) {
+    const float4 t = *reinterpret_cast<const float4 *>(p);
+    c.v[0] = t.x;
+    c.v[1] = t.y;
+    c.v[2] = t.z;
+    c.v[3] = t.w;
+  } else {
+    c.v[0] = *p;
+  }
+  return c;
+}
+template <int V>
+__device__ __forceinline__ Cells<V> cells_ldcg(const float *p) {
+  Cells<V> c;
+  if constexpr (V == 4) {
+    const float4 t = __ldcg(reinterpret_cast<const float4 *>(p));
+    c.v[0] = t.x;
+    c.v[1] = t.y;
+    c.v[2] = t.z;
+    c.v[3] = t.w;
+  } else {
+    c.v[0] = __ldcg(p);
+  }
+  return c;
+}
+template <int V>
+__device__ __forceinline__ void cells_st(float *p, const Cells<V> &c) {
+  if constexpr (V == 4)
+    *reinterpret_cast<float4 *>(p) = make_float4(c.v[0], c.v[1], c.v[2], c.v[3]);
+  else
+    *p = c.v[0];
+}
+
+// finish_cg32 on the loop's scalars (warp 0)
+__device__ __forceinline__ void loop_finish_cg32(LoopScal &L, double norm0, double tol, double delta, int maxit,
+                                                 double n2) {
+  const double rn = sqrt(n2);
+  double relres, beta, unused;
+  div3(rn, norm0, n2, L.rho, n2, L.rho, relres, beta, unused);
+  if (threadIdx.x != 0) return;
+  L.relres = relres;
+  if (relres < L.best) L.best = relres;
+  if (!isfinite(relres)) {
+    L.done = 1;
+    L.status = CFDGB_ENAN;
+  } else if (L.iter > 16 && relres > 1e3 * L.best) {
+    L.done = 1;
+    L.status = CFDGB_ENOCONV;
+  } else if (L.iter >= maxit) {
+    L.done = 1;
+    L.status = CFDGB_ENOCONV;
+    L.iter += 1;
+  } else if (relres < tol || rn < delta * L.rmax) {
+    L.done = 1;
+    L.status = kStatusRefine;
+    L.iter += 1;
+  } else {
+    L.beta = beta;
+    L.rho = n2;
+    L.restart = isfinite(beta) ? 0 : 1;
+    L.rmax = fmax(L.rmax, rn);
+    L.iter += 1;
+  }
+}
+
+template <int V, int K>
+__global__ void __launch_bounds__(kCgLoopBlock, 1) k32cg_loop(Geo g, Stencil<float> st, Vec32 v, double *part,
+                                                              SolverScal *sc, int iters, int chunk) {
+  extern __shared__ __align__(16) float csm[];
+  __shared__ LoopScal L;
+  loop_begin(L, sc);
+  if (L.done) return;  // the same in every block: sc is written only after the last barrier
+  LoopGrid G = loop_grid(sc, part);
+  const double norm0 = sc->norm0, tol = sc->tol, delta = sc->delta;
+  const int maxit = sc->maxit, tid = threadIdx.x;
+  const int n = (int)g.ncell, nz = g.nzc, H = g.nyc * nz;  // a plane
+  const int lo = min(n, (int)blockIdx.x * chunk), m = min(n - lo, chunk);
+  float *const ps = csm + H;                // p of the range's cells; the planes beside it at -H and m
+  float *const xs = csm + 2 * H + chunk;
+  const float *const r1 = v.r1;
+  float *const pg = sc->par ? v.p[1] : v.p[0];
+  const float *const c = st.c[13];  // uniform grid, SPE rows: an axis's coefficient where the neighbour exists
+  const float c0 = c[0], c1 = c[1], c2 = c[2], c4 = c[4], c5 = c[5], c6 = c[6];
+  // halo cells: h < H before the range, then after it
+  const int left = min(lo, H), right = min(n - (lo + m), H);
+  Cells<V> r[K], q[K];
+  unsigned fl[(K + 3) / 4];  // 8 bits a group: neighbours -x, -y, -z, +z, +y, +x; -z, +z across the wrap
+#pragma unroll
+  for (int u = 0; u < (K + 3) / 4; ++u) fl[u] = 0;
+#pragma unroll
+  for (int u = 0; u < K; ++u) {
+    const int b = V * (tid + kCgLoopBlock * u);
+    if (b >= m) break;
+    r[u] = cells_ldcg<V>(r1 + lo + b);
+    cells_st<V>(ps + b, cells_ldcg<V>(pg + lo + b));
+    cells_st<V>(xs + b, cells_ldcg<V>(v.x + lo + b));
+    int ic, jc, kc;
+    row_cijk(lo + b, g.nyc, nz, ic, jc, kc);
+    const bool pz = g.pz != 0, first = kc == 0, last = kc + V >= nz;
+    const unsigned f = (ic > 0) | (jc > 0) << 1 | (!first || pz) << 2 | (!last || pz) << 3 | (jc < g.nyc - 1) << 4 |
+                       (ic < g.nxc - 1) << 5 | (first && pz) << 6 | (last && pz) << 7;
+    fl[u / 4] |= f << (8 * (u % 4));
+  }
+  for (int h = V * tid; h < left; h += V * kCgLoopBlock) cells_st<V>(ps - left + h, cells_ldcg<V>(pg + lo - left + h));
+  for (int h = V * tid; h < right; h += V * kCgLoopBlock) cells_st<V>(ps + m + h, cells_ldcg<V>(pg + lo + m + h));
+  for (int it = 0; it < iters; ++it) {
+    const float be = (float)L.beta;
+    const bool rst = L.restart != 0;
+    auto next = [&](float *p, const Cells<V> &rr) {  // p = r + beta p (restart: r)
+      Cells<V> t = rr;
+      if (!rst) {
+        const Cells<V> o = cells_ld<V>(p);
+#pragma unroll
+        for (int e = 0; e < V; ++e) t.v[e] = fmaf(be, o.v[e], rr.v[e]);
+      }
+      cells_st<V>(p, t);
+    };
+#pragma unroll 4
+    for (int h = V * tid; h < left; h += V * kCgLoopBlock) next(ps - left + h, cells_ldcg<V>(r1 + lo - left + h));
+#pragma unroll 4
+    for (int h = V * tid; h < right; h += V * kCgLoopBlock) next(ps + m + h, cells_ldcg<V>(r1 + lo + m + h));
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      const int b = V * (tid + kCgLoopBlock * u);
+      if (b >= m) break;
+      next(ps + b, r[u]);
+    }
+    __syncthreads();
+    float a = 0.0f;
+#pragma unroll
+    for (int u = 0; u < K; ++u) {  // q = A p: stencil_apply_diff's terms in its order
+      const int b = V * (tid + kCgLoopBlock * u);
+      if (b >= m) break;
+      const unsigned f = fl[u / 4] >> (8 * (u % 4));
+      const Cells<V> p = cells_ld<V>(ps + b);
+      Cells<V> xm = p, ym = p, yp = p, xp = p;  // a missing neighbour: no difference
+      if (f & 1u) xm = cells_ld<V>(ps + b - H);
+      if (f & 2u) ym = cells_ld<V>(ps + b - nz);
+      if (f & 16u) yp = cells_ld<V>(ps + b + nz);
+      if (f & 32u) xp = cells_ld<V>(ps + b + H);
+      float zm = p.v[0], zp = p.v[V - 1];
+      if (f & 4u) zm = ps[b + ((f & 64u) ? nz - 1 : -1)];
+      if (f & 8u) zp = ps[b + ((f & 128u) ? V - nz : V)];
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const float fc = p.v[e];
+        float t = c0 * (xm.v[e] - fc);
+        t = fmaf(c1, ym.v[e] - fc, t);
+        t = fmaf(c2, (e == 0 ? zm : p.v[e > 0 ? e - 1 : 0]) - fc, t);
+        t = fmaf(c4, (e == V - 1 ? zp : p.v[e < V - 1 ? e + 1 : V - 1]) - fc, t);
+        t = fmaf(c5, yp.v[e] - fc, t);
+        t = fmaf(c6, xp.v[e] - fc, t);
+        q[u].v[e] = t;
+        a = fmaf(t, fc, a);
+      }
+    }
+    {
+      double d[1] = {(double)a};
+      if (!G.reduce<1>(L, d, 0, [&](const double (&o)[1]) {
+            const double al = L.rho / o[0];
+            if (threadIdx.x == 0) L.alpha = al;
+          }))
+        break;
+    }
+    const float al = (float)L.alpha;
+    a = 0.0f;
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      const int b = V * (tid + kCgLoopBlock * u);
+      if (b >= m) break;
+      const Cells<V> p = cells_ld<V>(ps + b);
+      Cells<V> x = cells_ld<V>(xs + b);
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        x.v[e] = fmaf(al, p.v[e], x.v[e]);
+        r[u].v[e] = fmaf(-al, q[u].v[e], r[u].v[e]);
+        a = fmaf(r[u].v[e], r[u].v[e], a);
+      }
+      cells_st<V>(xs + b, x);
+      if (b < H || b >= m - H) cells_st<V>(v.r1 + lo + b, r[u]);  // what other blocks read
+    }
+    {
+      double d[1] = {(double)a};
+      if (!G.reduce<1>(L, d, 1, [&](const double (&o)[1]) { loop_finish_cg32(L, norm0, tol, delta, maxit, o[0]); })) break;
+    }
+    if (L.done) break;
+  }
+#pragma unroll
+  for (int u = 0; u < K; ++u) {
+    const int b = V * (tid + kCgLoopBlock * u);
+    if (b >= m) break;
+    cells_st<V>(v.r1 + lo + b, r[u]);
+    cells_st<V>(v.x + lo + b, cells_ld<V>(xs + b));
+    cells_st<V>(pg + lo + b, cells_ld<V>(ps + b));
   }
   loop_end(L, G);
 }
@@ -2629,6 +2868,57 @@ int loop64_iters(long long ncell) {
   return (int)(n < 16 ? 16 : (n > 256 ? 256 : n));
 }
 size_t loop64_part_doubles() { return (size_t)kLoopSlots * kLoopMaxBlocks; }
+
+// blocks, cells a block and shared memory of k32cg_loop; 0 blocks: not this grid (not uniform, too
+// many cells for the multiprocessors' registers and shared memory) or device
+struct CgLoop {
+  int blocks, chunk, v, k;
+  size_t smem;
+};
+static CgLoop cg32_loop_plan(const Geo &g, const Stencil<float> &st, int nsm) {
+  CgLoop P{};
+  if (g.nonuni || st.jac || nsm < 1 || g.ncell > (long long)std::min(nsm, kLoopMaxBlocks) * kCgLoopBlock * kCgLoopCells)
+    return P;
+  for (int cls = 0; cls < 27; ++cls)  // one coefficient an axis side
+    for (int e = 0; e < 7; ++e)
+      if (e != 3 && st.c[cls][e] != 0.0f && st.c[cls][e] != st.c[13][e]) return P;
+  const int sms = std::min(nsm, kLoopMaxBlocks);
+  P.v = g.nzc % 4 == 0 ? 4 : 1;
+  P.chunk = (int)(((g.ncell + sms - 1) / sms + 31) / 32 * 32);
+  const int groups = (P.chunk / P.v + kCgLoopBlock - 1) / kCgLoopBlock;
+  P.k = P.v == 4 ? (groups <= 1 ? 1 : groups <= 2 ? 2 : 4) : (groups <= 4 ? 4 : 16);
+  P.smem = 4 * (2 * (size_t)g.nyc * g.nzc + 2 * (size_t)P.chunk);
+  if (groups > P.k || P.smem > kCgLoopShared) return P;
+  P.blocks = (int)((g.ncell + P.chunk - 1) / P.chunk);
+  return P;
+}
+static void (*cg32_loop_kernel(const CgLoop &P))(Geo, Stencil<float>, Vec32, double *, SolverScal *, int, int) {
+  if (P.v == 4) return P.k == 1 ? k32cg_loop<4, 1> : P.k == 2 ? k32cg_loop<4, 2> : k32cg_loop<4, 4>;
+  return P.k == 4 ? k32cg_loop<1, 4> : k32cg_loop<1, 16>;
+}
+bool cg32_loop_fits(const Geo &g, const Stencil<float> &st, int nsm) {
+  const CgLoop P = cg32_loop_plan(g, st, nsm);
+  if (P.blocks == 0 || loop64_blocks(1) == 0) return false;  // (loop64_blocks: the device takes cooperative launches)
+  int n = 0;
+  const auto kernel = cg32_loop_kernel(P);
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCgLoopShared) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kCgLoopBlock, P.smem) == cudaSuccess && n >= 1;
+}
+void launch_cg32_loop(cudaStream_t s, const Geo &g, const Stencil<float> &st, KrylovVecs<float> v, float *const p2[2],
+                      float *const ap2[2], double *part_buf, SolverScal *sc, int nsm) {
+  const CgLoop P = cg32_loop_plan(g, st, nsm);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(P.blocks);
+  cfg.blockDim = dim3(kCgLoopBlock);
+  cfg.dynamicSmemBytes = P.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, cg32_loop_kernel(P), g, st, v32(v, p2, ap2), part_buf, sc, kCg32LoopIters, P.chunk);
+}
 
 static void launch_loop(cudaStream_t s, bool cg, const Geo &g, const Stencil<double> &st, KrylovVecs<double> v,
                         double *part_buf, SolverScal *sc, int blocks, int iters) {
