@@ -366,15 +366,21 @@ __global__ void __launch_bounds__(kBlock) k_update_uf_fast(
     int i, j, k;
     row_ijk(g, row, i, j, k);
     const long long ic = pidx(g, i, j, k);
-    const double ec = eta[ic];
+    // every load first, from the cell itself where the face is a boundary one: behind the branches
+    // below they would wait for one another (512x256x64: 170 -> 161 us; floor 89, the FP64 pipe 92)
+    const bool fx = i < g.nx - 3, fy = j < g.ny - 3, fz = k < g.nz - 3 + g.pz;
+    const long long iX = fx ? ic + g.sx : ic, iY = fy ? ic + g.sy : ic;
+    // periodic z: the top face, its upper cell the first one
+    const long long iZ = !fz ? ic : (g.pz && k == g.nz - 3) ? ic - (g.nzc - 1) : ic + 1;
+    const double ec = eta[ic], eX = eta[iX], eY = eta[iY], eZ = eta[iZ];
+    const double pc = p[ic], pX = p[iX], pY = p[iY], pZ = p[iZ];
+    const double uc = us[ic], vc = vs[ic], wc = ws[ic];
     const bool bc = nonzero(ec);
-    if (i < g.nx - 3) {
-      const long long icP = ic + g.sx;
-      const double T2 = fma(UNI ? gx : -(dt * g.rDxs[i]), p[icP] - p[ic], us[ic]);
-      const double en = eta[icP];
+    if (fx) {
+      const double T2 = fma(UNI ? gx : -(dt * g.rDxs[i]), pX - pc, uc);
       double n3 = T2;
-      if (bc || nonzero(en)) {
-        const DfibFace d = dfib_face(T2, en, ec, g.hfx[i], rdt, g.Dx + i, g.Dy + j, g.Dz + k);
+      if (bc || nonzero(eX)) {
+        const DfibFace d = dfib_face(T2, eX, ec, g.hfx[i], rdt, g.Dx + i, g.Dy + j, g.Dz + k);
         n3 = d.n3;
         acc[0] += d.f;
       }
@@ -382,13 +388,11 @@ __global__ void __launch_bounds__(kBlock) k_update_uf_fast(
     } else if (ui) {
       u3[ic] = ui[ic];
     }
-    if (j < g.ny - 3) {
-      const long long icP = ic + g.sy;
-      const double T2 = fma(UNI ? gy : -(dt * g.rDys[j]), p[icP] - p[ic], vs[ic]);
-      const double en = eta[icP];
+    if (fy) {
+      const double T2 = fma(UNI ? gy : -(dt * g.rDys[j]), pY - pc, vc);
       double n3 = T2;
-      if (bc || nonzero(en)) {
-        const DfibFace d = dfib_face(T2, en, ec, g.hfy[j], rdt, g.Dx + i, g.Dy + j, g.Dz + k);
+      if (bc || nonzero(eY)) {
+        const DfibFace d = dfib_face(T2, eY, ec, g.hfy[j], rdt, g.Dx + i, g.Dy + j, g.Dz + k);
         n3 = d.n3;
         acc[1] += d.f;
       }
@@ -396,11 +400,9 @@ __global__ void __launch_bounds__(kBlock) k_update_uf_fast(
     } else if (vi) {
       v3[ic] = vi[ic];
     }
-    if (k < g.nz - 3 + g.pz) {  // periodic z: the top face, its upper cell the first one
-      const long long icP = (g.pz && k == g.nz - 3) ? ic - (g.nzc - 1) : ic + 1;
-      const double T2 = fma(UNI ? gz : -(dt * g.rDzs[k]), p[icP] - p[ic], ws[ic]);
-      const double en = eta[icP];
-      w3[ic] = (bc || nonzero(en)) ? dfib_face(T2, en, ec, g.hfz[k], rdt, nullptr, nullptr, nullptr).n3 : T2;
+    if (fz) {
+      const double T2 = fma(UNI ? gz : -(dt * g.rDzs[k]), pZ - pc, wc);
+      w3[ic] = (bc || nonzero(eZ)) ? dfib_face(T2, eZ, ec, g.hfz[k], rdt, nullptr, nullptr, nullptr).n3 : T2;
     } else if (wi) {
       w3[ic] = wi[ic];
     }
@@ -423,6 +425,14 @@ __global__ void __launch_bounds__(kBlock) k_rhs_fast(Geo g, double dt_arg, const
                                                      const double *__restrict__ ws, int jacobi, Stencil<double> st,
                                                      double *__restrict__ b) {
   const double ndt = -1.0 / (dtp ? *dtp : dt_arg);
+  // uniform grid: the row's factor by class, once a block (the FP64 pipe bounds the kernel: seven
+  // instructions a cell instead of eight, 512x256x64 136 -> 118 us)
+  __shared__ double fac[27];
+  const bool tab = !g.nonuni;
+  if (tab) {
+    if (threadIdx.x < 27) fac[threadIdx.x] = jacobi ? st.c[threadIdx.x][7] * ndt : ndt;
+    __syncthreads();
+  }
   for (long long row = blockIdx.x * (long long)kBlock + threadIdx.x; row < g.ncell;
        row += (long long)gridDim.x * kBlock) {
     int i, j, k;
@@ -431,7 +441,7 @@ __global__ void __launch_bounds__(kBlock) k_rhs_fast(Geo g, double dt_arg, const
     const long long zb = (g.pz && k == 2) ? ic + g.nzc - 1 : ic - 1;  // periodic z: face nz-3
     const double div = fma(us[ic] - us[ic - g.sx], g.rDx[i],
                            fma(vs[ic] - vs[ic - g.sy], g.rDy[j], (ws[ic] - ws[zb]) * g.rDz[k]));
-    b[row] = (jacobi ? row_jp(g, st, i - 2, j - 2, k - 2, row) * ndt : ndt) * div;
+    b[row] = (tab ? fac[row_class(g, i - 2, j - 2, k - 2)] : jacobi ? row_jp(g, st, i - 2, j - 2, k - 2, row) * ndt : ndt) * div;
   }
 }
 
