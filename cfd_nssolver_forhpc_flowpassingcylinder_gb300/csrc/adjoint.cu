@@ -32,8 +32,9 @@ namespace cfdgb {
 // ---- BC^T: transpose of the velocity part of k_bc_x/y/z --------------------------------
 // A write dst = a + s * src (chains dst1 = dst2 = ... = a + s * src) has adjoint
 // lam[src] += s * sum(lam[dst]); lam[dst] = 0.  Within a phase a thread owns one line.
-__global__ void __launch_bounds__(kBlock) k_adj_bc_x(Geo g, BcTable t, double *lu, double *lv, double *lw,
-                                                     double *linlet) {
+__global__ void __launch_bounds__(kBlock) k_adj_bc_x(Geo g, BcTable t, double *__restrict__ lu,
+                                                     double *__restrict__ lv, double *__restrict__ lw,
+                                                     double *__restrict__ linlet) {
   const int nyc = g.nyc, nzc = g.nzc, nx = g.nx;
   for (int q = blockIdx.x * kBlock + threadIdx.x; q < nyc * nzc; q += gridDim.x * kBlock) {
     const int j = q / nzc + 2, k = q % nzc + 2;
@@ -62,7 +63,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_bc_x(Geo g, BcTable t, double *l
   }
 }
 
-__global__ void __launch_bounds__(kBlock) k_adj_bc_y(Geo g, BcTable t, double *lu, double *lv, double *lw) {
+__global__ void __launch_bounds__(kBlock) k_adj_bc_y(Geo g, BcTable t, double *__restrict__ lu,
+                                                     double *__restrict__ lv, double *__restrict__ lw) {
   const int nxc = g.nxc, nzc = g.nzc, ny = g.ny;
   for (int q = blockIdx.x * kBlock + threadIdx.x; q < nxc * nzc; q += gridDim.x * kBlock) {
     const int i = q / nzc + 2, k = q % nzc + 2;
@@ -90,7 +92,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_bc_y(Geo g, BcTable t, double *l
   }
 }
 
-__global__ void __launch_bounds__(kBlock) k_adj_bc_z(Geo g, BcTable t, double *lu, double *lv, double *lw) {
+__global__ void __launch_bounds__(kBlock) k_adj_bc_z(Geo g, BcTable t, double *__restrict__ lu,
+                                                     double *__restrict__ lv, double *__restrict__ lw) {
   const int nxc = g.nxc, nyc = g.nyc, nz = g.nz;
   for (int q = blockIdx.x * kBlock + threadIdx.x; q < nxc * nyc; q += gridDim.x * kBlock) {
     const int i = q / nyc + 2, j = q % nyc + 2;
@@ -118,53 +121,63 @@ __global__ void __launch_bounds__(kBlock) k_adj_bc_z(Geo g, BcTable t, double *l
   }
 }
 
+// lambda of T2 on a face next to the body (out of line, so that the branch to it stays one)
+__device__ __noinline__ double adj_dfib(double l, double en, double ec, double h, double w) {
+  const double e = fma(en - ec, h, ec);
+  return (1.0 - e) * l + e * w;
+}
+
 // ---- correction^T, per face: lambda of T2 = u* - dt grad p and of eta_f -------------------
 // cw: weight of Cd^n in the objective times 2 / (lz dt) (0 outside the averaging window)
+// These kernels and RHS^T are FP64-pipe-bound (a warp instruction takes 64 cycles of a
+// scheduler whatever its lanes do), so the products of the metrics (the adjoint's grids are
+// uniform) are taken once a thread, the faces away from the body skip the DFIB terms (lambda* =
+// lambda there), and lambda of eta_f is T2 (cw vol - lambda).  256x128x32: correction 83 + 66 ->
+// 31 + 39 us, RHS^T 79 -> 41.
 __global__ void __launch_bounds__(kBlock) k_adj_corr(Geo g, double dt, double cw, const double *__restrict__ eta,
                                                      const double *__restrict__ p, const double *__restrict__ us,
                                                      const double *__restrict__ vs, const double *__restrict__ ws,
                                                      const double *__restrict__ lu, const double *__restrict__ lv,
-                                                     const double *__restrict__ lw, double *lus, double *lvs,
-                                                     double *lws, double *lex, double *ley, double *lez) {
+                                                     const double *__restrict__ lw, double *__restrict__ lus,
+                                                     double *__restrict__ lvs, double *__restrict__ lws,
+                                                     double *__restrict__ lex, double *__restrict__ ley,
+                                                     double *__restrict__ lez) {
+  const double gx = -(dt * g.rDxs[2]), gy = -(dt * g.rDys[2]), gz = -(dt * g.rDzs[2]);
+  const double cv = cw * (g.Dx[2] * g.Dy[2] * g.Dz[2]);
   ROWS(g) {
     int i, j, k;
     row_ijk(g, row, i, j, k);
     const long long c = pidx(g, i, j, k);
-    const double ec = eta[c];
-    if (i < g.nx - 3) {
-      const long long cp = c + g.sx;
-      const double T2 = us[c] - dt * (p[cp] - p[c]) * g.rDxs[i];
-      const double e = ec + (eta[cp] - ec) * g.hfx[i];
-      const double vol = g.Dx[i] * g.Dy[j] * g.Dz[k];
-      lus[c] = (1.0 - e) * lu[c] + cw * e * vol;
-      lex[c] = -T2 * lu[c] + cw * T2 * vol;
-    } else {
-      lus[c] = 0.0;
-      lex[c] = 0.0;
+    const bool fx = i < g.nx - 3, fy = j < g.ny - 3, fz = k < g.nz - 3;
+    const long long cx = fx ? c + g.sx : c, cy = fy ? c + g.sy : c, cz = fz ? c + 1 : c;
+    const double ec = eta[c], ex = eta[cx], ey = eta[cy], ez = eta[cz];
+    const double pc = p[c], px = p[cx], py = p[cy], pz = p[cz];
+    const double uc = us[c], vc = vs[c], wc = ws[c], lu0 = lu[c], lv0 = lv[c], lw0 = lw[c];
+    const bool solid = !is_zero(ec);
+    double o[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (fx) {
+      const double T2 = fma(gx, px - pc, uc);
+      o[0] = solid || !is_zero(ex) ? adj_dfib(lu0, ex, ec, g.hfx[i], cv) : lu0;
+      o[3] = T2 * (cv - lu0);
     }
-    if (j < g.ny - 3) {
-      const long long cp = c + g.sy;
-      const double T2 = vs[c] - dt * (p[cp] - p[c]) * g.rDys[j];
-      const double e = ec + (eta[cp] - ec) * g.hfy[j];
-      lvs[c] = (1.0 - e) * lv[c];
-      ley[c] = -T2 * lv[c];
-    } else {
-      lvs[c] = 0.0;
-      ley[c] = 0.0;
+    if (fy) {
+      const double T2 = fma(gy, py - pc, vc);
+      o[1] = solid || !is_zero(ey) ? adj_dfib(lv0, ey, ec, g.hfy[j], 0.0) : lv0;
+      o[4] = -T2 * lv0;
     }
-    if (k < g.nz - 3) {
-      const long long cp = c + 1;
-      const double T2 = ws[c] - dt * (p[cp] - p[c]) * g.rDzs[k];
-      const double e = ec + (eta[cp] - ec) * g.hfz[k];
-      lws[c] = (1.0 - e) * lw[c];
-      lez[c] = -T2 * lw[c];
-    } else {
-      lws[c] = 0.0;
-      lez[c] = 0.0;
+    if (fz) {
+      const double T2 = fma(gz, pz - pc, wc);
+      o[2] = solid || !is_zero(ez) ? adj_dfib(lw0, ez, ec, g.hfz[k], 0.0) : lw0;
+      o[5] = -T2 * lw0;
     }
+    lus[c] = o[0];
+    lvs[c] = o[1];
+    lws[c] = o[2];
+    lex[c] = o[3];
+    ley[c] = o[4];
+    lez[c] = o[5];
   }
 }
-
 // per cell: lambda_p (compact) from the faces around it, and eta's share of the faces'
 // interpolated solid fractions (accumulated over steps); ghost faces hold zeros
 __global__ void __launch_bounds__(kBlock) k_adj_corr_gather(Geo g, double dt, const double *__restrict__ lus,
@@ -172,21 +185,25 @@ __global__ void __launch_bounds__(kBlock) k_adj_corr_gather(Geo g, double dt, co
                                                             const double *__restrict__ lws,
                                                             const double *__restrict__ lex,
                                                             const double *__restrict__ ley,
-                                                            const double *__restrict__ lez, double *lx, double *leta,
-                                                            double *part, StepScal *ss) {
+                                                            const double *__restrict__ lez, double *__restrict__ lx,
+                                                            double *__restrict__ leta, double *part, StepScal *ss) {
   double acc[1] = {0.0};
+  const double fx = dt * g.rDxs[2], fy = dt * g.rDys[2], fz = dt * g.rDzs[2];
+  const double hx = g.hfx[2], hy = g.hfy[2], hz = g.hfz[2], ax = 1.0 - hx, ay = 1.0 - hy, az = 1.0 - hz;
   ROWS(g) {
     int i, j, k;
     row_ijk(g, row, i, j, k);
     const long long c = pidx(g, i, j, k);
-    const double l = dt * (lus[c] * g.rDxs[i] - lus[c - g.sx] * g.rDxs[i - 1] + lvs[c] * g.rDys[j] -
-                           lvs[c - g.sy] * g.rDys[j - 1] + lws[c] * g.rDzs[k] - lws[c - 1] * g.rDzs[k - 1]);
+    const double u0 = lus[c], u1 = lus[c - g.sx], v0 = lvs[c], v1 = lvs[c - g.sy], w0 = lws[c], w1 = lws[c - 1];
+    const double a0 = lex[c], a1 = lex[c - g.sx], b0 = ley[c], b1 = ley[c - g.sy], c0 = lez[c], c1 = lez[c - 1];
+    const double l = fma(fz, w0 - w1, fma(fy, v0 - v1, fx * (u0 - u1)));
+    double e = leta[c];
+    e = fma(ax, a0, fma(hx, a1, e));
+    e = fma(ay, b0, fma(hy, b1, e));
+    e = fma(az, c0, fma(hz, c1, e));
     lx[row] = l;
     acc[0] += l;
-    const double itx = g.hfx[i], itx1 = g.hfx[i - 1], ity = g.hfy[j], ity1 = g.hfy[j - 1];
-    const double itz = g.hfz[k], itz1 = g.hfz[k - 1];
-    leta[c] += (1.0 - itx) * lex[c] + itx1 * lex[c - g.sx] + (1.0 - ity) * ley[c] + ity1 * ley[c - g.sy] +
-               (1.0 - itz) * lez[c] + itz1 * lez[c - 1];
+    leta[c] = e;
   }
   double out[1];
   if (grid_sum<1>(acc, part, &ss->cnt[4], out) && threadIdx.x == 0) ss->fsum[0] = out[0];  // sum of lambda_x
@@ -207,24 +224,31 @@ __global__ void __launch_bounds__(kBlock) k_sum(Geo g, const double *__restrict_
 // ---- RHS^T: b = -(1/dt) div u* ---------------------------------------------------------
 // Interior faces feed lambda_u*; the faces T1 copies from U^n (x: i = 1 and nx-3; y, z
 // alike) feed lambda_U^n directly.  Each face is owned by one thread.
-__global__ void __launch_bounds__(kBlock) k_adj_rhs(Geo g, double dt, const double *__restrict__ lb, double *lus,
-                                                    double *lvs, double *lws, double *lu, double *lv, double *lw) {
-  const double ddt = 1.0 / dt;
+__global__ void __launch_bounds__(kBlock) k_adj_rhs(Geo g, double dt, const double *__restrict__ lb,
+                                                    double *__restrict__ lus, double *__restrict__ lvs,
+                                                    double *__restrict__ lws, double *__restrict__ lu,
+                                                    double *__restrict__ lv, double *__restrict__ lw) {
+  const double ddt = 1.0 / dt, ux = ddt * g.rDx[2], uy = ddt * g.rDy[2], uz = ddt * g.rDz[2];
   const long long nyz = (long long)g.nyc * g.nzc;
   ROWS(g) {
     int i, j, k;
     row_ijk(g, row, i, j, k);
     const long long c = pidx(g, i, j, k);
-    const double l = lb[row];
-    if (i < g.nx - 3) lus[c] += -ddt * g.rDx[i] * l + ddt * g.rDx[i + 1] * lb[row + nyz];
-    else lu[c] += -ddt * g.rDx[i] * l;
-    if (i == 2) lu[c - g.sx] += ddt * g.rDx[i] * l;
-    if (j < g.ny - 3) lvs[c] += -ddt * g.rDy[j] * l + ddt * g.rDy[j + 1] * lb[row + g.nzc];
-    else lv[c] += -ddt * g.rDy[j] * l;
-    if (j == 2) lv[c - g.sy] += ddt * g.rDy[j] * l;
-    if (k < g.nz - 3) lws[c] += -ddt * g.rDz[k] * l + ddt * g.rDz[k + 1] * lb[row + 1];
-    else lw[c] += -ddt * g.rDz[k] * l;
-    if (k == 2) lw[c - 1] += ddt * g.rDz[k] * l;
+    const bool fx = i < g.nx - 3, fy = j < g.ny - 3, fz = k < g.nz - 3;
+    const double l = lb[row], lxp = lb[fx ? row + nyz : row], lyp = lb[fy ? row + g.nzc : row], lzp = lb[fz ? row + 1 : row];
+    const double su = lus[c], sv = lvs[c], sw = lws[c];
+    // the cell's terms (one product an axis), and the next cell's on the face between them
+    const double tx = ux * l, ty = uy * l,
+                 tz = uz * l;
+    if (fx) lus[c] = fma(ux, lxp, su - tx);
+    else lu[c] -= tx;
+    if (i == 2) lu[c - g.sx] += tx;
+    if (fy) lvs[c] = fma(uy, lyp, sv - ty);
+    else lv[c] -= ty;
+    if (j == 2) lv[c - g.sy] += ty;
+    if (fz) lws[c] = fma(uz, lzp, sw - tz);
+    else lw[c] -= tz;
+    if (k == 2) lw[c - 1] += tz;
   }
 }
 
