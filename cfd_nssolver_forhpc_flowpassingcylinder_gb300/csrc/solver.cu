@@ -2666,10 +2666,10 @@ __device__ __forceinline__ float scaled_residual(const Geo &g, const Stencil<dou
   return jacobi ? fmaf(-mi, d2f_int(row_jp(g, st, ic, jc, kc, row)), r) : r - mi;
 }
 
-// start of a sweep: x = 0, r0 = r1 = scaled residual, rho = <r1, r1>; restart = 1 makes the
-// first k32_pap take p = r1 (the reference's p1 = r0); delta, peak: this sweep's residual
-// reductions (against its start and its largest residual).  first: also the solve's set-up
-// (iteration count, the FP32 estimate's normalisation).
+// start of a sweep: x = 0, r1 = scaled residual, rho = <r1, r1>; restart = 1 makes the first p
+// kernel set r0 = r1 and take p = r1 (the reference's p1 = r0); delta, peak: this sweep's
+// residual reductions (against its start and its largest residual).  first: also the solve's
+// set-up (iteration count, the FP32 estimate's normalisation).
 __global__ void __launch_bounds__(kBlock) k_refine_start32(Geo g, Stencil<double> st, int jacobi, Vec32 v,
                                                             const float *__restrict__ rf, const StepScal *ss,
                                                             double delta, double peak, int first, double *part,
@@ -2685,7 +2685,6 @@ __global__ void __launch_bounds__(kBlock) k_refine_start32(Geo g, Stencil<double
     const long long row = ROW(g);
     const float r = scaled_residual(g, st, jacobi, rf, mi, inv32, ic, jc, kc, row);
     v.x[row] = 0.0f;
-    v.r0[row] = r;
     v.r1[row] = r;
     acc.add(r, r);
   }
