@@ -992,8 +992,13 @@ __global__ void __launch_bounds__(1024) k_mg_coarse(MgLevelT<T> L, int sweeps, c
 // 48 KB: one block working on more cells per barrier (a 16K-cell level, 192 KB) ran slower
 // than the same level's launched kernels (measured on 512x256x64)
 constexpr int kMgTailBytes = 48 * 1024;
+// FP64: 1024 cells.  One multiprocessor's FP64 pipe (2 lanes a clock) takes longer for a level of
+// 2048 cells than that level's launched kernels: runs on 512x256x64 60.1 -> 59.2 ms, on
+// 256x128x32 12.1 -> 11.1 ms against 3072 cells (48 KB); 128 cells 59.3 and 11.3 ms
 template <typename T>
-constexpr int tail_cells_max() { return kMgTailBytes / (2 * (int)sizeof(T)); }
+constexpr int tail_cells_max() {
+  return sizeof(T) == sizeof(double) ? 1024 : kMgTailBytes / (2 * (int)sizeof(T));
+}
 
 // Unsigned division by an invariant d >= 1 (Granlund and Montgomery, "Division by invariant
 // integers using multiplication", PLDI 1994, the round-up method): with l = ceil(log2 d) and
