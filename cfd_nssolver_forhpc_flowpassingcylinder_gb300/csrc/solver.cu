@@ -2148,6 +2148,7 @@ __global__ void __launch_bounds__(kCgLoopBlock, 1) k32cg_loop(Geo g, Stencil<flo
                        (ic < g.nxc - 1) << 5 | (first && pz) << 6 | (last && pz) << 7;
     fl[u / 4] |= f << (8 * (u % 4));
   }
+  // (a cell beside the range is one thread's, here and in every iteration: no barrier in between)
   for (int h = V * tid; h < left; h += V * kCgLoopBlock) cells_st<V>(ps - left + h, cells_ldcg<V>(pg + lo - left + h));
   for (int h = V * tid; h < right; h += V * kCgLoopBlock) cells_st<V>(ps + m + h, cells_ldcg<V>(pg + lo + m + h));
   for (int it = 0; it < iters; ++it) {
@@ -2469,7 +2470,8 @@ __global__ void __launch_bounds__(kBlock) k_residual64(Geo g, Stencil<double> st
 // rounded entries, products and sums of 2^-53 each (root mean square against 80-bit on a
 // solution of 128x64x16: 1.2e-15 against 1.25e-14).  Two FP64 instructions a cell (the subtraction and the
 // norm).  A thread owns two rows of a pair of cells along k and marches along x; z neighbours
-// across pairs by shuffles.  Values of x outside the integer form's range (all zero, Inf, NaN,
+// across pairs by shuffles.  (All relative to the largest |x|: where x spans more than 2^7, small
+// values are rounded at 2^-60 of the largest.)  Values of x outside the integer form's range (all zero, Inf, NaN,
 // extreme exponents) take the FMA chain.  The next plane's loads are issued before this one's arithmetic.
 // 512x256x64: 164 -> 80 us (without the loads ahead 96; the integer chains of 16 warps).
 struct FixOp {
