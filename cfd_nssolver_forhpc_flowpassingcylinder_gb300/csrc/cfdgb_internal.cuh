@@ -176,16 +176,11 @@ __device__ __forceinline__ long long d2fix(double x, int em) {
   const long long q = (long long)((m << 7) >> s), n = (long long)(hi >> 31);
   return (q ^ n) - n;
 }
-// a 64-bit integer below 2^62, times 2^shift, to the nearest double by integer operations (the
-// result is a normal number or zero)
+// a 64-bit integer below 2^62, times 2^shift, to the nearest double (the result is a normal number
+// or zero)
 __device__ __forceinline__ double fix2d(long long t, int shift) {
-  if (t == 0) return 0.0;
-  unsigned long long a = (unsigned long long)(t < 0 ? -t : t);
-  const int lz = __clzll((long long)a);
-  a = (a << lz) >> 1;  // bit 62 the leading one
-  a = (a + 0x1ffu + ((a >> 10) & 1u)) >> 10;
-  const unsigned long long b = ((unsigned long long)(1085 - lz + shift) << 52) + a;
-  return __longlong_as_double((long long)(b | ((unsigned long long)t & 0x8000000000000000ULL)));
+  const double v = (double)t;
+  return __hiloint2double(t == 0 ? 0 : __double2hiint(v) + (int)((unsigned)shift << 20), __double2loint(v));
 }
 
 // compact row -> padded (i,j,k).  Grids below 2^31 cells divide in 32 bits: a 64-bit

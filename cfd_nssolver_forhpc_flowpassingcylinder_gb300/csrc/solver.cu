@@ -2468,12 +2468,14 @@ __global__ void __launch_bounds__(kBlock) k_residual64(Geo g, Stencil<double> st
 // (29 and 31 bits, so that the products' high parts are nine wide multiply-adds), converted once
 // and subtracted from b in FP64.  Its error is below 2^-54 of w |x|_max, against the FMA chain's
 // rounded entries, products and sums of 2^-53 each (root mean square against 80-bit on a
-// solution of 128x64x16: 1.2e-15 against 1.25e-14).  Two FP64 instructions a cell (the subtraction and the
-// norm).  A thread owns two rows of a pair of cells along k and marches along x; z neighbours
-// across pairs by shuffles.  (All relative to the largest |x|: where x spans more than 2^7, small
-// values are rounded at 2^-60 of the largest.)  Values of x outside the integer form's range (all zero, Inf, NaN,
-// extreme exponents) take the FMA chain.  The next plane's loads are issued before this one's arithmetic.
-// 512x256x64: 164 -> 80 us (without the loads ahead 96; the integer chains of 16 warps).
+// solution of 128x64x16: 1.2e-15 against 1.25e-14).  All relative to the largest |x|: where x spans
+// more than 2^7, small values are rounded at 2^-60 of the largest.  Three FP64-pipe instructions a
+// cell (the conversion, the subtraction and the norm).  A thread owns two rows of a pair of cells
+// along k and marches along x; z neighbours across pairs by shuffles.  Values of x outside the
+// integer form's range (all zero, Inf, NaN, extreme exponents) take the FMA chain.  The next
+// plane's loads are issued before this one's arithmetic.  512x256x64: 164 -> 73 us (80 with the
+// conversion on the integer pipe too, 95 without the loads ahead): FP64 pipe 64 %, issue 56 % at 16
+// warps a multiprocessor.
 struct FixOp {
   unsigned wh[3], wl[3];  // 1/h^2 per axis times 2^k, its parts above and below 2^31
   int k;
