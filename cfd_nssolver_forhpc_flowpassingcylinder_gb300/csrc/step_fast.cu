@@ -343,7 +343,7 @@ __device__ __noinline__ DfibFace dfib_face(double T2, double en, double ec, doub
 }
 
 template <bool UNI>
-__global__ void __launch_bounds__(kBlock) k_update_uf_fast(
+__global__ void __launch_bounds__(kBlock, 4) k_update_uf_fast(
     Geo g, double dt_arg, const double *dtp, int step_mode, double lz, const double *__restrict__ eta,
     const double *__restrict__ p, const double *__restrict__ us, const double *__restrict__ vs,
     const double *__restrict__ ws, double *__restrict__ u3, double *__restrict__ v3, double *__restrict__ w3,
@@ -360,14 +360,15 @@ __global__ void __launch_bounds__(kBlock) k_update_uf_fast(
     gz = -(dt * g.rDzs[2]);
   }
   double acc[2] = {0.0, 0.0};
-#pragma unroll 2
   for (long long row = blockIdx.x * (long long)kBlock + threadIdx.x; row < g.ncell;
        row += (long long)gridDim.x * kBlock) {
     int i, j, k;
     row_ijk(g, row, i, j, k);
     const long long ic = pidx(g, i, j, k);
     // every load first, from the cell itself where the face is a boundary one: behind the branches
-    // below they would wait for one another (512x256x64: 170 -> 161 us; floor 89, the FP64 pipe 92)
+    // below they would wait for one another.  Four blocks a multiprocessor (64 registers), so that
+    // the grid's eight are two whole waves.  512x256x64, CUDA events: 177 us, loads first 168, four
+    // blocks 148; the floor is 89, the FP64 pipe's time 92
     const bool fx = i < g.nx - 3, fy = j < g.ny - 3, fz = k < g.nz - 3 + g.pz;
     const long long iX = fx ? ic + g.sx : ic, iY = fy ? ic + g.sy : ic;
     // periodic z: the top face, its upper cell the first one
