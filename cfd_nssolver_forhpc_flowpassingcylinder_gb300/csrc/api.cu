@@ -1516,7 +1516,9 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
     c->use_mg = true;
   }
   if (cfg->solver != CFDGB_RBSOR && !std::getenv("CFDGB_NO_LOOP")) c->loop_blocks = loop64_blocks(c->ncell);
-  if (cfg->solver == CFDGB_CG && cfg->precision == CFDGB_MIXED && !c->use_mg && !std::getenv("CFDGB_NO_LOOP"))
+  // (the switches that choose an FP32 kernel family keep it)
+  if (cfg->solver == CFDGB_CG && cfg->precision == CFDGB_MIXED && !c->use_mg && !std::getenv("CFDGB_NO_LOOP") &&
+      !std::getenv("CFDGB_NO_TMA") && !std::getenv("CFDGB_SCALAR_FP32"))
     c->loop32 = cg32_loop_fits(g, c->spe32, c->nsm);
   if ((rc = dalloc(c, &c->part, std::max(8 * (size_t)std::max(c->nblk, nblk3), loop64_part_doubles())))) return bail(rc);
   if ((rc = dalloc(c, &c->sc, 1)) || (rc = dalloc(c, &c->sc32, 1)) || (rc = dalloc(c, &c->ss, 1))) return bail(rc);
