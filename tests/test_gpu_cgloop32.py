@@ -56,3 +56,19 @@ def test_wait_that_runs_out_ends_the_launch(monkeypatch):
     with cg.Solver(precision="mixed", solver="cg", tol=1e-11, seed=5, amp=1e-3, **kw) as s:
         s.init_fields()
         assert s.step(2)[1].status == 0
+
+
+def test_pipeline_wait_that_runs_out_ends_the_launch(monkeypatch):
+    """The kernels a phase that larger grids take keep their own bounded waits."""
+    monkeypatch.setenv("CFDGB_NO_LOOP", "1")
+    monkeypatch.setenv("CFDGB_TEST_WAIT_FAULT", "1")
+    kw = dict(nx=128, ny=64, nz=16, lx=32.0, ly=16.0, lz=4.0, cx=8.0, cy=8.0)
+    s = cg.Solver(precision="mixed", solver="cg", **kw)
+    monkeypatch.delenv("CFDGB_TEST_WAIT_FAULT")
+    with s:
+        s.init_fields()
+        s.step(1)  # step 1 has no pressure solve
+        with pytest.raises(cg.CfdgbError, match="FP32 stencil pipeline"):
+            s.step(1)
+        s.init_fields()
+        assert [r.status for r in s.step(3)] == [0, 0, 0]
