@@ -63,6 +63,7 @@ enum KId {
   K_PP32, K_MG, K_PV32, K_PS32, K_PT32, K_PXR32, K_MIRROR,
   K_PP64, K_MG64, K_PV64, K_PS64, K_PT64, K_PXR64, K_LOOP64, K_CGLOOP64, K_CGLOOP32, K_COUNT
 };
+const char *const kWaitGaveUp = "Krylov iteration: a bounded wait between blocks gave up";
 const char *const kKernelNames[K_COUNT] = {
     "convection_diffusion", "rhs", "bicg_setup64", "bicg_ap64", "bicg_s64", "bicg_as64", "bicg_xr64",
     "bicg_p64", "bicg_pap32", "bicg_sas32", "bicg_xr32", "residual64", "refine32",
@@ -642,8 +643,9 @@ int run_chunks(cfdgb_ctx *c, bool fp32, SolverScal *out) {
       std::fprintf(stderr, "[cfdgb]     %s it %d relres %.4e\n", fp32 ? "fp32" : "fp64", c->h_sc->iter,
                    c->h_sc->relres);
     if (c->h_sc->fault)
-      return fail(CFDGB_ECUDA, loop_iter(c, fp32) ? "Krylov iteration: a bounded wait between blocks gave up"
-                                                  : "FP32 stencil pipeline: a bounded wait gave up (block stopped early)");
+      return fail(CFDGB_ECUDA, "%s", loop_iter(c, fp32)
+                                         ? kWaitGaveUp
+                                         : "FP32 stencil pipeline: a bounded wait gave up (block stopped early)");
     if (c->h_sc->done) {
       *out = *c->h_sc;
       return 0;
@@ -1856,7 +1858,7 @@ int cfdgb_op_bicgstab(cfdgb_ctx *c, int solver, double tol, int maxit, const dou
   TRY(h2d(c, c->px2, save_2.data(), c->ncell));
   CK(cudaMemcpyAsync(c->sc, &save_sc, sizeof(SolverScal), cudaMemcpyHostToDevice, c->stream));
   TRY(sync(c));
-  if (rc < 0) fail(rc, "bicgstab hit its iteration cap");
+  if (rc < 0) fail(rc, rc == CFDGB_ECUDA ? kWaitGaveUp : "bicgstab hit its iteration cap");
   return rc;
 }
 
@@ -2080,6 +2082,7 @@ int adjoint_solve(cfdgb_ctx *c, const double *rhs, double tol, int *iters) {
     }
     CK(cudaMemcpyAsync(c->h_sc, c->sca, sizeof(SolverScal), cudaMemcpyDeviceToHost, c->stream));
     TRY(sync(c));
+    if (c->h_sc->fault) return fail(CFDGB_ECUDA, "%s", kWaitGaveUp);
     if (c->h_sc->done) {
       *iters = c->h_sc->iter;
       return c->h_sc->status;

@@ -356,9 +356,9 @@ struct SolverScal {
   int snap_iter;             // MIXED BiCGSTAB: the iteration that marked it (or started the sweep)
   int iter, maxit, done, status, timestep, restart;
   int par;                   // FP32: p[par], ap[par] hold the previous iteration's vectors
-  int fault;                 // FP32: a pipeline wait of a stencil kernel gave up (never expected)
-  int test_wait;             // FP32: one-shot test request: the next pipelined launch makes
-                             // one of its waits run out (CFDGB_TEST_WAIT_FAULT; tests only)
+  int fault;                 // a bounded wait of this solve gave up (never expected)
+  int test_wait;             // one-shot test request (CFDGB_TEST_WAIT_FAULT; tests only): the next
+                             // launch that waits makes one of its waits run out
   unsigned cnt[8];           // last-block counters, one per kernel kind
 };
 // status of an FP32 solve that stopped for an FP64 refinement (never returned to callers)

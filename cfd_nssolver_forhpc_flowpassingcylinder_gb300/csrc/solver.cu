@@ -175,6 +175,7 @@ __global__ void __launch_bounds__(kBlock) k_bicg_setup64(Geo g, Stencil<double> 
     sc->iter = 0;
     sc->done = 0;
     sc->status = 0;
+    sc->fault = 0;
     sc->restart = restart;
     sc->relres = 0.0;
   }
@@ -1414,6 +1415,7 @@ __global__ void __launch_bounds__(kBlock) k64cg_setup(Geo g, Stencil<double> st,
     sc->rho = out[1];
     sc->iter = 0;
     sc->status = 0;
+    sc->fault = 0;
     sc->relres = sqrt(out[1]) / sc->norm0;
     sc->done = (sc->relres < sc->tol) ? 1 : 0;
   }
