@@ -1153,6 +1153,7 @@ int run_step_graphs(cfdgb_ctx *c, int n, cfdgb_step_stats *stats, int *worst) {
                        c->stream));
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->stream));
+    bool gave_up = false;
     if (c->h_ring->n != b) return fail(CFDGB_ECUDA, "step graph: %d of %d step records", c->h_ring->n, b);
     for (int q = 0; q < b; ++q) {
       const StepRec &r = c->h_ring->rec[q];
@@ -1177,7 +1178,9 @@ int run_step_graphs(cfdgb_ctx *c, int n, cfdgb_step_stats *stats, int *worst) {
         st.time = r.time;
       }
       if (status < *worst) *worst = status;
+      gave_up = gave_up || status == CFDGB_ECUDA;
     }
+    if (gave_up) return fail(CFDGB_ECUDA, "%s", kWaitGaveUp);
     done += b;
   }
   return 0;
@@ -2253,6 +2256,7 @@ int cfdgb_backward(cfdgb_ctx *c, double *dJ_dinlet, double *dJ_deta) {
         launch_remove_mean(c->stream, c->nblk, c->g, c->lx, c->part, c->ss, true);
         int it = 0;
         const int rc = adjoint_solve(c, c->lx, c->cfg.tol, &it);
+        if (rc == CFDGB_ECUDA) return rc;
         if (rc < worst) worst = rc;
         launch_remove_mean(c->stream, c->nblk, c->g, c->ka.x, c->part, c->ss, false);
         launch_adj_rhs(c->stream, c->nblk, c->g, dt, c->ka.x, c->lus[0], c->lus[1], c->lus[2], c->lB[0], c->lB[1],

@@ -31,3 +31,13 @@ def test_the_next_solve_starts_clean(monkeypatch, solver):
             s.step(1)
         assert e.value.status == cg.ECUDA
         assert [r.status for r in s.step(2)] == [0, 0]
+
+
+@pytest.mark.parametrize("solver", ["jacobi", "cg"])
+@pytest.mark.parametrize("graph", [True, False])
+def test_capped_steps_of_the_same_call_do_not_hide_it(monkeypatch, solver, graph):
+    """Callers accept CFDGB_ENOCONV, the lower status: the call must still end with CFDGB_ECUDA."""
+    with started(monkeypatch, "1", graph, solver=solver, tol=1e-13, maxit=5) as s:
+        with pytest.raises(cg.CfdgbError, match="bounded wait between blocks") as e:
+            s.step(4, allow_noconv=True)
+        assert e.value.status == cg.ECUDA
