@@ -138,10 +138,10 @@ struct cfdgb_ctx {
   bool loop32 = false;  // FP32 CG sweeps in one launch a chunk (cg32_loop_fits)
   int loop_blocks = 0;  // blocks of the one-launch FP64 iterations (loop64_blocks); 0: a kernel a phase
   double omega = 0.0;  // SOR relaxation in use (cfg.omega, or the optimal one when that is 0)
-  // test switch (environment CFDGB_TEST_WAIT_FAULT at create): the next MIXED solve makes one
-  // bounded wait of the FP32 bulk-copy pipeline run out, the next FP64 one a wait between the
-  // blocks of its one-launch iterations, to exercise that failure path
-  bool test_wait_fault = false;
+  // test switch (environment CFDGB_TEST_WAIT_FAULT at create, 1 or 2): the next MIXED solve makes
+  // one bounded wait of the FP32 bulk-copy pipeline run out, the next FP64 one a wait between the
+  // blocks of its one-launch iterations (2: in the last block only), to exercise that failure path
+  int test_wait_fault = 0;
   // one CUDA graph per time step (FP64 Krylov solvers, after the first step, kernel timing
   // off): the whole step with its convergence loop as a conditional WHILE node; each step
   // appends its scalars to a device ring read back once per cfdgb_step call
@@ -606,9 +606,9 @@ int set_solver_params(cfdgb_ctx *c, SolverScal *dsc, double tol, int maxit) {
 // the test switch (one shot): the next launch that waits on dsc makes a bounded wait run out
 int request_test_wait(cfdgb_ctx *c, SolverScal *dsc) {
   if (!c->test_wait_fault) return 0;
-  static const int one = 1;
-  CK(cudaMemcpyAsync(&dsc->test_wait, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  c->test_wait_fault = false;
+  const int request = c->test_wait_fault;
+  CK(cudaMemcpyAsync(&dsc->test_wait, &request, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  c->test_wait_fault = 0;
   return 0;
 }
 
@@ -1302,7 +1302,7 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
   c->nblk = (int)std::min<long long>((c->ncell + kBlock - 1) / kBlock, (long long)c->nsm * 8);
   c->chunk_len = c->ncell > (1LL << 22) ? 8 : 32;
   c->omega = cfg->omega > 0.0 ? cfg->omega : sor_omega_opt(cfg);
-  c->test_wait_fault = std::getenv("CFDGB_TEST_WAIT_FAULT") != nullptr;
+  if (const char *t = std::getenv("CFDGB_TEST_WAIT_FAULT")) c->test_wait_fault = std::atoi(t) == 2 ? 2 : 1;
   c->no_step_graph = std::getenv("CFDGB_NO_STEP_GRAPH") != nullptr;
   int rc = 0;
   const int nmet = nx + ny + nz;

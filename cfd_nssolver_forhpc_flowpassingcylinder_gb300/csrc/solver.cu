@@ -1644,8 +1644,8 @@ __global__ void __launch_bounds__(kBlock) k32cg_xr(Geo g, Vec32 v, double *part,
 // 131 K 31.1 -> 21.3, 1.05 M 75.9 -> 65.1 (the FP64 pipe's time is 41.7), 2.1 M 131.8 -> 120.3,
 // stretched 1.6 M 117.6 -> 94.7; CG 8 K 12.6 -> 8.4, 314 K 24.7 -> 17.1.
 // The barrier counts arrivals (sc->cnt[6], back to zero through sc->cnt[7] when the last block
-// leaves).  A wait is bounded: one that gives up sets sc->fault and CFDGB_ECUDA, the block
-// leaves, and so do the others, each after its own bounded wait.  (Polling all blocks' sums,
+// leaves).  A wait is bounded: one that gives up sets sc->fault, the block leaves, and so do the
+// others, each after its own bounded wait; the last one out turns the fault into CFDGB_ECUDA.  (Polling all blocks' sums,
 // each word tagged with the reduction's number, instead of the counter: 152 x 152 polled words
 // slow the stores they wait for, 96x48x4 12.7 -> 23.7 us an iteration: not kept.)
 constexpr int kLoopBlock = 512;
@@ -1663,6 +1663,12 @@ struct LoopGrid {
   double *part;     // [slot][kLoopMaxBlocks]
   unsigned target;  // arrivals that complete the next barrier
   long long limit;  // cycles a wait may take
+  bool late;        // test request 2, in block 0: leave after another block's wait has run out
+  __device__ __forceinline__ void hold() const {
+    const long long t0 = clock64();
+    while (atomicAdd(&sc->fault, 0) == 0 && clock64() - t0 < 8 * limit) {
+    }
+  }
   // one thread: this block's arrival, and the wait for all (the block's stores come before, by the
   // barrier that its threads passed)
   __device__ __forceinline__ void arrive_wait(LoopScal &L) {
@@ -1731,11 +1737,13 @@ struct LoopGrid {
   }
 };
 
-// The test request (sc->test_wait, set only by the host's test switch): block 0 waits for one
-// arrival that never comes, every block with a short limit, so that the waits run out
+// The test requests (sc->test_wait, set only by the host's test switch), every block with a short
+// limit: 1, block 0 waits for one arrival too many, which runs out at the chunk's last barrier; 2,
+// the last block does, and block 0, whose waits all end, leaves after that
 __device__ __forceinline__ LoopGrid loop_grid(SolverScal *sc, double *part) {
   const int test = sc->test_wait;
-  return LoopGrid{sc, part, test && blockIdx.x == 0 ? 1u : 0u, test ? kTestWaitCycles : kLoopWaitCycles};
+  const unsigned one = test && blockIdx.x == (test == 2 ? gridDim.x - 1 : 0u) ? 1u : 0u;
+  return LoopGrid{sc, part, one, test ? kTestWaitCycles : kLoopWaitCycles, test == 2 && blockIdx.x == 0};
 }
 // scalars in, and out by block 0 when every block has left the loop's last barrier
 __device__ __forceinline__ void loop_begin(LoopScal &L, const SolverScal *sc) {
@@ -1761,10 +1769,8 @@ __device__ __forceinline__ void loop_end(const LoopScal &L, const LoopGrid &G) {
   if (threadIdx.x != 0) return;
   if (L.bad) {
     atomicExch(&sc->fault, 1);
-    sc->status = CFDGB_ECUDA;
-    sc->done = 1;
-    sc->test_wait = 0;
   } else if (blockIdx.x == 0) {
+    if (G.late) G.hold();
     sc->rho = L.rho;
     sc->alpha = L.alpha;
     sc->omega = L.omega;
@@ -1779,6 +1785,12 @@ __device__ __forceinline__ void loop_end(const LoopScal &L, const LoopGrid &G) {
   }
   __threadfence();
   if (atomicAdd(&sc->cnt[7], 1u) == gridDim.x - 1) {  // every block is past its last wait
+    __threadfence();
+    if (atomicAdd(&sc->fault, 0)) {  // over what block 0 left: its own waits may all have ended
+      sc->status = CFDGB_ECUDA;
+      sc->done = 1;
+      sc->test_wait = 0;
+    }
     sc->cnt[6] = 0u;
     sc->cnt[7] = 0u;
   }
