@@ -111,6 +111,7 @@ EXPORTS = {
     "cfdgb_op_bc_copy": (C.c_int, [C.c_void_p] + [_dp] * 6),
     "cfdgb_op_rhs": (C.c_int, [C.c_void_p, C.c_int] + [_dp] * 4),
     "cfdgb_op_spmv": (C.c_int, [C.c_void_p, C.c_int, _dp, _dp]),
+    "cfdgb_op_residual": (C.c_int, [C.c_void_p, _dp, _dp, _dp]),
     "cfdgb_op_bicgstab": (C.c_int, [C.c_void_p, C.c_int, C.c_double, C.c_int, _dp, _dp,
                                     C.POINTER(C.c_int), _dp]),
     "cfdgb_op_update_uf": (C.c_int, [C.c_void_p] + [_dp] * 11),
@@ -353,6 +354,13 @@ class Solver:
         y = np.zeros(self.cells)
         _check(self._L.cfdgb_op_spmv(self._h, int(jacobi), _ptr(np.ascontiguousarray(x, dtype=np.float64)), _ptr(y)))
         return y
+
+    def residual(self, b, x):
+        """MIXED: b - A x as the refinement forms it (rounded to FP32 there)."""
+        r = np.zeros(self.cells)
+        _check(self._L.cfdgb_op_residual(self._h, _ptr(np.ascontiguousarray(b, dtype=np.float64)),
+                                         _ptr(np.ascontiguousarray(x, dtype=np.float64)), _ptr(r)))
+        return r
 
     def bicgstab(self, rhs, x, tol, maxit=5000, jacobi=False):
         it, rr = C.c_int(), C.c_double()

@@ -1811,6 +1811,23 @@ int cfdgb_op_spmv(cfdgb_ctx *c, int jacobi, const double *x, double *y) {
   return sync(c);
 }
 
+int cfdgb_op_residual(cfdgb_ctx *c, const double *b, const double *x, double *r) {
+  if (!c || !b || !x || !r) return fail(CFDGB_EINVAL, "null argument");
+  if (c->cfg.precision != CFDGB_MIXED) return fail(CFDGB_EINVAL, "op_residual needs a MIXED context");
+  TRY(ensure_op_buffers(c));
+  TRY(h2d(c, c->opc[0], b, c->ncell));
+  TRY(h2d(c, c->opc[1], x, c->ncell));
+  const bool jac = c->cfg.solver == CFDGB_BICGSTAB_JACOBI;
+  // rf and the residual scalars are each solve's own
+  launch_residual64(c->stream, c->nsm, c->g, jac ? c->jac64 : c->spe64, jac ? c->jac32 : c->spe32, jac ? 1 : 0,
+                    c->opc[0], c->opc[1], c->rf, c->part, c->ss, c->sc32, 1, c->in_adjoint);
+  std::vector<float> rf(c->ncell);
+  CK(cudaMemcpyAsync(rf.data(), c->rf, rf.size() * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
+  TRY(sync(c));
+  for (size_t q = 0; q < rf.size(); ++q) r[q] = rf[q];
+  return 0;
+}
+
 int cfdgb_op_bicgstab(cfdgb_ctx *c, int solver, double tol, int maxit, const double *rhs, double *x, int *iters,
                       double *relres) {
   if (!c || !rhs || !x) return fail(CFDGB_EINVAL, "null argument");

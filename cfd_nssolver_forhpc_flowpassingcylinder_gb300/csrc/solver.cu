@@ -2479,7 +2479,7 @@ __global__ void __launch_bounds__(kBlock) k_residual64(Geo g, Stencil<double> st
 // taken in units of 2^-60 of the power of two above the largest |x| (xexp, the largest exponent
 // field, from the kernel that last wrote x, or k_xexp), so a row's differences x_c - x_nb are
 // exact integers; the row is jp sum_a w_a (2 x_c - x_l - x_r) with w_a = 1/h_a^2 a 60-bit integer
-// (29 and 31 bits, so that the products' high parts are nine wide multiply-adds), converted once
+// (30 and 30 bits: the products are twelve wide multiply-adds), converted once
 // and subtracted from b in FP64.  Its error is below 2^-54 of w |x|_max, against the FMA chain's
 // rounded entries, products and sums of 2^-53 each (root mean square against 80-bit on a
 // solution of 128x64x16: 1.2e-15 against 1.25e-14).  All relative to the largest |x|: where x spans
@@ -2491,7 +2491,7 @@ __global__ void __launch_bounds__(kBlock) k_residual64(Geo g, Stencil<double> st
 // conversion on the integer pipe too, 95 without the loads ahead): FP64 pipe 64 %, issue 56 % at 16
 // warps a multiprocessor.
 struct FixOp {
-  unsigned wh[3], wl[3];  // 1/h^2 per axis times 2^k, its parts above and below 2^31
+  unsigned wh[3], wl[3];  // 1/h^2 per axis times 2^k, its parts above and below 2^30
   int k;
   float dg[27];           // the unscaled diagonal per class, rounded to FP32
 };
@@ -2505,18 +2505,24 @@ __global__ void __launch_bounds__(kBlock) k_xexp(Geo g, const double *__restrict
   block_max_exp(m, ss);
 }
 
-// sum_a w_a s_a in units of 2^63 (three units at most are lost)
+// sum_a w_a s_a in units of 2^62, rounded to nearest (|s_a| <= 2^62, w_a < 2^60).  All four partial
+// products a pair (a 2^62 + b 2^32 + c 2^30 + d; three of each fit 64 bits) and one rounding: with the
+// lowest left out and the others truncated the sum lost up to five units, all of one sign.
 __device__ __forceinline__ long long fix_dot(const FixOp &F, long long sx, long long sy, long long sz) {
   const int hx = (int)(sx >> 32), hy = (int)(sy >> 32), hz = (int)(sz >> 32);
+  const unsigned lx = (unsigned)sx, ly = (unsigned)sy, lz = (unsigned)sz;
   long long a = (long long)hx * (int)F.wh[0], b = (long long)hx * (int)F.wl[0];
-  unsigned long long c = (unsigned long long)(unsigned)sx * F.wh[0];
+  unsigned long long c = (unsigned long long)lx * F.wh[0], d = (unsigned long long)lx * F.wl[0];
   a += (long long)hy * (int)F.wh[1];
   b += (long long)hy * (int)F.wl[1];
-  c += (unsigned long long)(unsigned)sy * F.wh[1];
+  c += (unsigned long long)ly * F.wh[1];
+  d += (unsigned long long)ly * F.wl[1];
   a += (long long)hz * (int)F.wh[2];
   b += (long long)hz * (int)F.wl[2];
-  c += (unsigned long long)(unsigned)sz * F.wh[2];
-  return a + (b >> 31) + (long long)(c >> 32);
+  c += (unsigned long long)lz * F.wh[2];
+  d += (unsigned long long)lz * F.wl[2];
+  c += (d >> 30) + ((unsigned long long)((unsigned)b & 0x3fffffffu) << 2) + 0x80000000ULL;
+  return a + (b >> 30) + (long long)(c >> 32);
 }
 
 template <bool FIRST>
@@ -2536,7 +2542,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_residual_fx(Geo g, Stencil<double
   const bool zl = kc > 0 || g.pz, zr = kc + 2 < nz || g.pz;  // cells left and right of the pair exist
   const bool sl = whole || lane > 0, sr = whole || (lane + 1 < W && kc + 2 < nz);  // and come by shuffle
   const int wl = kc > 0 ? -1 : nz - 1, wr = kc + 2 < nz ? 2 : 2 - nz;
-  const int shift = 63 - F.k - 1082 + em;
+  const int shift = 62 - F.k - 1082 + em;
   // classes of the four cells, less the plane's part
   const int cy0 = 3 * axis_class(jc, g.nyc), cy1 = 3 * axis_class(jc + 1, g.nyc);
   const int cz0 = g.pz ? 1 : axis_class(kc, nz), cz1 = g.pz ? 1 : axis_class(kc + 1, nz);
@@ -3139,8 +3145,8 @@ static FixOp fix_op(const Geo &g, const Stencil<float> &st32) {
   F.k = 59 - std::ilogb(top);
   for (int a = 0; a < 3; ++a) {
     const long long q = std::llround(std::ldexp(w[a], F.k));
-    F.wh[a] = (unsigned)(q >> 31);
-    F.wl[a] = (unsigned)(q & 0x7fffffff);
+    F.wh[a] = (unsigned)(q >> 30);
+    F.wl[a] = (unsigned)(q & 0x3fffffff);
   }
   for (int q = 0; q < 27; ++q) F.dg[q] = st32.dg[q];
   return F;

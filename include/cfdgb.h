@@ -313,6 +313,9 @@ int cfdgb_op_rhs(cfdgb_ctx *ctx, int jacobi, const double *us, const double *vs,
 /* SPE_matrix::multiply_omp (inc/matrix/SPE_sparseMatrix.hpp:92) or, jacobi != 0, the
  * scaled CSR_matrix::multiply_omp (inc/matrix/CSR_sparseMatrix.hpp:232); compact x, y. */
 int cfdgb_op_spmv(cfdgb_ctx *ctx, int jacobi, const double *x, double *y);
+/* MIXED contexts: the FP64 residual r = b - A x of the refinement as a step forms it (the rows of
+ * the context's solver; compact b, x), stored rounded to FP32 and returned widened. */
+int cfdgb_op_residual(cfdgb_ctx *ctx, const double *b, const double *x, double *r);
 /* bicgstabRe2::solve (inc/solver/bicgstabRe2.hpp:84) on compact rhs, x (x in: warm
  * start, out: solution).  solver: CFDGB_BICGSTAB or CFDGB_BICGSTAB_JACOBI (rhs must then
  * already be scaled, as createBMatrix_omp does). */
