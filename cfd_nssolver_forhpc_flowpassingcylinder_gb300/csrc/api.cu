@@ -765,7 +765,7 @@ int solve_mixed(cfdgb_ctx *c, double tol, int *iters, int *outer, double *relres
   static const bool trace = std::getenv("CFDGB_TRACE") != nullptr;
   const int jacf = jac ? 1 : 0;
   auto residual = [&](int flags, double *rel) -> int {
-    L(c, K_RESID64, residual64_launches(c->g, flags, c->in_adjoint), [&] {
+    L(c, K_RESID64, 1, [&] {
       launch_residual64(c->stream, c->nsm, c->g, st64, jac ? c->jac32 : c->spe32, jacf, c->b, c->x, c->rf,
                         c->part, c->ss, c->sc32, flags, c->in_adjoint);
     });

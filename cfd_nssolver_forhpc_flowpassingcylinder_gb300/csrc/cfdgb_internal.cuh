@@ -387,8 +387,7 @@ struct StepScal {
   double oflux;    // convective outflow: the outlet correction (net boundary flux / outlet area)
   int hist;        // Adams-Bashforth: increments stored by the steps since init (at most 2)
   int hslot;       // Adams-Bashforth order 3: the history slot that holds the last increment
-  int nan_flag;
-  unsigned xexp;   // MIXED: the largest exponent field of the solution x (k_residual_fx), 0: unknown
+  int nan_flag, pad;
   unsigned cnt[10];
 };
 

@@ -141,10 +141,8 @@ void launch_bicg_nan_reset(cudaStream_t s, int nblk, const Geo &g, double *x, co
                            const double *px2, double *part, SolverScal *sc);
 
 // MIXED refinement pieces: FP64 residual, stored rounded to FP32 in rf (flags: 1 = a solve's
-// first, also ||b||, 2 = also the sweep scale; chain: the FMA-chain kernel on every grid;
-// residual64_launches kernels) and the start of an FP32 sweep on it (first: also the solve's
-// set-up)
-int residual64_launches(const Geo &g, int flags, bool chain);
+// first, also ||b||, 2 = also the sweep scale; chain: the FMA-chain kernel on every grid) and the
+// start of an FP32 sweep on it (first: also the solve's set-up)
 void launch_residual64(cudaStream_t s, int nsm, const Geo &g, const Stencil<double> &st, const Stencil<float> &st32,
                        int jacobi, const double *b, const double *x, float *rf, double *part, StepScal *ss,
                        SolverScal *inner, int flags, bool chain);
@@ -154,7 +152,8 @@ void launch_refine_start32(cudaStream_t s, const Geo &g, const Stencil<double> &
 void launch_sum32(cudaStream_t s, const Geo &g, const float *e, double *part, StepScal *ss);
 // x += factor (e - mean e), the mean taken from the preceding launch_sum32; factor = +-2^k
 // (sweep_scale)
-void launch_correct64(cudaStream_t s, int nblk, const Geo &g, double *x, const float *e, double factor, StepScal *ss);
+void launch_correct64(cudaStream_t s, int nblk, const Geo &g, double *x, const float *e, double factor,
+                      const StepScal *ss);
 
 // adjoint.cu (discrete adjoint of the FP64 step)
 void launch_adj_bc(cudaStream_t s, const Geo &g, double *lu, double *lv, double *lw, double *linlet);

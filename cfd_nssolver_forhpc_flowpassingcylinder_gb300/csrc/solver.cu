@@ -2424,19 +2424,6 @@ __global__ void __launch_bounds__(kBlock) k_nan_restore(Geo g, double *x, const 
 // well: the FP32 vectors and stencil are the limit), while short restarted sweeps
 // converge to the FP64 tolerance.
 
-// the largest exponent field of the block's values into ss->xexp
-__device__ __forceinline__ void block_max_exp(unsigned m, StepScal *ss) {
-  __shared__ unsigned sh[32];
-  const int t = lin_tid(), nw = (int)(blockDim.x * blockDim.y * blockDim.z) >> 5;
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((t & 31) == 0) sh[t >> 5] = m;
-  __syncthreads();
-  if (t < 32) {
-    m = __reduce_max_sync(0xffffffffu, t < nw ? sh[t] : 0u);
-    if (t == 0) atomicMax(&ss->xexp, m);
-  }
-}
-
 // r = b - A x in FP64, stored rounded to FP32 (rf); ||r||, ||b|| (flags & 1) and the sweep
 // scale (flags & 2): the power of two at or below ||r||, so that scaling by it, here and in
 // k_correct64, is exact.  jacobi: st holds the jp-scaled rows (st.c[.][7] = jp), whose
@@ -2475,35 +2462,28 @@ __global__ void __launch_bounds__(kBlock) k_residual64(Geo g, Stencil<double> st
 }
 
 // The same residual on a uniform grid with an even nz, formed from 64-bit integers: at 1/32 of
-// the integer pipes' rate the seven FP64 FMAs of a row cost six times its memory traffic.  x is
-// taken in units of 2^-60 of the power of two above the largest |x| (xexp, the largest exponent
-// field, from the kernel that last wrote x, or k_xexp), so a row's differences x_c - x_nb are
-// exact integers; the row is jp sum_a w_a (2 x_c - x_l - x_r) with w_a = 1/h_a^2 a 60-bit integer
-// (30 and 30 bits: the products are twelve wide multiply-adds), converted once
-// and subtracted from b in FP64.  Its error is below 2^-54 of w |x|_max, against the FMA chain's
-// rounded entries, products and sums of 2^-53 each (root mean square against 80-bit on a
-// solution of 128x64x16: 1.2e-15 against 1.25e-14).  All relative to the largest |x|: where x spans
-// more than 2^7, small values are rounded at 2^-60 of the largest.  Three FP64-pipe instructions a
-// cell (the conversion, the subtraction and the norm).  A thread owns two rows of a pair of cells
-// along k and marches along x; z neighbours across pairs by shuffles.  Values of x outside the
-// integer form's range (all zero, Inf, NaN, extreme exponents) take the FMA chain.  The next
-// plane's loads are issued before this one's arithmetic.  512x256x64: 164 -> 73 us (80 with the
-// conversion on the integer pipe too, 95 without the loads ahead): FP64 pipe 64 %, issue 56 % at 16
-// warps a multiprocessor.
+// the integer pipes' rate the seven FP64 FMAs of a row cost six times its memory traffic.  A thread
+// owns two rows of a pair of cells along k and marches along x; z neighbours across pairs by
+// shuffles.  It takes the values its four cells need in units of its own, u = 2^(em - 1082) for an
+// exponent field em at or above all of theirs (|x| <= 2^60 u, truncated), so the differences
+// x_c - x_nb are integers; the row is jp sum_a w_a (2 x_c - x_l - x_r) with w_a = 1/h_a^2 a 60-bit
+// integer (30 and 30 bits: the products are twelve wide multiply-adds), converted once and
+// subtracted from b in FP64.  em is kept from plane to plane while it covers the values and
+// the largest |x| in each cell's stencil, m, is at least 2^-kFixSpan of 2^(em - 1023): then u <= 2^-54
+// m, and the error, 4 u w from each of three differences and 4 u w from the sum's rounding, is below
+// 2^-50 w m, the FMA chain's being up to seven roundings of 2^-53 of its partial sums, 12 w m.  (In
+// one unit for the whole grid, taken from its largest |x|, quiet regions kept fewer bits than
+// FP64: 73 us, but errors of 1e10 times that bound where x falls over twelve decades.)  Cells that no such em serves (zeros, Inf, NaN, extreme exponents, a peak beside values
+// 2^-5 of it) take the FMA chain.  Three FP64-pipe instructions a cell (the conversion, the
+// subtraction and the norm).  The next plane's loads are issued before this one's arithmetic.
+// 512x256x64: the FMA chain 164 us, this 95 (236 instructions a cell, issue 55 % at 16 warps a
+// multiprocessor).
+constexpr int kFixSpan = 5;
 struct FixOp {
   unsigned wh[3], wl[3];  // 1/h^2 per axis times 2^k, its parts above and below 2^30
   int k;
   float dg[27];           // the unscaled diagonal per class, rounded to FP32
 };
-
-__global__ void __launch_bounds__(kBlock) k_xexp(Geo g, const double *__restrict__ x, StepScal *ss) {
-  unsigned m = 0;
-  const long long stride = (long long)gridDim.x * kBlock;
-#pragma unroll 4
-  for (long long q = (long long)blockIdx.x * kBlock + threadIdx.x; q < g.ncell; q += stride)
-    m = max(m, ((unsigned)__double2hiint(x[q]) >> 20) & 0x7ffu);
-  block_max_exp(m, ss);
-}
 
 // sum_a w_a s_a in units of 2^62, rounded to nearest (|s_a| <= 2^62, w_a < 2^60).  All four partial
 // products a pair (a 2^62 + b 2^32 + c 2^30 + d; three of each fit 64 bits) and one rounding: with the
@@ -2535,23 +2515,18 @@ __global__ void __launch_bounds__(kBlock, 2) k_residual_fx(Geo g, Stencil<double
   const bool on = kc < nz && jc < g.nyc, on1 = on && jc + 1 < g.nyc;
   const int chunk = (g.nxc + gridDim.z - 1) / gridDim.z;
   const int i0 = min(g.nxc, (int)blockIdx.z * chunk), i1 = min(g.nxc, i0 + chunk);
-  const int em = (int)ss->xexp;
-  const bool fix = em >= 200 && em <= 1900;
   const int nyz = g.nyc * nz;
   const bool whole = nz == 2 * W;                      // a row is one segment of lanes
   const bool zl = kc > 0 || g.pz, zr = kc + 2 < nz || g.pz;  // cells left and right of the pair exist
   const bool sl = whole || lane > 0, sr = whole || (lane + 1 < W && kc + 2 < nz);  // and come by shuffle
   const int wl = kc > 0 ? -1 : nz - 1, wr = kc + 2 < nz ? 2 : 2 - nz;
-  const int shift = 62 - F.k - 1082 + em;
   // classes of the four cells, less the plane's part
   const int cy0 = 3 * axis_class(jc, g.nyc), cy1 = 3 * axis_class(jc + 1, g.nyc);
   const int cz0 = g.pz ? 1 : axis_class(kc, nz), cz1 = g.pz ? 1 : axis_class(kc + 1, nz);
   double acc[3] = {0.0, 0.0, 0.0};
   float ns = 0.0f;
-  // a row's pair: residuals from A x (y0, y1), stored
-  auto finish = [&](long long row, int c0, int c1, double y0, double y1, double2 bb) {
-    const double r0 = jacobi ? fma(-st.c[c0][7], y0, bb.x) : bb.x - y0;
-    const double r1 = jacobi ? fma(-st.c[c1][7], y1, bb.y) : bb.y - y1;
+  // a row's pair of residuals, stored; and from A x (y0, y1)
+  auto put = [&](long long row, int c0, int c1, double r0, double r1, double2 bb) {
     const float f0 = d2f_int(r0), f1 = d2f_int(r1);
     *reinterpret_cast<float2 *>(rf + row) = make_float2(f0, f1);
     acc[0] = fma(r0, r0, acc[0]);
@@ -2563,109 +2538,126 @@ __global__ void __launch_bounds__(kBlock, 2) k_residual_fx(Geo g, Stencil<double
     // the unscaled residual's sum: its component along the operator's null space
     ns += jacobi ? fmaf(f0, F.dg[c0], f1 * F.dg[c1]) : f0 + f1;
   };
+  auto finish = [&](long long row, int c0, int c1, double y0, double y1, double2 bb) {
+    put(row, c0, c1, jacobi ? fma(-st.c[c0][7], y0, bb.x) : bb.x - y0,
+        jacobi ? fma(-st.c[c1][7], y1, bb.y) : bb.y - y1, bb);
+  };
   long long row = ((long long)i0 * g.nyc + jc) * nz + kc;
-  if (fix) {  // the same for the whole grid
-    struct Pair {
-      long long a, b;
-    };
-    auto load = [&](long long r) {
-      const double2 v = *reinterpret_cast<const double2 *>(x + r);
-      return Pair{d2fix(v.x, em), d2fix(v.y, em)};
-    };
-    Pair c0{0, 0}, c1{0, 0}, dm0{0, 0}, dm1{0, 0};  // the two rows' cells, and their differences to the plane before
-    // the loads a plane needs, issued a plane ahead: both rows of the next plane, the rows below
-    // and above, b of both rows
-    double2 np0, np1, nlo, nhi, nb0, nb1;
-    np0 = np1 = nlo = nhi = nb0 = nb1 = make_double2(0.0, 0.0);
-    auto ahead = [&](int ic, long long r) {
-      if (!on || ic >= i1) return;
-      nb0 = *reinterpret_cast<const double2 *>(b + r);
-      if (on1) nb1 = *reinterpret_cast<const double2 *>(b + r + nz);
-      if (ic + 1 < g.nxc) {
-        np0 = *reinterpret_cast<const double2 *>(x + r + nyz);
-        if (on1) np1 = *reinterpret_cast<const double2 *>(x + r + nz + nyz);
-      }
-      if (jc > 0) nlo = *reinterpret_cast<const double2 *>(x + r - nz);
-      if (jc + 2 < g.nyc) nhi = *reinterpret_cast<const double2 *>(x + r + 2 * nz);
-    };
-    auto fix = [&](double2 v) { return Pair{d2fix(v.x, em), d2fix(v.y, em)}; };
-    ahead(i0, row);
-    if (on && i0 < i1) {
-      c0 = load(row);
-      c1 = on1 ? load(row + nz) : c0;
-      if (i0 > 0) {
-        const Pair m0 = load(row - nyz), m1 = on1 ? load(row + nz - nyz) : m0;
-        dm0 = Pair{c0.a - m0.a, c0.b - m0.b};
-        dm1 = Pair{c1.a - m1.a, c1.b - m1.b};
-      }
+  struct Pair {
+    long long a, b;
+  };
+  auto size = [](double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; };  // ordered as |v|
+  auto largest = [&](double2 p, double2 q) { return max(max(size(p.x), size(p.y)), max(size(q.x), size(q.y))); };
+  double2 x0, x1;                                // the two rows' cells
+  Pair c0{0, 0}, c1{0, 0}, dm0{0, 0}, dm1{0, 0};  // in units of em, and their differences to the plane before
+  int em = 0;                                    // 0: none
+  // the loads a plane needs, issued a plane ahead: both rows of the next plane, the rows below
+  // and above, b of both rows
+  double2 np0, np1, nlo, nhi, nb0, nb1;
+  x0 = x1 = np0 = np1 = nlo = nhi = nb0 = nb1 = make_double2(0.0, 0.0);
+  auto ahead = [&](int ic, long long r) {
+    if (!on || ic >= i1) return;
+    nb0 = *reinterpret_cast<const double2 *>(b + r);
+    if (on1) nb1 = *reinterpret_cast<const double2 *>(b + r + nz);
+    if (ic + 1 < g.nxc) {
+      np0 = *reinterpret_cast<const double2 *>(x + r + nyz);
+      if (on1) np1 = *reinterpret_cast<const double2 *>(x + r + nz + nyz);
     }
-    for (int ic = i0; ic < i1; ++ic, row += nyz) {
-      Pair p0 = c0, p1 = c1, lo = c0, hi = c1;  // next plane; rows below and above: a missing one has no difference
-      const double2 b0 = nb0, b1 = nb1;
-      if (on) {
-        if (ic + 1 < g.nxc) {
-          p0 = fix(np0);
-          if (on1) p1 = fix(np1);
-        }
-        if (jc > 0) lo = fix(nlo);
-        if (jc + 2 < g.nyc) hi = fix(nhi);
+    if (jc > 0) nlo = *reinterpret_cast<const double2 *>(x + r - nz);
+    if (jc + 2 < g.nyc) nhi = *reinterpret_cast<const double2 *>(x + r + 2 * nz);
+  };
+  auto fix = [&](double2 v) { return Pair{d2fix(v.x, em), d2fix(v.y, em)}; };
+  ahead(i0, row);
+  if (on && i0 < i1) {
+    x0 = *reinterpret_cast<const double2 *>(x + row);
+    x1 = on1 ? *reinterpret_cast<const double2 *>(x + row + nz) : x0;
+  }
+  for (int ic = i0; ic < i1; ++ic, row += nyz) {
+    double2 q0 = x0, q1 = x1, lo = x0, hi = x1;  // next plane; rows below and above: a missing one has no difference
+    const double2 b0 = nb0, b1 = nb1;
+    if (on) {
+      if (ic + 1 < g.nxc) {
+        q0 = np0;
+        q1 = on1 ? np1 : np0;
       }
-      ahead(ic + 1, row + nyz);
-      const int lf = (lane - 1) & (W - 1), rt = (lane + 1) & (W - 1);
-      long long l0 = __shfl_sync(0xffffffffu, c0.b, lf, W), r0 = __shfl_sync(0xffffffffu, c0.a, rt, W);
-      long long l1 = __shfl_sync(0xffffffffu, c1.b, lf, W), r1 = __shfl_sync(0xffffffffu, c1.a, rt, W);
-      if (on) {
-        if (!zl) {
-          l0 = c0.a;
-          l1 = c1.a;
-        } else if (!sl) {
-          l0 = d2fix(x[row + wl], em);
-          if (on1) l1 = d2fix(x[row + nz + wl], em);
+      if (jc > 0) lo = nlo;
+      if (jc + 2 < g.nyc) hi = nhi;
+    }
+    ahead(ic + 1, row + nyz);
+    const int lf = (lane - 1) & (W - 1), rt = (lane + 1) & (W - 1);
+    double l0 = __shfl_sync(0xffffffffu, x0.y, lf, W), r0 = __shfl_sync(0xffffffffu, x0.x, rt, W);
+    double l1 = __shfl_sync(0xffffffffu, x1.y, lf, W), r1 = __shfl_sync(0xffffffffu, x1.x, rt, W);
+    if (on) {
+      if (!zl) {
+        l0 = x0.x;
+        l1 = x1.x;
+      } else if (!sl) {
+        l0 = x[row + wl];
+        l1 = on1 ? x[row + nz + wl] : l0;
+      }
+      if (!zr) {
+        r0 = x0.y;
+        r1 = x1.y;
+      } else if (!sr) {
+        r0 = x[row + wr];
+        r1 = on1 ? x[row + nz + wr] : r0;
+      }
+      // the largest value, and a lower bound of each cell's: every one of the four stencils holds
+      // three of the four cells, so the second largest of them
+      const unsigned top = max(max(largest(x0, x1), largest(q0, q1)),
+                               max(largest(lo, hi), largest(make_double2(l0, l1), make_double2(r0, r1))));
+      const unsigned sa = size(x0.x), sb = size(x0.y), sc = size(x1.x), sd = size(x1.y);
+      const int least = (int)(max(min(max(sa, sb), max(sc, sd)), max(min(sa, sb), min(sc, sd))) >> 20);
+      if ((int)(top >> 20) > em || least + kFixSpan < em) {  // (rare: the values drift by powers of two)
+        double2 m0 = x0, m1 = x1;
+        if (ic > 0) {
+          m0 = *reinterpret_cast<const double2 *>(x + row - nyz);
+          m1 = on1 ? *reinterpret_cast<const double2 *>(x + row + nz - nyz) : m0;
         }
-        if (!zr) {
-          r0 = c0.b;
-          r1 = c1.b;
-        } else if (!sr) {
-          r0 = d2fix(x[row + wr], em);
-          if (on1) r1 = d2fix(x[row + nz + wr], em);
+        em = (int)(max(top, largest(m0, m1)) >> 20) + 1;  // room for a factor of two
+        if (least + kFixSpan < em) --em;
+        if (least + kFixSpan < em || em < 200 || em > 1900) em = 0;
+        if (em) {
+          c0 = fix(x0);
+          c1 = fix(x1);
+          const Pair f0 = fix(m0), f1 = fix(m1);
+          dm0 = Pair{c0.a - f0.a, c0.b - f0.b};
+          dm1 = Pair{c1.a - f1.a, c1.b - f1.b};
         }
-        const int cx = 9 * axis_class(ic, g.nxc);
+      }
+      const int cx = 9 * axis_class(ic, g.nxc);
+      if (em) {
+        const int shift = 62 - F.k - 1082 + em;
+        const Pair p0 = fix(q0), p1 = fix(q1), lw = fix(lo), up = fix(hi);
         const Pair dp0{p0.a - c0.a, p0.b - c0.b};
         const Pair dy{on1 ? c1.a - c0.a : 0, on1 ? c1.b - c0.b : 0};  // row 1 less row 0
         const long long dz0 = c0.b - c0.a;
-        const double y0 = fix2d(fix_dot(F, dm0.a - dp0.a, (c0.a - lo.a) - dy.a, (c0.a - l0) - dz0), shift);
-        const double y1 = fix2d(fix_dot(F, dm0.b - dp0.b, (c0.b - lo.b) - dy.b, dz0 - (r0 - c0.b)), shift);
+        const double y0 = fix2d(fix_dot(F, dm0.a - dp0.a, (c0.a - lw.a) - dy.a, (c0.a - d2fix(l0, em)) - dz0), shift);
+        const double y1 = fix2d(fix_dot(F, dm0.b - dp0.b, (c0.b - lw.b) - dy.b, dz0 - (d2fix(r0, em) - c0.b)), shift);
         finish(row, cx + cy0 + cz0, cx + cy0 + cz1, y0, y1, b0);
         dm0 = dp0;
         if (on1) {
           const Pair dp1{p1.a - c1.a, p1.b - c1.b};
           const long long dz1 = c1.b - c1.a;
-          const double y2 = fix2d(fix_dot(F, dm1.a - dp1.a, dy.a - (hi.a - c1.a), (c1.a - l1) - dz1), shift);
-          const double y3 = fix2d(fix_dot(F, dm1.b - dp1.b, dy.b - (hi.b - c1.b), dz1 - (r1 - c1.b)), shift);
+          const double y2 = fix2d(fix_dot(F, dm1.a - dp1.a, dy.a - (up.a - c1.a), (c1.a - d2fix(l1, em)) - dz1), shift);
+          const double y3 = fix2d(fix_dot(F, dm1.b - dp1.b, dy.b - (up.b - c1.b), dz1 - (d2fix(r1, em) - c1.b)), shift);
           finish(row + nz, cx + cy1 + cz0, cx + cy1 + cz1, y2, y3, b1);
           dm1 = dp1;
         }
-      }
-      c0 = p0;
-      c1 = p1;
-    }
-  } else if (on) {
-    for (int ic = i0; ic < i1; ++ic, row += nyz)
-      for (int e = 0; e < (on1 ? 2 : 1); ++e) {
-        const long long r = row + (long long)e * nz;
-        const double2 bb = *reinterpret_cast<const double2 *>(b + r);
-        const int c = 9 * axis_class(ic, g.nxc) + (e ? cy1 : cy0);
-        const double q0 = resid_at(g, st, x, ic, jc + e, kc, r, bb.x), q1 = resid_at(g, st, x, ic, jc + e, kc + 1, r + 1, bb.y);
-        const float f0 = d2f_int(q0), f1 = d2f_int(q1);
-        *reinterpret_cast<float2 *>(rf + r) = make_float2(f0, f1);
-        acc[0] = fma(q0, q0, acc[0]);
-        acc[0] = fma(q1, q1, acc[0]);
-        if (FIRST) {
-          acc[1] = fma(bb.x, bb.x, acc[1]);
-          acc[1] = fma(bb.y, bb.y, acc[1]);
+        c0 = p0;
+        c1 = p1;
+      } else {
+        for (int e = 0; e < (on1 ? 2 : 1); ++e) {
+          const long long r = row + (long long)e * nz;
+          const double2 bb = e ? b1 : b0;
+          const int c = cx + (e ? cy1 : cy0);
+          put(r, c + cz0, c + cz1, resid_at(g, st, x, ic, jc + e, kc, r, bb.x),
+              resid_at(g, st, x, ic, jc + e, kc + 1, r + 1, bb.y), bb);
         }
-        ns += jacobi ? fmaf(f0, F.dg[c + cz0], f1 * F.dg[c + cz1]) : f0 + f1;
       }
+    }
+    x0 = q0;
+    x1 = q1;
   }
   acc[2] = f2d_int(ns);
   double out[3];
@@ -2675,7 +2667,6 @@ __global__ void __launch_bounds__(kBlock, 2) k_residual_fx(Geo g, Stencil<double
     ss->relres = ss->rnorm / ss->bnorm;
     ss->rsum = out[2];
     if (flags & 2) inner->scale = sweep_scale(ss->rnorm);
-    ss->xexp = 0;  // of this x only: the next kernel that writes x leaves its own
   }
 }
 
@@ -2768,10 +2759,8 @@ __device__ __forceinline__ double correction(float e, float m, long long shift, 
   return __longlong_as_double((__float_as_uint(f) & 0x7f800000u) == 0u ? 0LL : (d + shift) ^ sign);
 }
 __global__ void __launch_bounds__(kBlock) k_correct64(Geo g, double *__restrict__ x, const float *__restrict__ e,
-                                                       int k, int neg, StepScal *ss) {
+                                                       int k, int neg, const StepScal *ss) {
   const float m = d2f_int(ss->esum / (double)g.ncell);
-  unsigned em = 0;  // the largest exponent field of the new x (k_residual_fx)
-  auto exps = [&](double v) { em = max(em, ((unsigned)__double2hiint(v) >> 20) & 0x7ffu); };
   const long long shift = (long long)k << 52, sign = neg ? (long long)0x8000000000000000ULL : 0LL;
   const long long nq = g.ncell / 4, stride = (long long)gridDim.x * blockDim.x;
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2785,17 +2774,8 @@ __global__ void __launch_bounds__(kBlock) k_correct64(Geo g, double *__restrict_
     b.y += correction(v.w, m, shift, sign);
     xp[0] = a;
     xp[1] = b;
-    exps(a.x);
-    exps(a.y);
-    exps(b.x);
-    exps(b.y);
   }
-  if (t0 < g.ncell - 4 * nq) {
-    const double v = x[4 * nq + t0] + correction(e[4 * nq + t0], m, shift, sign);
-    x[4 * nq + t0] = v;
-    exps(v);
-  }
-  block_max_exp(em, ss);
+  if (t0 < g.ncell - 4 * nq) x[4 * nq + t0] += correction(e[4 * nq + t0], m, shift, sign);
 }
 
 // ---- null-space projection of the right-hand side (project_rhs) ----
@@ -3151,9 +3131,6 @@ static FixOp fix_op(const Geo &g, const Stencil<float> &st32) {
   for (int q = 0; q < 27; ++q) F.dg[q] = st32.dg[q];
   return F;
 }
-int residual64_launches(const Geo &g, int flags, bool chain) {
-  return (flags & 1) && !chain && fix_residual(g) ? 2 : 1;
-}
 void launch_residual64(cudaStream_t s, int nsm, const Geo &g, const Stencil<double> &st, const Stencil<float> &st32,
                        int jacobi, const double *b, const double *x, float *rf, double *part, StepScal *ss,
                        SolverScal *inner, int flags, bool chain) {
@@ -3174,13 +3151,8 @@ void launch_residual64(cudaStream_t s, int nsm, const Geo &g, const Stencil<doub
       best = cost;
       grid.z = nz;
     }
-    if (flags & 1) {  // x as the last solve (or its caller) left it
-      cudaMemsetAsync(&ss->xexp, 0, sizeof(ss->xexp), s);
-      k_xexp<<<g.xgrid, kBlock, 0, s>>>(g, x, ss);
-      k_residual_fx<true><<<grid, block, 0, s>>>(g, st, F, jacobi, b, x, rf, part, ss, inner, flags);
-    } else {
-      k_residual_fx<false><<<grid, block, 0, s>>>(g, st, F, jacobi, b, x, rf, part, ss, inner, flags);
-    }
+    (flags & 1 ? k_residual_fx<true> : k_residual_fx<false>)<<<grid, block, 0, s>>>(g, st, F, jacobi, b, x, rf, part, ss,
+                                                                                    inner, flags);
     return;
   }
   if (flags & 1)
@@ -3197,7 +3169,8 @@ void launch_refine_start32(cudaStream_t s, const Geo &g, const Stencil<double> &
 void launch_sum32(cudaStream_t s, const Geo &g, const float *e, double *part, StepScal *ss) {
   k_sum32<<<g.xgrid, kBlock, 0, s>>>(g, e, part, ss);
 }
-void launch_correct64(cudaStream_t s, int, const Geo &g, double *x, const float *e, double factor, StepScal *ss) {
+void launch_correct64(cudaStream_t s, int, const Geo &g, double *x, const float *e, double factor,
+                      const StepScal *ss) {
   // factor = +-2^k (sweep_scale); a zero factor (a zero residual, never corrected) adds nothing
   if (!(std::fabs(factor) > 0.0) || !std::isfinite(factor)) return;
   k_correct64<<<g.xgrid, kBlock, 0, s>>>(g, x, e, std::ilogb(factor), factor < 0.0 ? 1 : 0, ss);

@@ -11,8 +11,8 @@ import cfd_nssolver_forhpc_flowpassingcylinder_gb300 as cg
 pytestmark = pytest.mark.gpu
 
 
-def exact_ax(x, h):
-    """Zero-gradient rows of -div grad on compact x: a list of rationals per cell (C order)."""
+def exact_ax(x, h, pz=False):
+    """Rows of -div grad on compact x, zero-gradient or periodic in z: a rational per cell."""
     w = [1 / (Fraction(d) * Fraction(d)) for d in h]
     f = np.array([Fraction(v) for v in x.ravel()], dtype=object).reshape(x.shape)
     y = np.zeros(x.shape, dtype=object) + Fraction(0)
@@ -22,21 +22,43 @@ def exact_ax(x, h):
         lo[a], hi[a] = slice(0, -1), slice(1, None)
         y[tuple(lo)] -= d
         y[tuple(hi)] += d
+    if pz:
+        d = (f[:, :, 0] - f[:, :, -1]) * w[2]
+        y[:, :, 0] += d
+        y[:, :, -1] -= d
     return y
 
 
-def errors(x, h, **kw):
-    """(computed - exact) residual in units of 2^-53 of w max|x| (w: the largest 1/h^2), per cell,
-    and w."""
+def solver(shape, h, **kw):
+    nx, ny, nz = shape
+    return cg.Solver(nx=nx, ny=ny, nz=nz, lx=nx * h[0], ly=ny * h[1], lz=nz * h[2], cx=nx * h[0] / 2,
+                     cy=ny * h[1] / 2, radius=min(h[:2]), precision="mixed", **kw)
+
+
+def errors(x, h, solver_="bicgstab", **kw):
+    """(computed - exact) residual of A x rounded to FP64, per cell, in units of 2^-53 of the largest
+    1/h^2 (Jacobi-scaled rows: unscaled)."""
     nx, ny, nz = x.shape
-    with cg.Solver(nx=nx, ny=ny, nz=nz, lx=nx * h[0], ly=ny * h[1], lz=nz * h[2], cx=nx * h[0] / 2, cy=ny * h[1] / 2,
-                   radius=min(h[:2]), precision="mixed", solver="bicgstab", **kw) as s:
-        ax = exact_ax(x, [s.cfg.lx / nx, s.cfg.ly / ny, s.cfg.lz / nz])
+    with solver(x.shape, h, solver=solver_, **kw) as s:
+        pz = kw.get("bc_z") == "periodic"
+        hh = [s.cfg.lx / nx, s.cfg.ly / ny, s.cfg.lz / nz]
+        ax = exact_ax(x, hh, pz)
+        scale = 1
+        if solver_ == "jacobi":
+            n = [np.full(k, 2) for k in x.shape]
+            for a in range(2 if pz else 3):
+                n[a][0] -= 1
+                n[a][-1] -= 1
+            w3 = [1 / (Fraction(d) * Fraction(d)) for d in hh]
+            scale = np.array([[[n[0][i] * w3[0] + n[1][j] * w3[1] + n[2][k] * w3[2] for k in range(nz)]
+                               for j in range(ny)] for i in range(nx)], dtype=object)
+            ax = ax / scale
         b = np.array([float(v) for v in ax.ravel()])
         got = s.residual(b, x.ravel())
     want = [Fraction(v) - e for v, e in zip(b, ax.ravel())]
     w = max(1.0 / (d * d) for d in h)
-    return np.array([float(Fraction(float(g)) - e) for g, e in zip(got, want)]).reshape(x.shape) / 2.0 ** -53 / w
+    err = np.array([Fraction(float(g)) - e for g, e in zip(got, want)], dtype=object).reshape(x.shape) * scale
+    return err.astype(float) / 2.0 ** -53 / w
 
 
 @pytest.mark.parametrize("shape,h", [((12, 10, 24), (0.3, 0.7, 0.45)), ((9, 7, 66), (0.11, 0.13, 0.17))])
@@ -47,3 +69,53 @@ def test_rounding_is_not_one_sided(shape, h):
     rounding of another number)."""
     e = errors(1.0 + np.random.default_rng(7).random(shape), h).ravel()
     assert abs(e.mean()) <= 5 * e.std() / np.sqrt(e.size), (e.mean(), e.std())
+
+
+def stencil_max(x, pz):
+    """The largest |x| in each cell's stencil."""
+    a = np.abs(x)
+    m = a.copy()
+    for ax in range(3):
+        lo, hi = [slice(None)] * 3, [slice(None)] * 3
+        lo[ax], hi[ax] = slice(0, -1), slice(1, None)
+        m[tuple(lo)] = np.maximum(m[tuple(lo)], a[tuple(hi)])
+        m[tuple(hi)] = np.maximum(m[tuple(hi)], a[tuple(lo)])
+    if pz:
+        m[:, :, 0] = np.maximum(m[:, :, 0], a[:, :, -1])
+        m[:, :, -1] = np.maximum(m[:, :, -1], a[:, :, 0])
+    return m
+
+
+def fields(shape):
+    """Values whose size changes over the grid: decades along each axis, a sign change, a peak of
+    one cell, quiet and zero regions, noise over 2^-40 .. 1."""
+    rng = np.random.default_rng(11)
+    i, j, k = np.meshgrid(*(np.linspace(0.0, 1.0, n) for n in shape), indexing="ij")
+    noise = 1.0 + 0.5 * rng.random(shape)
+    for a in (i, j, k):
+        yield noise * 10.0 ** (-12.0 * a)
+        yield noise * 10.0 ** (-12.0 * (1.0 - a))
+    yield np.sin(7.0 * i) * np.cos(5.0 * j) * np.cos(6.0 * k)
+    x = 1e-3 * noise
+    x[shape[0] // 2, shape[1] // 2, shape[2] // 2] = 1e6
+    yield x
+    x = noise * 1e-9
+    x[:2] = 1.0
+    x[-2:] = 0.0
+    yield x
+    yield rng.standard_normal(shape) * 2.0 ** rng.integers(-40, 1, shape)
+
+
+@pytest.mark.parametrize("solver_", ["bicgstab", "jacobi"])
+@pytest.mark.parametrize("bc_z", ["zero_gradient", "periodic"])
+@pytest.mark.parametrize("shape,h", [((12, 7, 10), (0.3, 0.4, 0.25)), ((5, 6, 66), (0.25, 0.25, 0.5)),
+                                     ((17, 5, 8), (0.2, 0.5, 0.3))])
+def test_every_cell_to_the_rounding_of_its_own_stencil(shape, h, bc_z, solver_):
+    """The FMA chain's error is at most seven roundings of partial sums up to 12 w m, m the largest |x|
+    in the cell's stencil and w the largest 1/h^2, and a few roundings of the entries (the
+    scaled diagonal's largest, twelve units): 100 units of 2^-53 w m.  The integer form's stays
+    below that everywhere, however large x is elsewhere."""
+    pz = bc_z == "periodic"
+    for n, x in enumerate(fields(shape)):
+        e, m = errors(x, h, solver_, bc_z=bc_z), stencil_max(x, pz)
+        assert np.all(np.abs(e) <= 100.0 * m), (n, float((np.abs(e) / np.where(m > 0, m, 1)).max()))
