@@ -3109,22 +3109,25 @@ void launch_bicg_nan_reset(cudaStream_t s, int, const Geo &g, double *x, const d
   k_nan_restore<<<cgrid(g), cblock(g), 0, s>>>(g, x, px2, sc);
 }
 
-// the integer form covers the grid: pairs along k, a plane's and two rows' offsets in 32 bits, and
-// spacings its exponents are safe with
+// the integer form covers the grid: pairs along k, a plane's and two rows' offsets in 32 bits,
+// spacings its exponents are safe with, and none so much wider than another that its weight, in
+// units of the largest one's, keeps fewer than FP64's 53 bits (cells of about 11 : 1)
+static long long fix_weight(double w, int k) { return std::llround(std::ldexp(w, k)); }
+static int fix_exponent(const double (&w)[3]) { return 59 - std::ilogb(std::max(w[0], std::max(w[1], w[2]))); }
 static bool fix_residual(const Geo &g) {
   if (g.nonuni || g.nzc % 2 != 0 || g.nzc < 4 || (long long)g.nyc * g.nzc >= (1LL << 30)) return false;
   for (double h : {g.hx, g.hy, g.hz})
     if (!(h > 1e-9 && h < 1e9)) return false;
-  return true;
+  const double w[3] = {1.0 / (g.hx * g.hx), 1.0 / (g.hy * g.hy), 1.0 / (g.hz * g.hz)};
+  return fix_weight(std::min(w[0], std::min(w[1], w[2])), fix_exponent(w)) >= 1LL << 52;
 }
 // the integer form's operator: w_a times the power of two that brings the largest below 2^60
 static FixOp fix_op(const Geo &g, const Stencil<float> &st32) {
   FixOp F{};
   const double w[3] = {1.0 / (g.hx * g.hx), 1.0 / (g.hy * g.hy), 1.0 / (g.hz * g.hz)};
-  const double top = std::max(w[0], std::max(w[1], w[2]));
-  F.k = 59 - std::ilogb(top);
+  F.k = fix_exponent(w);
   for (int a = 0; a < 3; ++a) {
-    const long long q = std::llround(std::ldexp(w[a], F.k));
+    const long long q = fix_weight(w[a], F.k);
     F.wh[a] = (unsigned)(q >> 30);
     F.wl[a] = (unsigned)(q & 0x3fffffff);
   }

@@ -119,3 +119,51 @@ def test_every_cell_to_the_rounding_of_its_own_stencil(shape, h, bc_z, solver_):
     for n, x in enumerate(fields(shape)):
         e, m = errors(x, h, solver_, bc_z=bc_z), stencil_max(x, pz)
         assert np.all(np.abs(e) <= 100.0 * m), (n, float((np.abs(e) / np.where(m > 0, m, 1)).max()))
+
+
+def chain(x, b, h):
+    """k_residual64's FMA chain on the unscaled zero-gradient rows, each FMA rounded once, stored
+    rounded to FP32."""
+    fma = lambda p, q, r: float(Fraction(p) * Fraction(q) + Fraction(r))
+    n = x.shape
+    c = [1.0 / d / d for d in h]
+    out = np.empty(n)
+    for p in np.ndindex(n):
+        diag = c[0] + c[1] + c[2] + c[0] + c[1] + c[2]
+        for a in range(3):
+            for end in (0, n[a] - 1):
+                if p[a] == end:
+                    diag -= c[a]
+        nb = lambda a, s: x[tuple(p[q] + (s if q == a else 0) for q in range(3))]
+        r = b[p]
+        for a in (0, 1, 2):
+            if p[a] > 0:
+                r = fma(c[a], nb(a, -1), r)
+        r = fma(-diag, x[p], r)
+        for a in (2, 1, 0):
+            if p[a] < n[a] - 1:
+                r = fma(c[a], nb(a, 1), r)
+        out[p] = np.float32(r)
+    return out
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("ratio,integer", [(8.0, True), (16.0, False), (1000.0, False)])
+def test_thin_cells_keep_the_entries_53_bits(ratio, integer, axis):
+    """A spacing R times another has a weight of 59 - 2 log2 R bits at least in the integer form, 53 up to
+    R = 8: wider ones take the FMA chain, whose every bit is checked; the integer form's sums
+    differ from it in most cells."""
+    h = [0.3, 0.3, 0.3]
+    h[axis] *= ratio
+    rng = np.random.default_rng(5)
+    x, b = 1.0 + rng.random((7, 6, 8)), rng.standard_normal((7, 6, 8))
+    with solver(x.shape, h, solver="bicgstab") as s:
+        hh = [s.cfg.lx / 7, s.cfg.ly / 6, s.cfg.lz / 8]
+        got = s.residual(b.ravel(), x.ravel()).reshape(x.shape)
+    # (r itself is large here, and FP32 hides the difference: b again as A x, so that r is what rounding left)
+    with solver(x.shape, h, solver="bicgstab") as s:
+        ax = np.array([float(v) for v in exact_ax(x, hh).ravel()]).reshape(x.shape)
+        tiny = s.residual(ax.ravel(), x.ravel()).reshape(x.shape)
+    np.testing.assert_allclose(got, chain(x, b, hh), rtol=2.0 ** -22, atol=1e-12 / min(hh) ** 2)
+    same = tiny == chain(x, ax, hh)
+    assert np.mean(same) < 0.5 if integer else np.all(same), np.mean(same)
