@@ -2189,6 +2189,7 @@ __global__ void __launch_bounds__(kCgLoopBlock, 1) k32cg_loop(Geo g, Stencil<flo
     }
     __syncthreads();
     float a = 0.0f;
+    double a8 = 0.0;
 #pragma unroll
     for (int u = 0; u < K; ++u) {  // q = A p: stencil_apply_diff's terms in its order
       const int b = V * (tid + kCgLoopBlock * u);
@@ -2215,9 +2216,13 @@ __global__ void __launch_bounds__(kCgLoopBlock, 1) k32cg_loop(Geo g, Stencil<flo
         q[u].v[e] = t;
         a = fmaf(t, fc, a);
       }
+      if (V == 1 && u % 8 == 7) {  // FP32 runs of eight products, as k32cg_pq's (AccF)
+        a8 += (double)a;
+        a = 0.0f;
+      }
     }
     {
-      double d[1] = {(double)a};
+      double d[1] = {a8 + (double)a};
       if (!G.reduce<1>(L, d, 0, [&](const double (&o)[1]) {
             const double al = L.rho / o[0];
             if (threadIdx.x == 0) L.alpha = al;
