@@ -354,6 +354,7 @@ struct SolverScal {
   double snap_rel;           // MIXED BiCGSTAB: relres of the best iterate kept so far
   int snap;                  // MIXED BiCGSTAB: 1 = the current iterate is the new one to keep
   int snap_iter;             // MIXED BiCGSTAB: the iteration that marked it (or started the sweep)
+  int stall;                 // MIXED BiCGSTAB: iterations without one that end the sweep
   int iter, maxit, done, status, timestep, restart;
   int par;                   // FP32: p[par], ap[par] hold the previous iteration's vectors
   int fault;                 // a bounded wait of this solve gave up (never expected)
@@ -363,11 +364,12 @@ struct SolverScal {
 };
 // status of an FP32 solve that stopped for an FP64 refinement (never returned to callers)
 constexpr int kStatusRefine = 1;
-// A MIXED BiCGSTAB sweep that has not halved its residual for this many iterations is given
-// up: the refinement goes on from the iterate it kept, or FP64 finishes where it kept none.
-// Sweeps that converge halve it every few dozen iterations to a few hundred (1024x512x128); one
-// whose FP32 recursion has stalled (the unscaled rows of the stretched grid) would otherwise
-// run to the iteration cap.
+// A MIXED BiCGSTAB sweep that has not halved its residual for this many iterations, or for twice
+// the sum of the grid's extents where that is more, is given up: the refinement goes on from the
+// iterate it kept, or FP64 finishes where it kept none.  Sweeps that converge halve it every few
+// dozen iterations to a few hundred (1024x512x128), and whole ones take up to 1040 iterations on 800
+// cells in a row and 1000 on 3000; one whose FP32 recursion has stalled (the unscaled rows of the
+// stretched grid, of 240 to 440 cells in all three extents) would otherwise run to the iteration cap.
 constexpr int kSweepStall = 1000;
 
 // Per-step scalars (drag, lift, outer residual of the mixed solve)

@@ -245,7 +245,8 @@ __device__ __forceinline__ void finish_iteration(SolverScal *sc, double n2, doub
   const double tol = sc->tol, rho_old = sc->rho, rn = sqrt(n2);
   const double peak_max = sc->rmax, rstart = sc->rstart, delta = sc->delta, peak = sc->peak, best = sc->best,
                snap_rel = sc->snap_rel, thr = sc->restart_thr;
-  const int iter = sc->iter, maxit = sc->maxit, timestep = sc->timestep, snap_iter = sc->snap_iter;
+  const int iter = sc->iter, maxit = sc->maxit, timestep = sc->timestep, snap_iter = sc->snap_iter,
+            stall = sc->stall;
   const double omega = sc->omega;
   double relres, ao, rq;
   div3(rn, sc->norm0, sc->alpha, omega, rr, rho_old, relres, ao, rq);
@@ -282,7 +283,7 @@ __device__ __forceinline__ void finish_iteration(SolverScal *sc, double n2, doub
       sc->done = 1;
       sc->status = kStatusRefine;
       sc->iter = iter + 1;
-    } else if (!snap && iter - snap_iter >= kSweepStall) {
+    } else if (!snap && iter - snap_iter >= stall) {
       sc->done = 1;
       sc->status = CFDGB_ENOCONV;
       sc->iter = iter + 1;
@@ -2727,6 +2728,7 @@ __global__ void __launch_bounds__(kBlock) k_refine_start32(Geo g, Stencil<double
     sc->snap_rel = sc->relres;  // x = 0, kept by the first x update
     sc->snap = 1;
     sc->snap_iter = sc->iter;
+    sc->stall = max(kSweepStall, 2 * (g.nxc + g.nyc + g.nzc));
     sc->done = 0;
     sc->status = 0;
     sc->restart = 1;
