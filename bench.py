@@ -325,13 +325,15 @@ def run_mode(cg, torch, dist, wl, steps, warmup, solver, precision, maxit=5000, 
         return out
 
 
-def e2e_mode(cg, torch, dist, wl, steps, warmup, solver, precision):
+def e2e_mode(cg, torch, dist, wl, steps, warmup, solver, precision, maxit=5000):
     """The public API with HOST buffers: per step, H2D of u,v,w,p from pinned memory,
-    one step, D2H of u,v,w,p; all on the library's stream inside the events."""
+    one step, D2H of u,v,w,p; all on the library's stream inside the events.  Returns the time, the
+    bytes of a direction and step, and the steps' results (a capped solve is reported in its
+    status, as in run_mode)."""
     cfg, wsolver, tol = workload(wl)
-    with cg.Solver(solver=solver or wsolver, precision=precision, tol=tol, **cfg) as s:
+    with cg.Solver(solver=solver or wsolver, precision=precision, tol=tol, maxit=maxit, **cfg) as s:
         s.init_fields()
-        s.step(warmup)
+        s.step(warmup, allow_noconv=True)
         host = {k: torch.empty(s.shape, dtype=torch.float64, pin_memory=True).numpy() for k in "uvwp"}
         s.get_fields(host)
         stream = torch.cuda.ExternalStream(s.stream)
@@ -339,16 +341,35 @@ def e2e_mode(cg, torch, dist, wl, steps, warmup, solver, precision):
         dist.barrier()
         torch.cuda.synchronize()
         e0.record(stream)
+        stats = []
         for _ in range(steps):
             s.set_fields(host["u"], host["v"], host["w"], host["p"])
-            s.step(1)
+            stats += s.step(1, allow_noconv=True)
             s.get_fields(host)
         e1.record(stream)
         torch.cuda.synchronize()
         dist.barrier()
         ms = e0.elapsed_time(e1)
         nbytes = 4 * int(host["u"].nbytes)
-        return ms, nbytes, s.cells
+        return ms, nbytes, stats
+
+
+def e2e_line(cg, torch, dist, wl, steps, warmup, maxit):
+    """The line's e2e entry, with the solves that hit the cap and any that missed the tolerance."""
+    _, _, tol = workload(wl)
+    ms, nbytes, stats = e2e_mode(cg, torch, dist, wl, steps, warmup, None, "fp64", maxit)
+    te = dist.max(ms)
+    out = {"value": cells_of(wl) * steps * dist.world / (te / 1e3), "unit": "cell-steps/s",
+           "h2d_bytes_per_step": nbytes, "d2h_bytes_per_step": nbytes, **solve_counts(stats, tol)}
+    if out["unconverged_solves"]:
+        out["failure"] = unconverged_text(out, steps, tol, maxit)
+    return out
+
+
+def unconverged_text(counts, steps, tol, maxit):
+    """The metric names the tolerance: say plainly that some timed solves missed it."""
+    return (f"{counts['unconverged_solves']} of {steps} timed solves ended at or above "
+            f"relres {tol:g} ({counts['capped_solves']} at the {maxit}-iteration cap)")
 
 
 def adjoint_mode(cg, torch, dist, nsteps, ckpt, wl="c4", first=0, precision="fp64", solver="jacobi",
@@ -846,9 +867,7 @@ def main(argv=None):
         "clocks": clk.summary(), "device_mem_gb": fp64["device_mem_gb"],
     }
     if rec64["unconverged_solves"]:
-        # the metric names the tolerance: say plainly that some timed solves missed it
-        line["failure"] = (f"{rec64['unconverged_solves']} of {args.steps} timed solves ended at or above "
-                           f"relres {tol:g} ({rec64['capped_solves']} at the {args.maxit}-iteration cap)")
+        line["failure"] = unconverged_text(rec64, args.steps, tol, args.maxit)
     results = {"fp64": fp64}
     for key in [m for m in MODES if m in modes]:
         try:
@@ -871,10 +890,10 @@ def main(argv=None):
         except cg.CfdgbError as e:
             line["boundary_set"] = {"error": str(e)}
     if "e2e" in modes:
-        ms, nbytes, _ = e2e_mode(cg, torch, dist, wl, args.steps, args.warmup, None, "fp64")
-        te = dist.max(ms)
-        line["e2e"] = {"value": cells * args.steps * dist.world / (te / 1e3), "unit": "cell-steps/s",
-                       "h2d_bytes_per_step": nbytes, "d2h_bytes_per_step": nbytes}
+        try:
+            line["e2e"] = e2e_line(cg, torch, dist, wl, args.steps, args.warmup, args.maxit)
+        except cg.CfdgbError as e:
+            line["e2e"] = {"value": None, "error": str(e)}
     if "adjoint" in modes:
         try:
             line["adjoint"] = adjoint_mode(cg, torch, dist, args.adj_steps, args.adj_ckpt, args.adj_workload,
