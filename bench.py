@@ -114,11 +114,30 @@ KERNEL_WORDS = {
     "bicgp_p64": 4, "bicgp_v64": 3, "bicgp_s64": 3, "bicgp_t64": 3, "bicgp_xr64": 8,
 }
 
+# The one-launch forms of those iterations: a launch is a chunk of iterations, so words an
+# iteration, those of the kernels above that they replace (the vectors of these grids live in L2, and
+# cg_loop32's on chip, so the algorithmic rate may pass the HBM peak)
+LOOP_WORDS = {"bicg_loop64": 19, "cg_loop64": 11, "cg_loop32": 10}
+
 
 # FP64 flops per interior cell and launch of the FP64 iteration kernels (an FMA counts 2):
 # SpMV 1 mul + 6 FMA, each dot 1 FMA, each axpy-like update 1 FMA per term
 KERNEL_FP64_FLOPS = {"bicg_ap64": 15, "bicg_s64": 2, "bicg_as64": 17, "bicg_xr64": 10, "bicg_p64": 4,
                      "cg_q64": 15, "cg_xr64": 6, "cg_p64": 2}
+LOOP_FP64_FLOPS = {"bicg_loop64": 48, "cg_loop64": 23}  # an iteration
+
+
+def launch_units(prof, iters, per_launch, per_iteration):
+    """Kernels of a profile that a table counts, with its entry per launch: the one-launch
+    iterations' entries times the profile's Krylov iterations a launch."""
+    out = {}
+    for k, (ms, n) in prof.items():
+        if n > 0 and ms > 0:
+            if k in per_launch:
+                out[k] = per_launch[k]
+            elif k in per_iteration and iters:
+                out[k] = per_iteration[k] * iters / n
+    return out
 
 
 
@@ -145,13 +164,13 @@ def alu_peaks():
         return {"error": str(e)}
 
 
-def alu_roofline(prof, cells, fp_peak):
-    ks = {k: v for k, v in prof.items() if k in KERNEL_FP64_FLOPS and v[1] > 0 and v[0] > 0}
-    if not ks or not fp_peak.get("fp64_tflops"):
+def alu_roofline(prof, cells, fp_peak, iters=0):
+    flops = launch_units(prof, iters, KERNEL_FP64_FLOPS, LOOP_FP64_FLOPS)
+    if not flops or not fp_peak.get("fp64_tflops"):
         return None
-    dom = max(ks, key=lambda k: ks[k][0])
-    ms, n = ks[dom]
-    achieved = KERNEL_FP64_FLOPS[dom] * cells / (ms / n / 1e3) / 1e12
+    dom = max(flops, key=lambda k: prof[k][0])
+    ms, n = prof[dom]
+    achieved = flops[dom] * cells / (ms / n / 1e3) / 1e12
     return {"kernel": dom, "bound": "fp64", "achieved": round(achieved, 4), "peak": fp_peak["fp64_tflops"],
             "unit": "TFLOP/s", "frac": round(achieved / fp_peak["fp64_tflops"], 4),
             "peak_kind": "measured (bench_fp_peak FMA chains)"}
@@ -167,7 +186,7 @@ STEP_KERNELS = {
     "update_uf": (64, 6),             # read eta, p, us, vs, ws; write u, v, w; 3 DADD + 3 DFMA (uniform grid)
     "rhs": (32, 7),                   # read us, vs, ws; write b
     "residual64": (20, 3),            # read b, x; write r (FP32); A x in integers: its conversion, the subtraction,
-                                      # the norm's DFMA
+                                      # the norm's DFMA (a solve's first one also the norm of b: 4)
     "correct64": (24, 1),             # read e (mean), then x, e; write x; 1 DADD (the scaling in integers)
     "mirror32": (36, 0),              # read u, v, w; write u32, v32, w32 (integer rounding; padded fields)
 }
@@ -319,7 +338,7 @@ def run_mode(cg, torch, dist, wl, steps, warmup, solver, precision, maxit=5000, 
             # kernel bracketed by CUDA events on the library's stream
             s.reset_counters()
             s.set_kernel_timing(True)
-            s.step(steps, allow_noconv=True)
+            out["kernel_iters"] = sum(r.iters for r in s.step(steps, allow_noconv=True))
             s.set_kernel_timing(False)
             out["kernels"] = s.kernel_stats()
         return out
@@ -465,15 +484,17 @@ def field_errors(a, b):
     return out
 
 
-def roofline(prof, cells, word_bytes, suffix, hbm_peak, peak_kind, traffic_file):
-    ks = {k: v for k, v in prof.items() if k.endswith(suffix) and k in KERNEL_WORDS and v[1] > 0 and v[0] > 0}
+def roofline(prof, cells, word_bytes, suffix, hbm_peak, peak_kind, traffic_file, iters=0):
+    """iters: the profiled steps' Krylov iterations (for the one-launch kernels)."""
+    words = launch_units(prof, iters, KERNEL_WORDS, LOOP_WORDS)
+    ks = {k: prof[k] for k in words if k.endswith(suffix)}
     if not ks:
         return None, {}
     total = sum(v[0] for v in prof.values())
     dom = max(ks, key=lambda k: ks[k][0])
     ms, n = ks[dom]
     per_launch_s = ms / n / 1e3
-    alg = KERNEL_WORDS[dom] * word_bytes * cells
+    alg = words[dom] * word_bytes * cells
     achieved = alg / per_launch_s / 1e9
     traffic = None
     if traffic_file.exists():
@@ -484,7 +505,7 @@ def roofline(prof, cells, word_bytes, suffix, hbm_peak, peak_kind, traffic_file)
     each = {}
     for k, (kms, kn) in sorted(ks.items(), key=lambda kv: -kv[1][0]):
         us = kms / kn * 1e3
-        gbs = KERNEL_WORDS[k] * word_bytes * cells / (us * 1e-6) / 1e9
+        gbs = words[k] * word_bytes * cells / (us * 1e-6) / 1e9
         each[k] = {"avg_launch_us": round(us, 2), "achieved": round(gbs, 1), "frac": round(gbs / hbm_peak, 4)}
     r = {"kernel": dom, "bound": "hbm", "achieved": round(achieved, 1), "peak": hbm_peak,
          "unit": "GB/s", "frac": round(achieved / hbm_peak, 4), "traffic": traffic,
@@ -534,7 +555,7 @@ def measure_mode(cg, torch, dist, wl, key, steps, warmup, maxit, fp64, t64, hbm_
     if profile:
         word, suffix = (4, "32") if prec == "mixed" else (8, "64")
         out["roofline"], out["kernel_share"] = roofline(rm["kernels"], cells, word, suffix, hbm_peak, peak_kind,
-                                                        traffic_file)
+                                                        traffic_file, rm["kernel_iters"])
         if prec == "mixed":
             c = WORKLOADS[wl]
             npad = (c["nx"] + 4) * (c["ny"] + 4) * (c["nz"] + 4)
@@ -612,7 +633,8 @@ def boundary_set_line(cg, torch, dist, wl, steps, warmup, maxit, hbm_peak, peak_
              "gpu_launches": r["launches"]}
         if prec == "mixed":
             o["error_vs_fp64"] = field_errors(r, runs["fp64"])
-            roof, _ = roofline(r["kernels"], r["cells"], 4, "32", hbm_peak, peak_kind, Path("/nonexistent"))
+            roof, _ = roofline(r["kernels"], r["cells"], 4, "32", hbm_peak, peak_kind, Path("/nonexistent"),
+                               r["kernel_iters"])
             if roof:
                 o["hbm_frac"] = {k: v["frac"] for k, v in roof["per_kernel"].items()}
             base = PRECISION_PAIR[key]
@@ -851,7 +873,7 @@ def main(argv=None):
     t64 = dist.max(fp64["ms"])
     cells = fp64["cells"]
     value = cells * args.steps * dist.world / (t64 / 1e3)
-    roof, share = roofline(fp64["kernels"], cells, 8, "64", hbm_peak, peak_kind, traffic_file)
+    roof, share = roofline(fp64["kernels"], cells, 8, "64", hbm_peak, peak_kind, traffic_file, fp64["kernel_iters"])
     iters64 = [r.iters for r in fp64["stats"]]
     _, _, tol = workload(wl)
     rec64 = solve_record(fp64["stats"], tol)
@@ -863,7 +885,7 @@ def main(argv=None):
         "iters_per_step": iters64, "relres": max(r.relres for r in fp64["stats"]),
         "solves": rec64,
         "gpu_launches": fp64["launches"], "roofline": roof, "kernel_share": share,
-        "alu_roofline": alu_roofline(fp64["kernels"], cells, fp_peak), "fp_peaks": fp_peak,
+        "alu_roofline": alu_roofline(fp64["kernels"], cells, fp_peak, fp64["kernel_iters"]), "fp_peaks": fp_peak,
         "clocks": clk.summary(), "device_mem_gb": fp64["device_mem_gb"],
     }
     if rec64["unconverged_solves"]:
