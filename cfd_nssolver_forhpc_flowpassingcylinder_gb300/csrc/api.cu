@@ -1511,7 +1511,13 @@ int cfdgb_create(const cfdgb_config *cfg, cfdgb_ctx **out) {
       for (int l = 0; l < c->mg.nlev; ++l) c->mg.lev[l].march = 0;
     mg_prepare<float>();
     if ((rc = upload_dense_coarse(c, c->mg))) return bail(rc);
-    if (std::getenv("CFDGB_MG_PER_PASS")) c->mg.ttab = nullptr;  // (and the general tail)
+    if (std::getenv("CFDGB_MG_PER_PASS") || std::getenv("CFDGB_MG_GENERAL_TAIL")) c->mg.ttab = nullptr;
+    if (std::getenv("CFDGB_TRACE")) {
+      int march = 0;
+      for (int l = 0; l < c->mg.nlev; ++l) march += c->mg.lev[l].march;
+      std::fprintf(stderr, "[cfdgb] multigrid: %d levels, %d marching, from level %d in one block%s\n", c->mg.nlev, march,
+                   c->mg.tail, c->mg.tail >= c->mg.nlev ? " (none)" : c->mg.ttab ? " on cell pairs" : "");
+    }
     if ((rc = dalloc(c, &c->ph32, c->ncell)) || (rc = dalloc(c, &c->sh32, c->ncell))) return bail(rc);
     for (int l = 1; l < c->mg.nlev; ++l) {
       MgLevel &L = c->mg.lev[l];
