@@ -1650,7 +1650,7 @@ __global__ void __launch_bounds__(kBlock) k32cg_xr(Geo g, Vec32 v, double *part,
 // each word tagged with the reduction's number, instead of the counter: 152 x 152 polled words
 // slow the stores they wait for, 96x48x4 12.7 -> 23.7 us an iteration: not kept.)
 constexpr int kLoopBlock = 512;
-constexpr int kLoopMaxBlocks = 512;  // sums of the blocks, read by one thread each
+constexpr int kLoopMaxBlocks = 512;  // the most blocks whose sums a slot holds
 constexpr long long kLoopWaitCycles = 1LL << 32;  // ~2 s
 constexpr int kLoopSlots = 5;        // values reduced in an iteration
 
@@ -3013,7 +3013,7 @@ static void launch_loop(cudaStream_t s, bool cg, const Geo &g, const Stencil<dou
   // whole warps of cells a block, and no more blocks than hold any
   const long long chunk = ((g.ncell + blocks - 1) / blocks + 31) / 32 * 32;
   const int nb = (int)((g.ncell + chunk - 1) / chunk);
-  const bool one = !cg && chunk <= kLoopBlock;  // a cell a thread; and a thread for each block's sum
+  const bool one = !cg && chunk <= kLoopBlock;  // a cell a thread
   auto kernel = cg        ? k64cg_loop
                 : one     ? k64_bicg_loop1
                 : !g.nonuni ? k64_bicg_loop<0>
@@ -3021,7 +3021,7 @@ static void launch_loop(cudaStream_t s, bool cg, const Geo &g, const Stencil<dou
                           : k64_bicg_loop<2>;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(nb);
-  cfg.blockDim = dim3(one ? std::max((int)chunk, (nb + 31) / 32 * 32) : kLoopBlock);
+  cfg.blockDim = dim3(one ? (int)chunk : kLoopBlock);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;

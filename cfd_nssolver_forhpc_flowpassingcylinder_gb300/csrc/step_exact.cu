@@ -15,48 +15,6 @@
 
 namespace cfdgb {
 
-// inc/source/Convection_Difussion.hpp:20-51 (QuickUnitA)
-__device__ __forceinline__ void quick_a(bool two, double Up, double Un, long long pp, long long p, long long ic,
-                                        long long n, long long nn, const double *__restrict__ Di,
-                                        const double *__restrict__ Ds, const double *__restrict__ rDi,
-                                        const double *__restrict__ rDs, int I,
-                                        const double *__restrict__ phi, double &P, double &N) {
-  const double fc = phi[ic], fp = phi[p], fn = phi[n];
-  auto oi = [&](double a, int q) { return div_by(a, Di[q], rDi[q], two); };  // a / Di[q]
-  auto os = [&](double a, int q) { return div_by(a, Ds[q], rDs[q], two); };  // a / Ds[q]
-  if (Up > 0.0)
-    P = 0.5 * (fc + fp) - os(0.125 * Di[I + 1] * Di[I + 1], I) * (oi(fp - fc, I + 1) - oi(fc - fn, I));
-  else
-    P = 0.5 * (fc + fp) -
-        os(0.125 * Di[I + 1] * Di[I + 1], I + 1) * (oi(phi[pp] - fp, I + 2) - oi(fp - fc, I + 1));
-  if (Un > 0.0)
-    N = 0.5 * (fn + fc) -
-        os(0.125 * Di[I] * Di[I], I - 1) * (oi(fc - fn, I) - oi(fn - phi[nn], I - 1));
-  else
-    N = 0.5 * (fn + fc) - os(0.125 * Di[I] * Di[I], I) * (oi(fp - fc, I + 1) - oi(fc - fn, I));
-}
-
-// inc/source/Convection_Difussion.hpp:55-90 (QuickUnitB)
-__device__ __forceinline__ void quick_b(bool two, double Up, double Un, long long pp, long long p, long long ic,
-                                        long long n, long long nn, const double *__restrict__ Di,
-                                        const double *__restrict__ Ds, const double *__restrict__ rDi,
-                                        const double *__restrict__ rDs, int I,
-                                        const double *__restrict__ phi, double &P, double &N) {
-  const double fc = phi[ic], fp = phi[p], fn = phi[n];
-  auto oi = [&](double a, int q) { return div_by(a, Di[q], rDi[q], two); };  // a / Di[q]
-  auto os = [&](double a, int q) { return div_by(a, Ds[q], rDs[q], two); };  // a / Ds[q]
-  if (Up > 0.0)
-    P = 0.5 * (fc + fp) - oi(0.125 * Ds[I] * Ds[I], I) * (os(fp - fc, I) - os(fc - fn, I - 1));
-  else
-    P = 0.5 * (fc + fp) -
-        oi(0.125 * Ds[I] * Ds[I], I + 1) * (os(phi[pp] - fp, I + 1) - os(fp - fc, I));
-  if (Un > 0.0)
-    N = 0.5 * (fn + fc) -
-        oi(0.125 * Ds[I - 1] * Ds[I - 1], I - 1) * (os(fc - fn, I - 1) - os(fn - phi[nn], I - 2));
-  else
-    N = 0.5 * (fn + fc) - oi(0.125 * Ds[I - 1] * Ds[I - 1], I) * (os(fp - fc, I) - os(fc - fn, I - 1));
-}
-
 // inc/source/Convection_Difussion.hpp:96-147 (LudUnitA; LudUnitB has the same body)
 __device__ __forceinline__ void lud(bool two, double Up, double Un, long long pp, long long p, long long ic, long long n,
                                     long long nn, const double *__restrict__ Di, const double *__restrict__ Ds,
@@ -74,22 +32,18 @@ __device__ __forceinline__ void lud(bool two, double Up, double Un, long long pp
     N = (fc + oi(0.5 * Ds[I] * (fc - fp), I + 1));
 }
 
-// face values of one axis under the convection switch (inc/0_General.hpp:114-118): QUICK,
-// LUD or UD (UdUnit, :150-168); OWN: the component's own axis (the "A" units)
-template <int S, bool OWN>
+// face values of one axis under the convection switch (inc/0_General.hpp:114-118): LUD or UD
+// (UdUnit, :150-168; QUICK is k_convdiff_quick)
+template <int S>
 __device__ __forceinline__ void face(bool two, double Up, double Un, long long pp, long long p, long long ic, long long n,
                                      long long nn, const double *__restrict__ Di, const double *__restrict__ Ds,
                                      const double *__restrict__ rDi, const double *__restrict__ rDs, int I,
                                      const double *__restrict__ phi, double &P, double &N) {
   if (S == CFDGB_LUD) {
     lud(two, Up, Un, pp, p, ic, n, nn, Di, Ds, rDi, rDs, I, phi, P, N);
-  } else if (S == CFDGB_UD) {
+  } else {
     P = Up > 0.0 ? phi[ic] : phi[p];
     N = Un > 0.0 ? phi[n] : phi[ic];
-  } else if (OWN) {
-    quick_a(two, Up, Un, pp, p, ic, n, nn, Di, Ds, rDi, rDs, I, phi, P, N);
-  } else {
-    quick_b(two, Up, Un, pp, p, ic, n, nn, Di, Ds, rDi, rDs, I, phi, P, N);
   }
 }
 
@@ -124,7 +78,7 @@ __global__ void __launch_bounds__(kBlock) k_smagorinsky(Geo g, const double *__r
   }
 }
 
-// inc/source/Convection_Difussion.hpp:174-450: explicit Euler convection (QUICK, LUD or UD)
+// inc/source/Convection_Difussion.hpp:174-450: explicit Euler convection (LUD or UD here)
 // + central diffusion; the last face along a component's own axis is a boundary face and
 // skipped.
 // S: the convection scheme; nut (compact, may be null): the Smagorinsky eddy viscosity
@@ -178,9 +132,9 @@ __global__ void __launch_bounds__(kBlock, 2) k_convdiff_exact(Geo g, double dt_a
       const double Wp = w[ic] + (w[xp] - w[ic]) * IT;
       const double Wn = w[zm] + (w[zm + xp - ic] - w[zm]) * IT;
       double uPx, uNx, uPy, uNy, uPz, uNz;
-      face<S, true>(two, Up, Un, ic + 2 * sx, xp, ic, xm, ic - 2 * sx, Dx, Dxs, rDx, rDxs, i, u, uPx, uNx);
-      face<S, false>(two, Vp, Vn, ic + 2 * sy, yp, ic, ym, ic - 2 * sy, Dy, Dys, rDy, rDys, j, u, uPy, uNy);
-      face<S, false>(two, Wp, Wn, ic + 2 * sz, zp, ic, zm, ic - 2 * sz, Dz, Dzs, rDz, rDzs, k, u, uPz, uNz);
+      face<S>(two, Up, Un, ic + 2 * sx, xp, ic, xm, ic - 2 * sx, Dx, Dxs, rDx, rDxs, i, u, uPx, uNx);
+      face<S>(two, Vp, Vn, ic + 2 * sy, yp, ic, ym, ic - 2 * sy, Dy, Dys, rDy, rDys, j, u, uPy, uNy);
+      face<S>(two, Wp, Wn, ic + 2 * sz, zp, ic, zm, ic - 2 * sz, Dz, Dzs, rDz, rDzs, k, u, uPz, uNz);
       const double convection = -dt * (oxs(uPx * uPx - uNx * uNx, i) + oy(uPy * Vp - uNy * Vn, j) +
                                        oz(uPz * Wp - uNz * Wn, k));
       const double difussion =
@@ -203,9 +157,9 @@ __global__ void __launch_bounds__(kBlock, 2) k_convdiff_exact(Geo g, double dt_a
       const double Wp = w[ic] + (w[yp] - w[ic]) * IT;
       const double Wn = w[zm] + (w[zm + yp - ic] - w[zm]) * IT;
       double vPx, vNx, vPy, vNy, vPz, vNz;
-      face<S, false>(two, Up, Un, ic + 2 * sx, xp, ic, xm, ic - 2 * sx, Dx, Dxs, rDx, rDxs, i, v, vPx, vNx);
-      face<S, true>(two, Vp, Vn, ic + 2 * sy, yp, ic, ym, ic - 2 * sy, Dy, Dys, rDy, rDys, j, v, vPy, vNy);
-      face<S, false>(two, Wp, Wn, ic + 2 * sz, zp, ic, zm, ic - 2 * sz, Dz, Dzs, rDz, rDzs, k, v, vPz, vNz);
+      face<S>(two, Up, Un, ic + 2 * sx, xp, ic, xm, ic - 2 * sx, Dx, Dxs, rDx, rDxs, i, v, vPx, vNx);
+      face<S>(two, Vp, Vn, ic + 2 * sy, yp, ic, ym, ic - 2 * sy, Dy, Dys, rDy, rDys, j, v, vPy, vNy);
+      face<S>(two, Wp, Wn, ic + 2 * sz, zp, ic, zm, ic - 2 * sz, Dz, Dzs, rDz, rDzs, k, v, vPz, vNz);
       const double convection = -dt * (ox(Up * vPx - Un * vNx, i) + oys(vPy * vPy - vNy * vNy, j) +
                                        oz(Wp * vPz - Wn * vNz, k));
       const double difussion =
@@ -228,9 +182,9 @@ __global__ void __launch_bounds__(kBlock, 2) k_convdiff_exact(Geo g, double dt_a
       const double Vp = v[ic] + (v[zp] - v[ic]) * IT;
       const double Vn = v[ym] + (v[ym + zp - ic] - v[ym]) * IT;
       double wPx, wNx, wPy, wNy, wPz, wNz;
-      face<S, false>(two, Up, Un, ic + 2 * sx, xp, ic, xm, ic - 2 * sx, Dx, Dxs, rDx, rDxs, i, w, wPx, wNx);
-      face<S, false>(two, Vp, Vn, ic + 2 * sy, yp, ic, ym, ic - 2 * sy, Dy, Dys, rDy, rDys, j, w, wPy, wNy);
-      face<S, true>(two, Wp, Wn, ic + 2 * sz, zp, ic, zm, ic - 2 * sz, Dz, Dzs, rDz, rDzs, k, w, wPz, wNz);
+      face<S>(two, Up, Un, ic + 2 * sx, xp, ic, xm, ic - 2 * sx, Dx, Dxs, rDx, rDxs, i, w, wPx, wNx);
+      face<S>(two, Vp, Vn, ic + 2 * sy, yp, ic, ym, ic - 2 * sy, Dy, Dys, rDy, rDys, j, w, wPy, wNy);
+      face<S>(two, Wp, Wn, ic + 2 * sz, zp, ic, zm, ic - 2 * sz, Dz, Dzs, rDz, rDzs, k, w, wPz, wNz);
       const double convection = -dt * (ox(Up * wPx - Un * wNx, i) + oy(Vp * wPy - Vn * wNy, j) +
                                        ozs(wPz * wPz - wNz * wNz, k));
       const double difussion =
@@ -248,11 +202,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_convdiff_exact(Geo g, double dt_a
   if (sc.ss) cfl_finish(cfl, dt, sc);
 }
 
-// The same for QUICK, with every face computed once.  The kernel is bound by the FP64 pipe
-// (one warp instruction per 64 cycles and scheduler, idle lanes included), so what counts is
-// the number of FP64 instructions a cell: the per-cell form above evaluates both faces of each
-// axis (every face twice), divides every difference up to four times and forms the QUICK
-// factors by division, about 1050 instructions; here
+// The same for QUICK (QuickUnitA and QuickUnitB, Convection_Difussion.hpp:20-90), with every face
+// computed once.  The kernel is bound by the FP64 pipe (one warp instruction per 64 cycles and
+// scheduler, idle lanes included), so what counts is the number of FP64 instructions a cell: in the
+// per-cell form above both faces of each axis (every face twice), up to four divisions of
+// every difference and the QUICK factors' divisions took about 1050; here
 //   - a block of (tk + 2) x (rows + 1) threads marches along x, a thread owning one (j, k)
 //     column: the x face of plane i is kept in registers as the lower face of plane i + 1;
 //   - the differences and the upper faces along y and z go through shared memory to the
