@@ -241,7 +241,10 @@ int cfdgb_step(cfdgb_ctx *ctx, int nsteps, cfdgb_step_stats *stats);
  * transposed Poisson solve (the operator is symmetric on the uniform grid) is the
  * context's own: FP64 BiCGSTAB (preconditioned by the FP64 V-cycle when the context has
  * the multigrid preconditioner), or for a MIXED context the same FP32 sweeps in FP64
- * refinement as its forward solves, to the same FP64 tolerance.  Memory beyond the
+ * refinement as its forward solves, to the same FP64 tolerance.  MIXED: both calls form the
+ * refinement's residual by FMAs on every grid where cfdgb_step forms it in 64-bit integers on
+ * uniform ones, so J is the mean of the drag that cfdgb_step reports to the solves' tolerance, not to
+ * the last bit.  Memory beyond the
  * forward's: per checkpoint u, v, w (padded FP64) and the solver's warm start (compact; p
  * is rebuilt from it), plus p for the first; per window step u, v, w (padded FP64) and p
  * (padded FP32); about 14 padded FP64 fields of adjoint state, and 1 compact one (MIXED)
