@@ -140,7 +140,8 @@ struct cfdgb_ctx {
   double omega = 0.0;  // SOR relaxation in use (cfg.omega, or the optimal one when that is 0)
   // test switch (environment CFDGB_TEST_WAIT_FAULT at create, 1 or 2): the next MIXED solve makes
   // one bounded wait of the FP32 bulk-copy pipeline run out, the next FP64 one a wait between the
-  // blocks of its one-launch iterations (2: in the last block only), to exercise that failure path
+  // blocks of its one-launch iterations (2: its set-up leaves the mark of one that ran out in another
+  // block than 0), to exercise that failure path
   int test_wait_fault = 0;
   // one CUDA graph per time step (FP64 Krylov solvers, after the first step, kernel timing
   // off): the whole step with its convergence loop as a conditional WHILE node; each step

@@ -149,6 +149,14 @@ __device__ __forceinline__ T spmv_at(const Geo &g, const Stencil<T> &st, const T
   return stencil_apply<T>(g, st, ic, jc, kc, row, [&](long long q) { return x[q]; }, c);
 }
 
+// a solve starts without a fault (the host's test request 2: with one, as another block's wait leaves
+// it that runs out at the last barrier while block 0's all end)
+__device__ __forceinline__ void take_test_fault(SolverScal *sc) {
+  const bool planted = sc->test_wait == 2;
+  sc->fault = planted;
+  if (planted) sc->test_wait = 0;
+}
+
 // ---- FP64 set-up: bicgstabRe2.hpp:86-106 ----
 // restart: 1 for the preconditioned iteration, whose first p kernel then takes p = r0 = r1
 __global__ void __launch_bounds__(kBlock) k_bicg_setup64(Geo g, Stencil<double> st, KrylovVecs<double> v,
@@ -175,7 +183,7 @@ __global__ void __launch_bounds__(kBlock) k_bicg_setup64(Geo g, Stencil<double> 
     sc->iter = 0;
     sc->done = 0;
     sc->status = 0;
-    sc->fault = 0;
+    take_test_fault(sc);
     sc->restart = restart;
     sc->relres = 0.0;
   }
@@ -1416,7 +1424,7 @@ __global__ void __launch_bounds__(kBlock) k64cg_setup(Geo g, Stencil<double> st,
     sc->rho = out[1];
     sc->iter = 0;
     sc->status = 0;
-    sc->fault = 0;
+    take_test_fault(sc);
     sc->relres = sqrt(out[1]) / sc->norm0;
     sc->done = (sc->relres < sc->tol) ? 1 : 0;
   }
@@ -1664,12 +1672,6 @@ struct LoopGrid {
   double *part;     // [slot][kLoopMaxBlocks]
   unsigned target;  // arrivals that complete the next barrier
   long long limit;  // cycles a wait may take
-  bool late;        // test request 2, in block 0: leave after another block's wait has run out
-  __device__ __forceinline__ void hold() const {
-    const long long t0 = clock64();
-    while (atomicAdd(&sc->fault, 0) == 0 && clock64() - t0 < 8 * limit) {
-    }
-  }
   // one thread: this block's arrival, and the wait for all (the block's stores come before, by the
   // barrier that its threads passed)
   __device__ __forceinline__ void arrive_wait(LoopScal &L) {
@@ -1738,13 +1740,12 @@ struct LoopGrid {
   }
 };
 
-// The test requests (sc->test_wait, set only by the host's test switch), every block with a short
-// limit: 1, block 0 waits for one arrival too many, which runs out at the chunk's last barrier; 2,
-// the last block does, and block 0, whose waits all end, leaves after that
+// The test request (sc->test_wait, set only by the host's test switch): block 0 waits for one
+// arrival too many, every block with a short limit, so that its wait at the chunk's last barrier runs
+// out
 __device__ __forceinline__ LoopGrid loop_grid(SolverScal *sc, double *part) {
   const int test = sc->test_wait;
-  const unsigned one = test && blockIdx.x == (test == 2 ? gridDim.x - 1 : 0u) ? 1u : 0u;
-  return LoopGrid{sc, part, one, test ? kTestWaitCycles : kLoopWaitCycles, test == 2 && blockIdx.x == 0};
+  return LoopGrid{sc, part, test && blockIdx.x == 0 ? 1u : 0u, test ? kTestWaitCycles : kLoopWaitCycles};
 }
 // scalars in, and out by block 0 when every block has left the loop's last barrier
 __device__ __forceinline__ void loop_begin(LoopScal &L, const SolverScal *sc) {
@@ -1771,7 +1772,6 @@ __device__ __forceinline__ void loop_end(const LoopScal &L, const LoopGrid &G) {
   if (L.bad) {
     atomicExch(&sc->fault, 1);
   } else if (blockIdx.x == 0) {
-    if (G.late) G.hold();
     sc->rho = L.rho;
     sc->alpha = L.alpha;
     sc->omega = L.omega;

@@ -36,8 +36,8 @@ def test_the_next_solve_starts_clean(monkeypatch, solver):
 @pytest.mark.parametrize("solver", ["jacobi", "cg"])
 @pytest.mark.parametrize("graph", [True, False])
 def test_block_0_leaving_last_does_not_hide_it(monkeypatch, solver, graph):
-    """Request 2: the last block gives up at the chunk's last barrier; block 0, whose own waits
-    all ended, writes the solve's scalars after that."""
+    """Request 2: the solve carries the fault of a block that gave up at the chunk's last barrier;
+    block 0, whose own waits all ended, writes the solve's scalars after that."""
     with started(monkeypatch, "2", graph, solver=solver) as s:
         with pytest.raises(cg.CfdgbError, match="bounded wait between blocks") as e:
             s.step(1)
