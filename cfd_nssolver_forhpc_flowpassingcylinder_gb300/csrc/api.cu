@@ -140,7 +140,7 @@ struct cfdgb_ctx {
   double omega = 0.0;  // SOR relaxation in use (cfg.omega, or the optimal one when that is 0)
   // test switch (environment CFDGB_TEST_WAIT_FAULT at create, 1 or 2): the next MIXED solve makes
   // one bounded wait of the FP32 bulk-copy pipeline run out, the next FP64 one a wait between the
-  // blocks of its one-launch iterations (2: its set-up leaves the mark of one that ran out in another
+  // blocks of its one-launch iterations (2: that solve finds the mark of one that ran out in another
   // block than 0), to exercise that failure path
   int test_wait_fault = 0;
   // one CUDA graph per time step (FP64 Krylov solvers, after the first step, kernel timing
@@ -607,8 +607,11 @@ int set_solver_params(cfdgb_ctx *c, SolverScal *dsc, double tol, int maxit) {
 // the test switch (one shot): the next launch that waits on dsc makes a bounded wait run out
 int request_test_wait(cfdgb_ctx *c, SolverScal *dsc) {
   if (!c->test_wait_fault) return 0;
-  const int request = c->test_wait_fault;
-  CK(cudaMemcpyAsync(&dsc->test_wait, &request, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  static const int one = 1;
+  if (c->test_wait_fault == 2 && dsc == c->sc)
+    CK(cudaMemcpyAsync(&dsc->cnt[7], &kLoopGaveUp, sizeof(unsigned), cudaMemcpyHostToDevice, c->stream));
+  else
+    CK(cudaMemcpyAsync(&dsc->test_wait, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   c->test_wait_fault = 0;
   return 0;
 }

@@ -108,6 +108,7 @@ int loop64_blocks(long long ncell);
 // state fits the multiprocessors (cg32_loop_fits: uniform grids, up to 2.4 M cells on 152 of them);
 // the launch ends early when the sweep does
 constexpr int kCg32LoopIters = 256;
+constexpr unsigned kLoopGaveUp = 1u << 16;  // a block's mark in SolverScal::cnt[7] (fewer blocks than that)
 bool cg32_loop_fits(const Geo &g, const Stencil<float> &st, int nsm);
 void launch_cg32_loop(cudaStream_t s, const Geo &g, const Stencil<float> &st, KrylovVecs<float> v, float *const p2[2],
                       float *const ap2[2], double *part_buf, SolverScal *sc, int nsm);

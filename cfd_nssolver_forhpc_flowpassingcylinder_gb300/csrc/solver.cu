@@ -149,14 +149,6 @@ __device__ __forceinline__ T spmv_at(const Geo &g, const Stencil<T> &st, const T
   return stencil_apply<T>(g, st, ic, jc, kc, row, [&](long long q) { return x[q]; }, c);
 }
 
-// a solve starts without a fault (the host's test request 2: with one, as another block's wait leaves
-// it that runs out at the last barrier while block 0's all end)
-__device__ __forceinline__ void take_test_fault(SolverScal *sc) {
-  const bool planted = sc->test_wait == 2;
-  sc->fault = planted;
-  if (planted) sc->test_wait = 0;
-}
-
 // ---- FP64 set-up: bicgstabRe2.hpp:86-106 ----
 // restart: 1 for the preconditioned iteration, whose first p kernel then takes p = r0 = r1
 __global__ void __launch_bounds__(kBlock) k_bicg_setup64(Geo g, Stencil<double> st, KrylovVecs<double> v,
@@ -183,7 +175,7 @@ __global__ void __launch_bounds__(kBlock) k_bicg_setup64(Geo g, Stencil<double> 
     sc->iter = 0;
     sc->done = 0;
     sc->status = 0;
-    take_test_fault(sc);
+    sc->fault = 0;
     sc->restart = restart;
     sc->relres = 0.0;
   }
@@ -1424,7 +1416,7 @@ __global__ void __launch_bounds__(kBlock) k64cg_setup(Geo g, Stencil<double> st,
     sc->rho = out[1];
     sc->iter = 0;
     sc->status = 0;
-    take_test_fault(sc);
+    sc->fault = 0;
     sc->relres = sqrt(out[1]) / sc->norm0;
     sc->done = (sc->relres < sc->tol) ? 1 : 0;
   }
@@ -1653,10 +1645,11 @@ __global__ void __launch_bounds__(kBlock) k32cg_xr(Geo g, Vec32 v, double *part,
 // 131 K 31.1 -> 21.3, 1.05 M 75.9 -> 65.1 (the FP64 pipe's time is 41.7), 2.1 M 131.8 -> 120.3,
 // stretched 1.6 M 117.6 -> 94.7; CG 8 K 12.6 -> 8.4, 314 K 24.7 -> 17.1.
 // The barrier counts arrivals (sc->cnt[6], back to zero through sc->cnt[7] when the last block
-// leaves).  A wait is bounded: one that gives up sets sc->fault, the block leaves, and so do the
-// others, each after its own bounded wait; the last one out turns the fault into CFDGB_ECUDA.  (Polling all blocks' sums,
-// each word tagged with the reduction's number, instead of the counter: 152 x 152 polled words
-// slow the stores they wait for, 96x48x4 12.7 -> 23.7 us an iteration: not kept.)
+// leaves).  A wait is bounded: a block whose wait gives up leaves with a mark in the second counter,
+// and so do the others, each after its own bounded wait; the last one out turns it into sc->fault and
+// CFDGB_ECUDA.  (Polling all blocks' sums, each word tagged with the reduction's number, instead of the
+// counter: 152 x 152 polled words slow the stores they wait for, 96x48x4 12.7 -> 23.7 us an iteration:
+// not kept.)
 constexpr int kLoopBlock = 512;
 constexpr int kLoopMaxBlocks = 512;  // the most blocks whose sums a slot holds
 constexpr long long kLoopWaitCycles = 1LL << 32;  // ~2 s
@@ -1769,9 +1762,7 @@ __device__ __forceinline__ void loop_end(const LoopScal &L, const LoopGrid &G) {
   SolverScal *const sc = G.sc;
   __syncthreads();
   if (threadIdx.x != 0) return;
-  if (L.bad) {
-    atomicExch(&sc->fault, 1);
-  } else if (blockIdx.x == 0) {
+  if (L.bad == 0 && blockIdx.x == 0) {
     sc->rho = L.rho;
     sc->alpha = L.alpha;
     sc->omega = L.omega;
@@ -1785,9 +1776,12 @@ __device__ __forceinline__ void loop_end(const LoopScal &L, const LoopGrid &G) {
     sc->restart = L.restart;
   }
   __threadfence();
-  if (atomicAdd(&sc->cnt[7], 1u) == gridDim.x - 1) {  // every block is past its last wait
-    __threadfence();
-    if (atomicAdd(&sc->fault, 0)) {  // over what block 0 left: its own waits may all have ended
+  // blocks that left, and above them those whose wait gave up
+  const unsigned own = L.bad ? kLoopGaveUp + 1u : 1u, left = atomicAdd(&sc->cnt[7], own) + own;
+  if ((left & (kLoopGaveUp - 1u)) == gridDim.x) {  // every block is past its last wait
+    if (left >= kLoopGaveUp) {  // over what block 0 left: its own waits may all have ended
+      __threadfence();
+      sc->fault = 1;
       sc->status = CFDGB_ECUDA;
       sc->done = 1;
       sc->test_wait = 0;
