@@ -23,8 +23,8 @@ __device__ __forceinline__ int nblocks() { return gridDim.x * gridDim.y * gridDi
 // bits below its last place kept, rounded), is split into 26-bit fields whose sums over 32
 // lanes fit 32 bits (three redux.sync), and the total is converted back once.  The rounding
 // is at most 1/32 ulp of the largest value per lane, below that of a tree of FP64 additions,
-// and the result does not depend on the order.  With the scalar work below on three lanes:
-// FP64 BiCGSTAB on 256x128x32 88 -> 74 us an iteration, FP64 CG on 151x77x27 29.5 -> 24.3,
+// and the result does not depend on the order.  With the scalar work on three lanes (div3), on the
+// kernels a phase: FP64 BiCGSTAB on 256x128x32 88 -> 74 us an iteration, FP64 CG on 151x77x27 29.5 -> 24.3,
 // FP32 CG sweeps on 256x128x64 24.0 -> 21.5.  Values that do not fit this (Inf, NaN, and
 // exponents near either end of the range) take the shuffle tree.
 constexpr int kSumGuard = 4;  // bits kept below the largest value's last place

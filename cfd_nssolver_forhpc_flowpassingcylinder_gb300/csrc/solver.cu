@@ -1641,9 +1641,8 @@ __global__ void __launch_bounds__(kBlock) k32cg_xr(Geo g, Vec32 v, double *part,
 // reducing phase every block sums the block partials itself, in the same order, so the
 // scalars need no second round trip.  Same operations per cell as the kernels above; the dot
 // products are summed in this partition's order.
-// Measured, us an iteration, a kernel a phase -> one launch: BiCGSTAB 8 K cells 21.4 -> 11.9,
-// 131 K 31.1 -> 21.3, 1.05 M 75.9 -> 65.1 (the FP64 pipe's time is 41.7), 2.1 M 131.8 -> 120.3,
-// stretched 1.6 M 117.6 -> 94.7; CG 8 K 12.6 -> 8.4, 314 K 24.7 -> 17.1.
+// Measured, us an iteration, a kernel a phase -> one launch: BiCGSTAB 18 K cells 26 -> 11.7, 1.05 M
+// 76 -> 61 (the FP64 pipe's time is 41.7), stretched 1.6 M 118 -> 83; CG 314 K 24.7 -> 15.6.
 // The barrier counts arrivals (sc->cnt[6], back to zero through sc->cnt[7] when the last block
 // leaves).  A wait is bounded: a block whose wait gives up leaves with a mark in the second counter,
 // and so do the others, each after its own bounded wait; the last one out turns it into sc->fault and
